@@ -161,7 +161,7 @@ struct rp_world {
     DevBuf d_rec, d_slot_entity;                   // the records on the device; entity of each body slot
     cudaEvent_t ev_rec = nullptr;                  // the last record upload (h_rec is refilled after it)
     double adj_prof[6] = {0, 0, 0, 0, 0, 0};      // last adjoint's slowest scene (rp_adjoint_profile)
-    DevBuf d_pose_f, d_body_scene, d_col_body, d_scene_order, d_gjk_list, d_hit_list, d_work_list, d_work_state, d_work_simplex, d_work_epa, d_queue, d_work_off, d_work_face, d_fallback, d_tstamp, d_tlist, d_single_hull, d_pair_base, d_ext_base;
+    DevBuf d_pose_f, d_body_scene, d_col_body, d_scene_order, d_gjk_list, d_hit_list, d_work_list, d_work_state, d_work_simplex, d_work_epa, d_queue, d_work_off, d_work_face, d_fallback, d_tstamp, d_tlist, d_single_hull, d_pair_base, d_solve_scenes;
     int mode = RP_MODE_AUTO;          // RP_MODE_*: how a frame is launched
     int solo_nodes = 512;             // tunable: grid sweeps run levels up to this size on one CTA
     int cta_from = 0;                 // tunable: batched sweeps give a whole CTA to scenes of this cost or more (0: none)
@@ -172,6 +172,7 @@ struct rp_world {
     bool pipe_ready = false;
     PipeConfig pipe;
     PipeDims dims;
+    bool solve_fits = false;          // every scene fits k_solve (its bodies and joints in shared memory)
     uint64_t layout_gen = 0;          // bumped whenever device buffers are (re)allocated
     cudaGraphExec_t graph = nullptr;  // one captured frame of the pipeline
     uint64_t graph_gen = ~0ull;
@@ -314,8 +315,9 @@ rp_status build_device(rp_world* w) {
         if (pc > (1LL << 30) || cc > (1LL << 30)) return fail(RP_ERR_CAPACITY, "scratch sizes beyond 2^30 entries");
         w->scene_pair_cap[(size_t)s + 1] = w->scene_pair_cap[(size_t)s] + (int32_t)pc;
         w->scene_contact_cap[(size_t)s + 1] = w->scene_contact_cap[(size_t)s] + (int32_t)cc;
-        w->scene_node_cap[(size_t)s + 1] = w->scene_node_cap[(size_t)s] + (int32_t)pc +
-                                           (w->scene_ext[(size_t)s + 1] - w->scene_ext[(size_t)s]);
+        // a scene's nodes start on a word of the node bitmap of their own
+        w->scene_node_cap[(size_t)s + 1] = (w->scene_node_cap[(size_t)s] + (int32_t)pc +
+                                            (w->scene_ext[(size_t)s + 1] - w->scene_ext[(size_t)s]) + 31) & ~31;
     }
     w->grid_mode = (S == 1 && max_bodies >= 256);
     w->max_levels = w->grid_mode ? 8192 : 1024;
@@ -577,7 +579,6 @@ rp_status build_device(rp_world* w) {
         RP_CUDA(w->d_work_epa.ensure(std::max<size_t>(P, 1) * 4 * 8));
         RP_CUDA(w->d_work_off.ensure(std::max<size_t>(P, 1) * 16));
         RP_CUDA(w->d_pair_base.ensure(std::max<size_t>(P, 1) * 16));
-        RP_CUDA(w->d_ext_base.ensure(std::max<size_t>(E, 1) * 16));
         RP_CUDA(w->d_fallback.ensure(std::max<size_t>(P, 1) * 4));
         RP_CUDA(w->d_work_face.ensure(std::max<size_t>(P, 1) * 12 * 4));
         std::vector<int32_t> order((size_t)S);
@@ -592,6 +593,36 @@ rp_status build_device(rp_world* w) {
         w->order_cost.assign((size_t)S, 0);
         for (int sc = 0; sc < S; ++sc) w->order_cost[(size_t)sc] = cost(order[(size_t)sc]);
         set_cta_scenes(w);
+        {   // scene-resident solves: two size classes, each in decreasing cost order
+            std::vector<int32_t> list;
+            PipeDims& d = w->dims;
+            d.solve_count[0] = d.solve_count[1] = 0;
+            size_t smem = 0;
+            bool fits = true;
+            for (int k = 0; k < 2; ++k) {
+                d.solve_bodies[k] = d.solve_joints[k] = 0;
+                for (int32_t sc : order) {
+                    const int nb = w->scene_body[(size_t)sc + 1] - w->scene_body[(size_t)sc];
+                    const int nj = w->scene_ext[(size_t)sc + 1] - w->scene_ext[(size_t)sc];
+                    const bool small = nb <= SOLVE_SMALL_BODIES && nj <= SOLVE_SMALL_BODIES;
+                    if (small != (k == 1)) continue;
+                    list.push_back(sc);
+                    d.solve_count[k]++;
+                    d.solve_bodies[k] = std::max(d.solve_bodies[k], nb);
+                    d.solve_joints[k] = std::max(d.solve_joints[k], nj);
+                    fits = fits && nb <= SOLVE_SCENE_BODIES;
+                }
+                if (d.solve_count[k] && fits) {
+                    smem = w->precision == RP_PRECISION_FP64 ? pipe_solve_smem_f64(d.solve_bodies[k], d.solve_joints[k])
+                                                             : pipe_solve_smem_f32(d.solve_bodies[k], d.solve_joints[k]);
+                    fits = smem <= (size_t)SOLVE_MAX_SMEM;
+                }
+            }
+            // one large scene of the exact build is bound by FP64 arithmetic: its sweeps keep every SM
+            w->solve_fits = fits && !(w->grid_mode && w->precision == RP_PRECISION_FP64);
+            RP_CUDA(upload(w->d_solve_scenes, list, st));
+            d.solve_scenes = w->d_solve_scenes.as<int32_t>();
+        }
         RP_CUDA(w->d_queue.ensure(64));
         RP_CUDA(cudaMemsetAsync(w->d_queue.p, 0, 64, st));
         // transform-list stamps restart with the substep counter
@@ -736,7 +767,6 @@ WorldView<R> make_view(rp_world* w) {
     V.work_epa = w->d_work_epa.as<double>();
     V.work_off = w->d_work_off.as<float4>();
     V.pair_base = w->d_pair_base.as<float4>();
-    V.ext_base = w->d_ext_base.as<float4>();
     V.fallback_list = w->d_fallback.as<int32_t>();
     V.work_face = w->d_work_face.as<float>();
     V.queue = w->d_queue.as<int32_t>();
@@ -935,7 +965,15 @@ cudaError_t launch_pipeline(rp_world* w, const StepParams& P) {
         if (e != cudaSuccess) return e;
         w->pipe_ready = true;
     }
-    w->launches += (uint64_t)(w->precision == RP_PRECISION_FP64 ? pipe_launches_f64(P) : pipe_launches_f32(P));
+    // the coloured order has a schedule of its own
+    w->dims.solve = w->solve_fits && w->sweep_order == RP_SWEEP_REFERENCE ? 1 : 0;
+    if (w->dims.solve && w->dims.solve_count[0] && w->dims.solve_count[1] && !w->pipe.join) {   // two branches
+        e = cudaStreamCreateWithFlags(&w->pipe.side, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->pipe.fork, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->pipe.join, cudaEventDisableTiming);
+        if (e != cudaSuccess) return e;
+    }
+    w->launches += (uint64_t)(w->precision == RP_PRECISION_FP64 ? pipe_launches_f64(P, w->dims) : pipe_launches_f32(P, w->dims));
     if (!w->timing && w->stream == nullptr) {
         // the legacy default stream cannot be captured: launch the frame's kernels directly
         return pipe_frame(w, P, nullptr);
@@ -1080,6 +1118,12 @@ void rp_world_destroy(rp_world* w) {
     if (w->ev_rec) cudaEventDestroy(w->ev_rec);
     if (w->graph) cudaGraphExecDestroy(w->graph);
     for (cudaEvent_t ev : w->marks) cudaEventDestroy(ev);
+    if (w->pipe.side) {
+        cudaStreamSynchronize(w->pipe.side);
+        cudaStreamDestroy(w->pipe.side);
+    }
+    if (w->pipe.fork) cudaEventDestroy(w->pipe.fork);
+    if (w->pipe.join) cudaEventDestroy(w->pipe.join);
     if (w->own_stream && w->stream) cudaStreamDestroy(w->stream);
     delete w;
 }

@@ -14,12 +14,24 @@ struct PipeConfig {
     // tunable (rp_autotune): the schedule does not depend on them (FP64 results identical, FP32 to rounding)
     int transform_group = 4;     // threads per collider in the hull transform
     int sweep_cta = 0;           // batched sweeps: one CTA per scene instead of one warp per scene
+    // a second stream and its fork / join events: the two size classes of k_solve run side by side
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
 };
 struct PipeDims {
     int nbodies = 0, ncolliders = 0, next = 0, num_scenes = 0;
     int node_words = 0;  // words of the node bitmap (node capacity / 32 + 1)
     int grid_mode = 0;   // one large scene: cooperative setup and sweeps
+    // scene-resident solves (k_solve) in place of the sweep, velocity and predict kernels: the scenes in two
+    // size classes (0: the larger ones), solve_scenes lists class 0 then class 1
+    int solve = 0;
+    const int32_t* solve_scenes = nullptr;
+    int solve_count[2] = {0, 0};
+    int solve_bodies[2] = {0, 0}, solve_joints[2] = {0, 0};   // largest scene of each class
 };
+constexpr int SOLVE_SCENE_BODIES = 640;   // scenes of more bodies keep the sweep kernels
+constexpr int SOLVE_SMALL_BODIES = 128;   // class 1
+constexpr int SOLVE_MAX_SMEM = 200 * 1024;
 // Optional events recorded after each phase (timing runs; never inside a captured graph).
 struct PipeMarks {
     cudaEvent_t* ev = nullptr;
@@ -38,7 +50,8 @@ struct PipeMarks {
     cudaError_t pipe_configure_##SUF(PipeConfig& c, int sms);                                                 \
     cudaError_t pipe_frame_##SUF(const WorldView<R>& W, const StepParams& P, const PipeConfig& c, const PipeDims& d, \
                                  cudaStream_t st, PipeMarks* marks);                                          \
-    int pipe_launches_##SUF(const StepParams& P);
+    int pipe_launches_##SUF(const StepParams& P, const PipeDims& d);                                          \
+    size_t pipe_solve_smem_##SUF(int bodies, int joints);
 
 // Adjoint of the substep (rp_adjoint.cu): one scene per thread.
 struct AdjGeom {                           // the world's collider geometry (FP64), shared by all scenes

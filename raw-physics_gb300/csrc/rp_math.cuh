@@ -39,6 +39,24 @@ template <typename T> RP_HD V3<T> vnorm(V3<T> v) {
 }
 template <typename T> RP_HD V3<T> vinv(V3<T> v) { return vsub(v3<T>(0, 0, 0), v); }
 #ifdef __CUDACC__
+// FP32 algebra with every rounding spelled out: which product of a sum is fused is the source's choice,
+// not the compiler's, so a solve gives the same bits in every kernel and in every arrangement of its
+// work over threads. sum2 / dif2 fuse the left product and round the right one first; where the solves
+// fuse the right one, the products are passed in that order.
+__device__ __forceinline__ float sum2(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }   // ab + cd
+__device__ __forceinline__ float dif2(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }  // ab - cd
+__device__ __forceinline__ float sum3(float a, float b, float c, float d, float e, float f) { return __fmaf_rn(e, f, sum2(a, b, c, d)); }
+__device__ __forceinline__ V3<float> add_f(V3<float> a, V3<float> b) { return {__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z)}; }
+__device__ __forceinline__ V3<float> sub_f(V3<float> a, V3<float> b) { return {__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z)}; }
+__device__ __forceinline__ V3<float> scale_f(float s, V3<float> v) { return {__fmul_rn(s, v.x), __fmul_rn(s, v.y), __fmul_rn(s, v.z)}; }
+// c + s v
+__device__ __forceinline__ V3<float> axpy_f(float s, V3<float> v, V3<float> c) {
+    return {__fmaf_rn(s, v.x, c.x), __fmaf_rn(s, v.y, c.y), __fmaf_rn(s, v.z, c.z)};
+}
+__device__ __forceinline__ float dot_f(V3<float> a, V3<float> b) { return sum3(a.x, b.x, a.y, b.y, a.z, b.z); }
+__device__ __forceinline__ V3<float> cross_f(V3<float> a, V3<float> b) {
+    return {dif2(a.y, b.z, a.z, b.y), dif2(a.z, b.x, a.x, b.z), dif2(a.x, b.y, a.y, b.x)};
+}
 // FP64 unit vector without FP64 square root or division (GB300 issues FP64 at 1/64 of the FP32
 // rate): an FP32 reciprocal-square-root seed refined by two Newton-Raphson steps,
 // r <- r (3 - d r^2) / 2, which reach full FP64 precision from the seed's ~23 bits. Lengths outside
@@ -106,6 +124,47 @@ template <typename T> RP_HD V3<T> qaxis(Qt<T> q, int axis) {
     default: return v3<T>(two * q.x * q.z - two * q.w * q.y, two * q.y * q.z + two * q.w * q.x, one - (two * q.x * q.x) - (two * q.y * q.y));
     }
 }
+
+#ifdef __CUDACC__
+// qrotate, qmat3, mmulv and the product (v, 0) q with their roundings spelled out. left_x, left_yz: which
+// product of the first pair of the x, and of the y and z components is fused.
+__device__ __forceinline__ V3<float> rotate_f(Qt<float> q, V3<float> v, bool left_x = false, bool left_yz = false) {
+    const float ix = __fmaf_rn(-q.z, v.y, left_x ? sum2(q.w, v.x, q.y, v.z) : sum2(q.y, v.z, q.w, v.x));
+    const float iy = __fmaf_rn(-q.x, v.z, left_yz ? sum2(q.w, v.y, q.z, v.x) : sum2(q.z, v.x, q.w, v.y));
+    const float iz = __fmaf_rn(-q.y, v.x, left_yz ? sum2(q.w, v.z, q.x, v.y) : sum2(q.x, v.y, q.w, v.z));
+    const float iw = __fmaf_rn(-q.z, v.z, dif2(-q.x, v.x, q.y, v.y));
+    return {__fmaf_rn(iz, q.y, __fmaf_rn(iy, -q.z, sum2(ix, q.w, iw, -q.x))),
+            __fmaf_rn(ix, q.z, __fmaf_rn(iz, -q.x, sum2(iy, q.w, iw, -q.y))),
+            __fmaf_rn(iy, q.x, __fmaf_rn(ix, -q.y, sum2(iz, q.w, iw, -q.z)))};
+}
+// right_xy: the two xy elements fuse their second product
+__device__ __forceinline__ M3<float> mat3_f(Qt<float> q, bool right_xy = false) {
+    const float x2 = 2.f * q.x, y2 = 2.f * q.y, z2 = 2.f * q.z, w2 = 2.f * q.w;
+    M3<float> r;
+    r.d[0][0] = __fmaf_rn(-z2, q.z, __fmaf_rn(-y2, q.y, 1.f));
+    r.d[1][1] = __fmaf_rn(-z2, q.z, __fmaf_rn(-x2, q.x, 1.f));
+    r.d[2][2] = __fmaf_rn(-y2, q.y, __fmaf_rn(-x2, q.x, 1.f));
+    r.d[1][0] = right_xy ? sum2(w2, q.z, x2, q.y) : sum2(x2, q.y, w2, q.z);
+    r.d[0][1] = right_xy ? sum2(-w2, q.z, x2, q.y) : dif2(x2, q.y, w2, q.z);
+    r.d[2][0] = dif2(x2, q.z, w2, q.y);
+    r.d[0][2] = sum2(x2, q.z, w2, q.y);
+    r.d[2][1] = sum2(y2, q.z, w2, q.x);
+    r.d[1][2] = dif2(y2, q.z, w2, q.x);
+    return r;
+}
+__device__ __forceinline__ V3<float> mulv_f(const M3<float>& m, V3<float> v) {
+    return {sum3(m.d[0][0], v.x, m.d[0][1], v.y, m.d[0][2], v.z), sum3(m.d[1][0], v.x, m.d[1][1], v.y, m.d[1][2], v.z),
+            sum3(m.d[2][0], v.x, m.d[2][1], v.y, m.d[2][2], v.z)};
+}
+__device__ __forceinline__ Qt<float> qmul_pure_f(V3<float> a, Qt<float> b) {
+    Qt<float> r;
+    r.w = __fmaf_rn(-a.z, b.z, __fmaf_rn(-a.y, b.y, -__fmul_rn(a.x, b.x)));
+    r.x = __fmaf_rn(-a.z, b.y, sum2(a.y, b.z, a.x, b.w));
+    r.y = __fmaf_rn(-a.x, b.z, sum2(a.z, b.x, a.y, b.w));
+    r.z = __fmaf_rn(-a.y, b.x, sum2(a.x, b.y, a.z, b.w));
+    return r;
+}
+#endif
 
 template <typename T> RP_HD M3<T> mmul(const M3<T>& a, const M3<T>& b) {
     M3<T> r;

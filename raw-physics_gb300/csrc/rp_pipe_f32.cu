@@ -8,5 +8,6 @@ cudaError_t pipe_frame_f32(const WorldView<float>& W, const StepParams& P, const
                            cudaStream_t st, PipeMarks* marks) {
     return PipeLauncher<float, false>::frame(W, P, c, d, st, marks);
 }
-int pipe_launches_f32(const StepParams& P) { return PipeLauncher<float, false>::launches_per_frame(P); }
+int pipe_launches_f32(const StepParams& P, const PipeDims& d) { return PipeLauncher<float, false>::launches_per_frame(P, d); }
+size_t pipe_solve_smem_f32(int bodies, int joints) { return PipeLauncher<float, false>::solve_bytes(bodies, joints); }
 }  // namespace rp

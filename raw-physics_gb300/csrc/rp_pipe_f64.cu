@@ -8,5 +8,6 @@ cudaError_t pipe_frame_f64(const WorldView<double>& W, const StepParams& P, cons
                            cudaStream_t st, PipeMarks* marks) {
     return PipeLauncher<double, true>::frame(W, P, c, d, st, marks);
 }
-int pipe_launches_f64(const StepParams& P) { return PipeLauncher<double, true>::launches_per_frame(P); }
+int pipe_launches_f64(const StepParams& P, const PipeDims& d) { return PipeLauncher<double, true>::launches_per_frame(P, d); }
+size_t pipe_solve_smem_f64(int bodies, int joints) { return PipeLauncher<double, true>::solve_bytes(bodies, joints); }
 }  // namespace rp

@@ -24,6 +24,7 @@
 //   k_manifold  warp per hit_list entry: contact manifold (or the general path); writes contacts
 #pragma once
 #include "rp_step.cuh"
+#include "rp_scene.cuh"
 #include "rp_launch.h"
 
 namespace rp {
@@ -181,14 +182,7 @@ __global__ void __launch_bounds__(PIPE_BLOCK) k_predict(WorldView<R> W, int nbod
     if (frame_abandoned(W.status)) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
     for (int b = t; b < nbodies; b += n) {
-        predict_body<R, EXACT>(W, b, h);
-        if constexpr (EXACT) {
-            const double4_32a p = W.pos[b], q = W.rot[b];
-            W.pose_f[2 * b] = make_float4((float)p.x, (float)p.y, (float)p.z, 0.f);
-            W.pose_f[2 * b + 1] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
-        } else {
-            stage_body(W, b);
-        }
+        predict_stage<R, EXACT, true>(W, b, h);
     }
     for (int e = t; e < next; e += n)
         for (int k = 0; k < 4; ++k) W.ext_lambda[4 * (size_t)e + k] = 0.0;
@@ -197,7 +191,7 @@ __global__ void __launch_bounds__(PIPE_BLOCK) k_predict(WorldView<R> W, int nbod
         W.act_count[2 * s] = 0;
         W.act_count[2 * s + 1] = 0;
     }
-    if (t == 0) { W.queue[2] = 0; W.queue[3] = 0; W.queue[4] += 1; W.queue[5] = 0; W.queue[7] = 0; }
+    if (t == 0) reset_narrow_queue(W);
 }
 
 // The hulls of the bodies k_cull listed for this substep (tlist: bodies of the pairs that go on to
@@ -251,14 +245,6 @@ __global__ void __launch_bounds__(PIPE_BLOCK) k_cull(WorldView<R> W, int enabled
     if (frame_abandoned(W.status)) return;
     __shared__ int scan_smem[32];
     __shared__ int base_smem;
-    if constexpr (!std::is_same<R, double>::value) {   // the joints' FP32 solve frames of this substep
-        const int ne = W.scene_ext[W.num_scenes];
-        for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += gridDim.x * blockDim.x) {
-            const ExtConstraint& C = W.ext[e];
-            const double4_32a pa = W.pos[C.e1], pb = W.pos[C.e2];
-            W.ext_base[e] = make_float4((float)(pa.x - pb.x), (float)(pa.y - pb.y), (float)(pa.z - pb.z), 0.f);
-        }
-    }
     const int n = W.queue[0];
     unsigned long long apart = 0;
     for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
@@ -775,7 +761,11 @@ __device__ bool resched_serial(const WorldView<R>& W, int s, SerialSmem& sm) {
         *v1.levels = 0;
     }
     __syncwarp();
-    if (sm.overflow) return false;
+    if (sm.overflow) {   // resched counts the active nodes itself, from zero
+        if (lane == 0) { *v0.active = 0; *v1.active = 0; }
+        __syncwarp();
+        return false;
+    }
     // bucket by level from the shared counts: prefix (the level table the sweep reads), then every
     // lane places list entries at its level's cursor (shared-memory atomics)
     for (int which = 0; which < 2; ++which) {
@@ -890,6 +880,7 @@ struct PipeLauncher {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k_manifold<R, EXACT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)narrow_smem());
         if (e == cudaSuccess && !EXACT)
             e = cudaFuncSetAttribute(k_fallback<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fallback_smem());
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_solve<R, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SOLVE_MAX_SMEM);
         if (e != cudaSuccess) return e;
         int nb = 0;
         auto occ = [&](const void* f, int block, size_t smem) {
@@ -941,6 +932,28 @@ struct PipeLauncher {
         return cudaGetLastError();
     }
 
+    static size_t solve_bytes(int bodies, int joints) { return solve_smem<R>(solve_room(bodies, joints)); }
+
+    // The solver half of a substep, scene by scene (k_solve): the larger scenes with 256 threads each, the
+    // others with 128 and less shared memory, side by side on two branches.
+    static cudaError_t solve(const WorldView<R>& W, const StepParams& P, const PipeConfig& c, const PipeDims& d, cudaStream_t st,
+                             double h, int predict) {
+        cudaError_t e = cudaSuccess;
+        const int alike = d.grid_mode;
+        auto launch = [&](int k, cudaStream_t s, int reset) -> cudaError_t {
+            const SolveRoom room = solve_room(d.solve_bodies[k], d.solve_joints[k]);
+            k_solve<R, EXACT><<<d.solve_count[k], k == 0 ? SOLVE_BLOCK : SOLVE_BLOCK / 2, solve_smem<R>(room), s>>>(
+                W, d.solve_scenes + (k ? d.solve_count[0] : 0), room, h, P.num_pos_iters, alike, predict, reset);
+            return cudaGetLastError();
+        };
+        if (d.solve_count[0] == 0) return launch(1, st, 1);
+        if (d.solve_count[1] == 0) return launch(0, st, 1);
+        if ((e = cudaEventRecord(c.fork, st)) != cudaSuccess || (e = cudaStreamWaitEvent(c.side, c.fork, 0)) != cudaSuccess) return e;
+        if ((e = launch(0, st, 1)) != cudaSuccess || (e = launch(1, c.side, 0)) != cudaSuccess) return e;
+        if ((e = cudaEventRecord(c.join, c.side)) != cudaSuccess) return e;
+        return cudaStreamWaitEvent(st, c.join, 0);
+    }
+
     static cudaError_t frame(const WorldView<R>& W, const StepParams& P, const PipeConfig& c, const PipeDims& d,
                              cudaStream_t st, PipeMarks* marks) {
         cudaError_t e = cudaMemsetAsync(W.queue, 0, sizeof(int32_t), st);
@@ -961,12 +974,16 @@ struct PipeLauncher {
         else k_setup_cta<R><<<d.num_scenes, BLOCK, 0, st>>>(W, P.dt), e = cudaGetLastError();
         if (e != cudaSuccess || (e = mark(PH_BROAD)) != cudaSuccess) return e;
         for (int sub = 0; sub < P.num_substeps; ++sub) {
-            k_predict<R, EXACT><<<body_blocks, PIPE_BLOCK, 0, st>>>(W, d.nbodies, d.next, h);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            if ((e = cudaMemsetAsync(W.node_bits, 0, (size_t)d.node_words * 4, st)) != cudaSuccess) return e;
-            if ((e = mark(PH_PREDICT)) != cudaSuccess) return e;
-            k_cull<R><<<c.cull_blocks, PIPE_BLOCK, 0, st>>>(W, P.enable_collisions);
-            if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(PH_NARROW)) != cudaSuccess) return e;
+            if (sub == 0 || !d.solve) {   // k_solve predicts the next substep and clears the bits it has read
+                k_predict<R, EXACT><<<body_blocks, PIPE_BLOCK, 0, st>>>(W, d.nbodies, d.next, h);
+                if ((e = cudaGetLastError()) != cudaSuccess) return e;
+                if ((e = cudaMemsetAsync(W.node_bits, 0, (size_t)d.node_words * 4, st)) != cudaSuccess) return e;
+                if ((e = mark(PH_PREDICT)) != cudaSuccess) return e;
+            }
+            if (P.enable_collisions || sub == 0 || !d.solve) {   // without collisions it only empties the pairs' contacts
+                k_cull<R><<<c.cull_blocks, PIPE_BLOCK, 0, st>>>(W, P.enable_collisions);
+                if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(PH_NARROW)) != cudaSuccess) return e;
+            }
             if (P.enable_collisions) {
                 k_transform<R, EXACT><<<col_blocks, PIPE_BLOCK, 0, st>>>(W, c.transform_group);
                 if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(PH_TRANSFORM)) != cudaSuccess) return e;
@@ -989,6 +1006,11 @@ struct PipeLauncher {
                 }
                 if ((e = mark(PH_MANIFOLD)) != cudaSuccess) return e;
             }
+            if (d.solve) {
+                if ((e = solve(W, P, c, d, st, h, sub + 1 < P.num_substeps ? 1 : 0)) != cudaSuccess) return e;
+                if ((e = mark(PH_SOLVE)) != cudaSuccess) return e;
+                continue;
+            }
             for (int it = 0; it < P.num_pos_iters; ++it) {
                 const int first = it == 0 ? 1 : 0;   // the substep's schedules are built by its first sweep
                 if (d.grid_mode) e = coop(k_sweep_grid<R, EXACT, false>, c.sweep_grid_blocks, BLOCK, st, W, h, first);
@@ -1007,7 +1029,10 @@ struct PipeLauncher {
         return cudaSuccess;
     }
 
-    static int launches_per_frame(const StepParams& P) {
+    static int launches_per_frame(const StepParams& P, const PipeDims& d) {
+        if (d.solve)
+            return 2 + (P.enable_collisions ? 0 : 1) +
+                   P.num_substeps * ((P.enable_collisions ? (EXACT ? 6 : 8) : 0) + (d.solve_count[0] > 0) + (d.solve_count[1] > 0));
         const int per_sub = 2 + (P.enable_collisions ? (EXACT ? 6 : 8) : 1) + P.num_pos_iters + 1;
         return 1 + P.num_substeps * per_sub;
     }

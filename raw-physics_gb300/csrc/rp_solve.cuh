@@ -1,9 +1,14 @@
 // XPBD constraint solves, integration and velocity passes on the device.
 //
-// Bodies touched by one solver node (a broad-phase pair with its contacts, or one external joint)
-// are loaded into registers, updated in the order the reference applies its corrections, and
-// written back once; nodes of one level never share a non-fixed body, so no two threads write the
-// same body.
+// Two lanes of a warp solve one solver node (a broad-phase pair with its contacts, or one external
+// joint), one lane per body (Duo): each lane loads its body into registers, applies the corrections in
+// the reference's order and writes it back once; nodes of one level never share a non-fixed body, so no
+// two lanes write the same body. The corrections of the two bodies differ only in sign, so the second
+// body's lane works on negated vectors (separation, normal, impulse): negation is exact, every product
+// and sum rounds as in the one-thread form, and both lanes take the same branches.
+// What bounds a node is the instruction stream of one warp with two active lanes: a contact is
+// about a thousand dependent instructions in the one-thread form. Half of them belong to each body,
+// so the lane pair halves the stream.
 //
 // EXACT=true mirrors the reference's FP64 expressions term for term (built without FMA
 // contraction it reproduces the reference bit for bit). EXACT=false keeps positions and
@@ -58,34 +63,29 @@ template <typename R>
 __device__ __forceinline__ Qt<R> wq(const Qt<double>& q) { return qcast<R>(q); }
 
 // --------------------------------------------------------------------------------------------
-// Position_Constraint_Preprocessed_Data / positional constraint (pbd_base_constraints.cpp:6-123)
-template <typename R>
-struct Pcpd {
-    V3<R> r1, r2;      // r_wc
-    M3<R> I1, I2;      // world inverse inertia
+// The lane pair of one solver node: lanes 2i and 2i + 1 of a warp hold the node's first and second
+// body. Both lanes of a pair always call these together.
+struct Duo {
+    unsigned mask;
+    int side;          // 0: the node's first body, 1: its second
+    bool second_right; // FP32 contacts: this lane's sums are fused as a second body's (see JOINT)
+    template <typename T> __device__ __forceinline__ T other(T v) const { return __shfl_xor_sync(mask, v, 1); }
+    template <typename T> __device__ __forceinline__ V3<T> other(V3<T> v) const { return v3<T>(other(v.x), other(v.y), other(v.z)); }
+    template <typename T> __device__ __forceinline__ Qt<T> other(Qt<T> q) const {
+        return qt<T>(other(q.x), other(q.y), other(q.z), other(q.w));
+    }
+    // the vector as the first body sees it, from this lane's body's side
+    template <typename T> __device__ __forceinline__ V3<T> own(V3<T> v) const {
+        return side ? v3<T>(-v.x, -v.y, -v.z) : v;
+    }
+    // the first / second body's value, given this lane's value and the other's
+    template <typename V> __device__ __forceinline__ V first(const V& mine, const V& theirs) const { return side ? theirs : mine; }
+    template <typename V> __device__ __forceinline__ V second(const V& mine, const V& theirs) const { return side ? mine : theirs; }
 };
 
-template <typename R>
-__device__ __forceinline__ Pcpd<R> pcpd(const Body<R>& a, const Body<R>& b, V3<R> r1_lc, V3<R> r2_lc) {
-    Pcpd<R> p;
-    Qt<R> qa = wq<R>(a.q), qb = wq<R>(b.q);
-    p.r1 = qrotate(qa, r1_lc);
-    p.r2 = qrotate(qb, r2_lc);
-    p.I1 = world_tensor(qa, a.Iinv);
-    p.I2 = world_tensor(qb, b.Iinv);
-    return p;
-}
-
-template <typename R>
-__device__ __forceinline__ R pos_dlambda(const Body<R>& a, const Body<R>& b, const Pcpd<R>& p, R h, R compliance, R lambda,
-                                         V3<R> dx) {
-    R c = vlen(dx);
-    if (c <= Tiny<R>::v) return (R)0;
-    V3<R> n = v3<R>(dx.x / c, dx.y / c, dx.z / c);
-    R w1 = a.invm + vdot(vcross(p.r1, n), mmulv(p.I1, vcross(p.r1, n)));
-    R w2 = b.invm + vdot(vcross(p.r2, n), mmulv(p.I2, vcross(p.r2, n)));
-    R til = compliance / (h * h);
-    return (-c - til * lambda) / (w1 + w2 + til);
+__device__ __forceinline__ Duo duo_of_lane() {
+    const unsigned lane = threadIdx.x & 31u;
+    return Duo{3u << (lane & 30u), (int)(lane & 1u), (lane & 1u) != 0u};
 }
 
 // Normalisation of an FP64 quaternion in the FP32 build: an FP32 reciprocal square root refined by
@@ -111,107 +111,83 @@ __device__ __forceinline__ void q_add_normalize(Qt<double>& q, Qt<R> d, double s
     }
 }
 
-template <typename R>
-__device__ __forceinline__ void pos_apply(Body<R>& a, Body<R>& b, const Pcpd<R>& p, R dl, V3<R> dx) {
-    R c = vlen(dx);
-    if (c <= Tiny<R>::v) return;
-    V3<R> n = v3<R>(dx.x / c, dx.y / c, dx.z / c);
-    V3<R> imp = vscale(dl, n);
-    if (!a.fixed) a.x = vadd(a.x, v3cast<double>(vscale(a.invm, imp)));
-    if (!b.fixed) b.x = vadd(b.x, v3cast<double>(vscale(-b.invm, imp)));
-    V3<R> a1 = mmulv(p.I1, vcross(p.r1, imp));
-    V3<R> a2 = mmulv(p.I2, vcross(p.r2, imp));
-    Qt<R> q1 = qmul(qt<R>(a1.x, a1.y, a1.z, (R)0), wq<R>(a.q));
-    Qt<R> q2 = qmul(qt<R>(a2.x, a2.y, a2.z, (R)0), wq<R>(b.q));
-    if (!a.fixed) q_add_normalize(a.q, q1, 0.5);
-    if (!b.fixed) q_add_normalize(b.q, q2, -0.5);
-}
-
-// Angular constraint (pbd_base_constraints.cpp:125-227)
-template <typename R>
-struct Acpd { M3<R> I1, I2; };
-
-template <typename R>
-__device__ __forceinline__ Acpd<R> acpd(const Body<R>& a, const Body<R>& b) {
-    Acpd<R> r;
-    r.I1 = world_tensor(wq<R>(a.q), a.Iinv);
-    r.I2 = world_tensor(wq<R>(b.q), b.Iinv);
-    return r;
-}
-
-template <typename R>
-__device__ __forceinline__ R ang_dlambda(const Acpd<R>& A, R h, R compliance, R lambda, V3<R> dq) {
-    R th = vlen(dq);
-    if (th <= Tiny<R>::v) return (R)0;
-    V3<R> n = v3<R>(dq.x / th, dq.y / th, dq.z / th);
-    R w1 = vdot(n, mmulv(A.I1, n));
-    R w2 = vdot(n, mmulv(A.I2, n));
-    R til = compliance / (h * h);
-    return (-th - til * lambda) / (w1 + w2 + til);
-}
-
-template <typename R>
-__device__ __forceinline__ void ang_apply(Body<R>& a, Body<R>& b, const Acpd<R>& A, R dl, V3<R> dq) {
-    R th = vlen(dq);
-    if (th <= Tiny<R>::v) return;
-    V3<R> n = v3<R>(dq.x / th, dq.y / th, dq.z / th);
-    V3<R> imp = vscale(-dl, n);
-    V3<R> a1 = mmulv(A.I1, imp);
-    V3<R> a2 = mmulv(A.I2, imp);
-    Qt<R> q1 = qmul(qt<R>(a1.x, a1.y, a1.z, (R)0), wq<R>(a.q));
-    Qt<R> q2 = qmul(qt<R>(a2.x, a2.y, a2.z, (R)0), wq<R>(b.q));
-    if (!a.fixed) q_add_normalize(a.q, q1, 0.5);
-    if (!b.fixed) q_add_normalize(b.q, q2, -0.5);
-}
-
-// x_a + r_a - (x_b + r_b), with the position difference formed in FP64 in the FP32 build
-template <typename R, bool EXACT>
-__device__ __forceinline__ V3<R> anchor_delta(const Body<R>& a, const Body<R>& b, V3<R> ra, V3<R> rb) {
-    if (EXACT) return v3cast<R>(vsub(vadd(a.x, v3cast<double>(ra)), vadd(b.x, v3cast<double>(rb))));
-    return vadd(v3cast<R>(vsub(a.x, b.x)), vsub(ra, rb));
-}
-
 // --------------------------------------------------------------------------------------------
+// Exact build: positional corrections (pbd_base_constraints.cpp:6-123) of this lane's body. r: the
+// anchor in world axes, I: the body's world inverse inertia, dx: the separation seen from this body.
+__device__ __forceinline__ double pos_dlambda(const Duo& D, const Body<double>& B, V3<double> r, const M3<double>& I, double h,
+                                              double compliance, double lambda, V3<double> dx) {
+    const double c = vlen(dx);
+    if (c <= Tiny<double>::v) return 0.0;
+    const V3<double> n = v3<double>(dx.x / c, dx.y / c, dx.z / c);
+    const double w = B.invm + vdot(vcross(r, n), mmulv(I, vcross(r, n)));
+    const double til = compliance / (h * h);
+    return (-c - til * lambda) / (w + D.other(w) + til);
+}
+
+__device__ __forceinline__ void pos_apply(Body<double>& B, V3<double> r, const M3<double>& I, double dl, V3<double> dx) {
+    const double c = vlen(dx);
+    if (c <= Tiny<double>::v) return;
+    const V3<double> n = v3<double>(dx.x / c, dx.y / c, dx.z / c);
+    const V3<double> imp = vscale(dl, n);
+    const V3<double> a = mmulv(I, vcross(r, imp));
+    const Qt<double> dq = qmul(qt<double>(a.x, a.y, a.z, 0.0), B.q);
+    if (!B.fixed) {
+        B.x = vadd(B.x, vscale(B.invm, imp));
+        q_add_normalize(B.q, dq, 0.5);
+    }
+}
+
+// Angular corrections (pbd_base_constraints.cpp:125-227); dq seen from this body
+__device__ __forceinline__ double ang_dlambda(const Duo& D, const M3<double>& I, double h, double compliance, double lambda,
+                                              V3<double> dq) {
+    const double th = vlen(dq);
+    if (th <= Tiny<double>::v) return 0.0;
+    const V3<double> n = v3<double>(dq.x / th, dq.y / th, dq.z / th);
+    const double w = vdot(n, mmulv(I, n));
+    const double til = compliance / (h * h);
+    return (-th - til * lambda) / (w + D.other(w) + til);
+}
+
+__device__ __forceinline__ void ang_apply(Body<double>& B, const M3<double>& I, double dl, V3<double> dq) {
+    const double th = vlen(dq);
+    if (th <= Tiny<double>::v) return;
+    const V3<double> n = v3<double>(dq.x / th, dq.y / th, dq.z / th);
+    const V3<double> a = mmulv(I, vscale(-dl, n));
+    const Qt<double> q1 = qmul(qt<double>(a.x, a.y, a.z, 0.0), B.q);
+    if (!B.fixed) q_add_normalize(B.q, q1, 0.5);
+}
+
 // collision_constraint_solve (pbd.cpp:107-154). c points at the contact record
 // {r1_lc, lambda_n, r2_lc, lambda_t, normal, -}.
-template <typename R, bool EXACT>
-__device__ void collision_solve(const WorldView<R>& W, Body<R>& a, Body<R>& b, R* c, R h, const R mus) {
-    V3<R> r1 = v3<R>(c[0], c[1], c[2]), r2 = v3<R>(c[4], c[5], c[6]), n = v3<R>(c[8], c[9], c[10]);
-    R lambda_n = c[3], lambda_t = c[7];
-    Pcpd<R> p = pcpd(a, b, r1, r2);
-    V3<R> d12 = anchor_delta<R, EXACT>(a, b, p.r1, p.r2);
-    R d = vdot(d12, n);
-    if (d > (R)0) {
-        V3<R> dx = vscale(d, n);
-        R dl = pos_dlambda(a, b, p, h, (R)0, lambda_n, dx);
-        pos_apply(a, b, p, dl, dx);
-        lambda_n += dl;
-        p = pcpd(a, b, r1, r2);
-        dl = pos_dlambda(a, b, p, h, (R)0, lambda_t, dx);
-        R lt = lambda_t + dl;
-        if (lt > mus * lambda_n) {
-            // p1 - p1_til - (p2 - p2_til) with p_til from the previous pose (pbd.cpp:142-148)
-            double4_32a pa = W.prev_pos[a.idx], qa = W.prev_rot[a.idx], pb = W.prev_pos[b.idx], qb = W.prev_rot[b.idx];
-            V3<double> xa_prev = v3<double>(pa.x, pa.y, pa.z), xb_prev = v3<double>(pb.x, pb.y, pb.z);
-            Qt<R> qa_prev = qcast<R>(qt<double>(qa.x, qa.y, qa.z, qa.w)), qb_prev = qcast<R>(qt<double>(qb.x, qb.y, qb.z, qb.w));
-            V3<R> dp;
-            if (EXACT) {
-                V3<double> p1 = vadd(a.x, v3cast<double>(p.r1)), p2 = vadd(b.x, v3cast<double>(p.r2));
-                V3<double> p1t = vadd(xa_prev, v3cast<double>(qrotate(qa_prev, r1)));
-                V3<double> p2t = vadd(xb_prev, v3cast<double>(qrotate(qb_prev, r2)));
-                dp = v3cast<R>(vsub(vsub(p1, p1t), vsub(p2, p2t)));
-            } else {
-                V3<R> da = vadd(v3cast<R>(vsub(a.x, xa_prev)), vsub(p.r1, qrotate(qa_prev, r1)));
-                V3<R> db = vadd(v3cast<R>(vsub(b.x, xb_prev)), vsub(p.r2, qrotate(qb_prev, r2)));
-                dp = vsub(da, db);
-            }
-            V3<R> dpt = vsub(dp, vscale(vdot(dp, n), n));
-            pos_apply(a, b, p, dl, dpt);
-            lambda_t += dl;
-        }
+static __device__ void collision_solve(const WorldView<double>& W, const Duo& D, Body<double>& B, double* c, double h, double mus) {
+    const V3<double> r_lc = v3<double>(c[4 * D.side], c[4 * D.side + 1], c[4 * D.side + 2]);
+    const V3<double> n = D.own(v3<double>(c[8], c[9], c[10]));
+    V3<double> r = qrotate(B.q, r_lc);
+    const V3<double> p0 = vadd(B.x, r);
+    const double d = vdot(vsub(p0, D.other(p0)), n);
+    if (!(d > 0.0)) return;
+    double lambda_n = c[3], lambda_t = c[7];
+    const V3<double> dx = vscale(d, n);
+    M3<double> I = world_tensor(B.q, B.Iinv);
+    double dl = pos_dlambda(D, B, r, I, h, 0.0, lambda_n, dx);
+    pos_apply(B, r, I, dl, dx);
+    lambda_n += dl;
+    r = qrotate(B.q, r_lc);
+    I = world_tensor(B.q, B.Iinv);
+    dl = pos_dlambda(D, B, r, I, h, 0.0, lambda_t, dx);
+    const double lt = lambda_t + dl;
+    if (lt > mus * lambda_n) {
+        // p1 - p1_til - (p2 - p2_til) with p_til from the previous pose (pbd.cpp:142-148)
+        const double4_32a x4 = W.prev_pos[B.idx], q4 = W.prev_rot[B.idx];
+        const V3<double> pt = vadd(v3<double>(x4.x, x4.y, x4.z), qrotate(qt<double>(q4.x, q4.y, q4.z, q4.w), r_lc));
+        const V3<double> u = vsub(vadd(B.x, r), pt);
+        const V3<double> dp = vsub(u, D.other(u));
+        pos_apply(B, r, I, dl, vsub(dp, vscale(vdot(dp, n), n)));
+        lambda_t += dl;
     }
-    c[3] = lambda_n;
-    c[7] = lambda_t;
+    // both lanes hold the same multipliers: each writes one
+    __syncwarp(D.mask);
+    c[D.side ? 7 : 3] = D.side ? lambda_t : lambda_n;
 }
 
 // limit_angle (pbd.cpp:175-217)
@@ -256,127 +232,100 @@ __device__ __forceinline__ bool limit_may_act(V3<float> n, V3<float> n1, V3<floa
     return !(phi >= (float)lo + 0.01f && phi <= (float)hi - 0.01f);
 }
 
-template <typename R, bool EXACT>
-__device__ void ext_solve(const WorldView<R>& W, const ExtConstraint& C, double* lam, R h) {
-    Body<R> a = load_body(W, C.e1), b = load_body(W, C.e2);
-    V3<R> r1 = v3<R>((R)C.r1[0], (R)C.r1[1], (R)C.r1[2]), r2 = v3<R>((R)C.r2[0], (R)C.r2[1], (R)C.r2[2]);
+// one joint limit of the exact build: the angle between n1 (first body) and n2 (second body) about n,
+// clamped to [lo, hi] (limit_angle), corrected with a zero-compliance angular solve
+__device__ __forceinline__ void limit_solve(const Duo& D, Body<double>& B, V3<double> n, V3<double> n1, V3<double> n2, double lo,
+                                            double hi, double h, double* lam) {
+    if (lo <= -PI_REF && hi >= PI_REF) return;   // the wrapped angle can never leave limits at or beyond +-pi
+    V3<double> dq;
+    if (!limit_angle<double>(n, n1, n2, lo, hi, dq)) return;
+    dq = D.own(dq);
+    const M3<double> I = world_tensor(B.q, B.Iinv);
+    const double l = *lam;
+    const double dl = ang_dlambda(D, I, h, 0.0, l, dq);
+    ang_apply(B, I, dl, dq);
+    __syncwarp(D.mask);
+    if (D.side == 0) *lam = l + dl;
+}
+
+// External constraints of the exact build (pbd.cpp:81-379), one lane per body
+static __device__ void ext_solve(const WorldView<double>& W, const Duo& D, const ExtConstraint& C, double* lam, double h) {
+    Body<double> B = load_body(W, D.side ? C.e2 : C.e1);
+    const double* rl = D.side ? C.r2 : C.r1;
+    const V3<double> r_lc = v3<double>(rl[0], rl[1], rl[2]);
+    // one positional correction with lambda lam[k]
+    auto positional = [&](int k, double compliance, V3<double> r, V3<double> dx) {
+        const M3<double> I = world_tensor(B.q, B.Iinv);
+        const double l = lam[k];
+        const double dl = pos_dlambda(D, B, r, I, h, compliance, l, dx);
+        pos_apply(B, r, I, dl, dx);
+        __syncwarp(D.mask);
+        if (D.side == 0) lam[k] = l + dl;
+    };
+    auto angular = [&](int k, V3<double> dq) {
+        const M3<double> I = world_tensor(B.q, B.Iinv);
+        const double l = lam[k];
+        const double dl = ang_dlambda(D, I, h, C.compliance, l, dq);
+        ang_apply(B, I, dl, dq);
+        __syncwarp(D.mask);
+        if (D.side == 0) lam[k] = l + dl;
+    };
+    // an axis of the first and of the second body, in both lanes
+    auto axes = [&](int k1, int k2, V3<double>& u1, V3<double>& u2) {
+        const V3<double> mine = qaxis(B.q, D.side ? k2 : k1), theirs = D.other(mine);
+        u1 = D.first(mine, theirs);
+        u2 = D.second(mine, theirs);
+    };
     switch (C.type) {
     case CON_POSITIONAL: {  // pbd.cpp:81-97
-        V3<R> dx = vsub(v3cast<R>(vsub(a.x, b.x)), v3<R>((R)C.distance[0], (R)C.distance[1], (R)C.distance[2]));
-        if (EXACT) dx = v3cast<R>(vsub(vsub(a.x, b.x), v3<double>(C.distance[0], C.distance[1], C.distance[2])));
-        Pcpd<R> p = pcpd(a, b, r1, r2);
-        R dl = pos_dlambda(a, b, p, h, (R)C.compliance, (R)lam[0], dx);
-        pos_apply(a, b, p, dl, dx);
-        lam[0] += (double)dl;
+        const V3<double> dist = D.own(v3<double>(C.distance[0], C.distance[1], C.distance[2]));
+        positional(0, C.compliance, qrotate(B.q, r_lc), vsub(vsub(B.x, D.other(B.x)), dist));
     } break;
     case CON_MUTUAL_ORIENTATION: {  // pbd.cpp:156-173
-        Acpd<R> A = acpd(a, b);
-        Qt<R> aux = qmul(wq<R>(a.q), qinverse(wq<R>(b.q)));
-        V3<R> dq = v3<R>((R)2.0 * aux.x, (R)2.0 * aux.y, (R)2.0 * aux.z);
-        R dl = ang_dlambda(A, h, (R)C.compliance, (R)lam[0], dq);
-        ang_apply(a, b, A, dl, dq);
-        lam[0] += (double)dl;
+        const Qt<double> oq = D.other(B.q);
+        const Qt<double> aux = qmul(D.first(B.q, oq), qinverse(D.second(B.q, oq)));
+        angular(0, D.own(v3<double>(2.0 * aux.x, 2.0 * aux.y, 2.0 * aux.z)));
     } break;
     case CON_HINGE: {  // pbd.cpp:245-299
-        Acpd<R> A = acpd(a, b);
-        V3<R> dq = vcross(qaxis(wq<R>(a.q), C.a1), qaxis(wq<R>(b.q), C.a2));
-        R dl = ang_dlambda(A, h, (R)C.compliance, (R)lam[1], dq);
-        ang_apply(a, b, A, dl, dq);
-        lam[1] += (double)dl;
-        Pcpd<R> p = pcpd(a, b, r1, r2);
-        V3<R> dx = anchor_delta<R, EXACT>(a, b, p.r1, p.r2);
-        dl = pos_dlambda(a, b, p, h, (R)0, (R)lam[0], dx);
-        pos_apply(a, b, p, dl, dx);
-        lam[0] += (double)dl;
-        bool act = C.limited != 0;
-        if (act && !EXACT) {
-            const Qt<float> qa = qcast<float>(a.q), qb = qcast<float>(b.q);
-            act = limit_may_act(qaxis(qa, C.a1), qaxis(qa, C.l1), qaxis(qb, C.l2), C.lo, C.hi);
-        }
-        if (act) {
-            V3<double> n1 = qaxis(a.q, C.l1), n2 = qaxis(b.q, C.l2), n = qaxis(a.q, C.a1), dq64;
-            if (limit_angle<double>(n, n1, n2, C.lo, C.hi, dq64)) {
-                dq = v3cast<R>(dq64);
-                Acpd<R> B = acpd(a, b);
-                R dl2 = ang_dlambda(B, h, (R)0, (R)lam[2], dq);
-                ang_apply(a, b, B, dl2, dq);
-                lam[2] += (double)dl2;
-            }
+        V3<double> u1, u2;
+        axes(C.a1, C.a2, u1, u2);
+        angular(1, D.own(vcross(u1, u2)));
+        const V3<double> r = qrotate(B.q, r_lc), p = vadd(B.x, r);
+        positional(0, 0.0, r, vsub(p, D.other(p)));
+        if (C.limited) {
+            V3<double> n1, n2;
+            axes(C.l1, C.l2, n1, n2);
+            axes(C.a1, C.a2, u1, u2);
+            limit_solve(D, B, u1, n1, n2, C.lo, C.hi, h, lam + 2);
         }
     } break;
     case CON_SPHERICAL: {  // pbd.cpp:301-379
-        Pcpd<R> p = pcpd(a, b, r1, r2);
-        V3<R> dx = anchor_delta<R, EXACT>(a, b, p.r1, p.r2);
-        R dl = pos_dlambda(a, b, p, h, (R)0, (R)lam[0], dx);
-        pos_apply(a, b, p, dl, dx);
-        lam[0] += (double)dl;
-        // swing and twist limits: axes and angles in FP64 (see limit_angle), after an FP32 screen
         const double EPS64 = 1e-50;
-        bool swing = true, twist = true;
-        if (!EXACT) {
-            const Qt<float> qa = qcast<float>(a.q), qb = qcast<float>(b.q);
-            V3<float> f1 = qaxis(qa, C.a1), f2 = qaxis(qb, C.a2), fn = vcross(f1, f2);
-            const float fl = vlen(fn);
-            // limits at or beyond +-pi never act, however parallel the swing axes are
-            swing = !(C.lo <= -PI_REF && C.hi >= PI_REF) && (fl < 1e-3f || limit_may_act(vscale(1.f / fl, fn), f1, f2, C.lo, C.hi));
-        }
-        V3<double> n1 = qaxis(a.q, C.a1), n2 = qaxis(b.q, C.a2);
+        const V3<double> r = qrotate(B.q, r_lc), p = vadd(B.x, r);
+        positional(0, 0.0, r, vsub(p, D.other(p)));
+        V3<double> n1, n2;
+        axes(C.a1, C.a2, n1, n2);
         V3<double> n = vcross(n1, n2);
-        double nl = swing ? vlen(n) : 0.0;
-        if (nl > EPS64) {
-            n = v3<double>(n.x / nl, n.y / nl, n.z / nl);
-            V3<double> dq64;
-            if (limit_angle<double>(n, n1, n2, C.lo, C.hi, dq64)) {
-                V3<R> dq = v3cast<R>(dq64);
-                Acpd<R> A = acpd(a, b);
-                R d2 = ang_dlambda(A, h, (R)0, (R)lam[1], dq);
-                ang_apply(a, b, A, d2, dq);
-                lam[1] += (double)d2;
-            }
-        }
-        if (!EXACT) {   // screened on the orientations after the swing correction
-            const Qt<float> qa = qcast<float>(a.q), qb = qcast<float>(b.q);
-            V3<float> f1 = qaxis(qa, C.a1), f2 = qaxis(qb, C.a2);
-            V3<float> g1 = qaxis(qa, C.l1), g2 = qaxis(qb, C.l2), gn = vadd(f1, f2);
-            const float gl = vlen(gn);
-            const bool never = C.lo2 <= -PI_REF && C.hi2 >= PI_REF;
-            if (gl < 1e-3f) {
-                twist = !never;
-            } else {
-                gn = vscale(1.f / gl, gn);
-                V3<float> h1 = vsub(g1, vscale(vdot(gn, g1), gn)), h2 = vsub(g2, vscale(vdot(gn, g2), gn));
-                const float l1 = vlen(h1), l2 = vlen(h2);
-                twist = (l1 < 1e-3f || l2 < 1e-3f) ? !never
-                                                   : limit_may_act(gn, vscale(1.f / l1, h1), vscale(1.f / l2, h2), C.lo2, C.hi2);
-            }
-        }
-        V3<double> a1 = qaxis(a.q, C.a1), b1 = qaxis(a.q, C.l1);
-        V3<double> a2 = qaxis(b.q, C.a2), b2 = qaxis(b.q, C.l2);
+        double nl = vlen(n);
+        if (nl > EPS64) limit_solve(D, B, v3<double>(n.x / nl, n.y / nl, n.z / nl), n1, n2, C.lo, C.hi, h, lam + 1);
+        V3<double> a1, a2, b1, b2;   // on the orientations after the swing correction
+        axes(C.a1, C.a2, a1, a2);
+        axes(C.l1, C.l2, b1, b2);
         n = vadd(a1, a2);
-        nl = twist ? vlen(n) : 0.0;
+        nl = vlen(n);
         if (nl > EPS64) {
             n = v3<double>(n.x / nl, n.y / nl, n.z / nl);
             n1 = vsub(b1, vscale(vdot(n, b1), n));
             n2 = vsub(b2, vscale(vdot(n, b2), n));
-            double l1 = vlen(n1), l2 = vlen(n2);
-            if (l1 > EPS64 && l2 > EPS64) {
-                n1 = v3<double>(n1.x / l1, n1.y / l1, n1.z / l1);
-                n2 = v3<double>(n2.x / l2, n2.y / l2, n2.z / l2);
-                V3<double> dq64;
-                if (limit_angle<double>(n, n1, n2, C.lo2, C.hi2, dq64)) {
-                    V3<R> dq = v3cast<R>(dq64);
-                    Acpd<R> A = acpd(a, b);
-                    R d2 = ang_dlambda(A, h, (R)0, (R)lam[2], dq);
-                    ang_apply(a, b, A, d2, dq);
-                    lam[2] += (double)d2;
-                }
-            }
+            const double l1 = vlen(n1), l2 = vlen(n2);
+            if (l1 > EPS64 && l2 > EPS64)
+                limit_solve(D, B, n, v3<double>(n1.x / l1, n1.y / l1, n1.z / l1), v3<double>(n2.x / l2, n2.y / l2, n2.z / l2), C.lo2,
+                            C.hi2, h, lam + 2);
         }
     } break;
     default: break;
     }
-    store_pose(W, a);
-    store_pose(W, b);
+    store_pose(W, B);
 }
 
 // --------------------------------------------------------------------------------------------
@@ -401,7 +350,9 @@ struct FBody {
     float S[6];   // local inverse inertia, symmetric storage (xx yy zz xy xz yz)
     bool fixed;
     int idx;
-    __device__ __forceinline__ Qt<float> q() const { return qt<float>(q0f.x + dq.x, q0f.y + dq.y, q0f.z + dq.z, q0f.w + dq.w); }
+    __device__ __forceinline__ Qt<float> q() const {
+        return qt<float>(__fadd_rn(q0f.x, dq.x), __fadd_rn(q0f.y, dq.y), __fadd_rn(q0f.z, dq.z), __fadd_rn(q0f.w, dq.w));
+    }
 };
 
 __device__ __forceinline__ FBody load_fbody(const WorldView<float>& W, int b) {
@@ -424,35 +375,47 @@ __device__ __forceinline__ void store_fbody(const WorldView<float>& W, const FBo
     W.sdq[B.idx] = make_float4(B.dq.x, B.dq.y, B.dq.z, B.dq.w);
 }
 
-// (float)(x_a - x_b) of two bodies' predicted positions, as stored in pair_base / ext_base
+// (float)(x_a - x_b) of two bodies' predicted positions, as stored in pair_base
 __device__ __forceinline__ float4 fbase4(const WorldView<float>& W, int a, int b) {
     const double4_32a pa = W.pos[a], pb = W.pos[b];
     return make_float4((float)(pa.x - pb.x), (float)(pa.y - pb.y), (float)(pa.z - pb.z), 0.f);
 }
 
 
-// The position sweep's corrections into the FP64 pose (x += dx, q = normalize(q + dq)), and the
-// FP32 orientation copy the velocity sweep reads; bodies the sweep did not touch keep their pose.
-__device__ __forceinline__ void fold_body(const WorldView<float>& W, int b) {
-    const float4 d = W.sdx[b], q = W.sdq[b];
-    if (d.x == 0.f && d.y == 0.f && d.z == 0.f && q.x == 0.f && q.y == 0.f && q.z == 0.f && q.w == 0.f) return;
+// The position sweep's corrections d, q into the FP64 pose (x += dx, q = normalize(q + dq)), and the
+// FP32 orientation copy the velocity sweep reads (returned; q0 before); bodies the sweep did not touch keep
+// their pose.
+__device__ __forceinline__ float4 fold_pose(const WorldView<float>& W, int b, float4 d, float4 q, float4 q0) {
+    if (d.x == 0.f && d.y == 0.f && d.z == 0.f && q.x == 0.f && q.y == 0.f && q.z == 0.f && q.w == 0.f) return q0;
     const double4_32a p4 = W.pos[b], q4 = W.rot[b];
     const Qt<double> nq = qnormalize_fast(qt<double>(q4.x + (double)q.x, q4.y + (double)q.y, q4.z + (double)q.z,
                                                      q4.w + (double)q.w));
     W.pos[b] = make_double4_32a(p4.x + (double)d.x, p4.y + (double)d.y, p4.z + (double)d.z, 0.0);
     W.rot[b] = make_double4_32a(nq.x, nq.y, nq.z, nq.w);
-    W.pose_f[2 * b + 1] = make_float4((float)nq.x, (float)nq.y, (float)nq.z, (float)nq.w);
+    return make_float4((float)nq.x, (float)nq.y, (float)nq.z, (float)nq.w);
+}
+__device__ __forceinline__ void fold_body(const WorldView<float>& W, int b) {
+    W.pose_f[2 * b + 1] = fold_pose(W, b, W.sdx[b], W.sdq[b], W.pose_f[2 * b + 1]);
 }
 
+// JOINT in the functions below: the contact solve and the joint solves fuse some of their sums in
+// different order (the last step of frot_update, the y component of R^T v; the xy elements of a
+// contact's second body, D.second_right), and each keeps its own.
+
 // q <- normalize(q + inc), in delta form
+template <bool JOINT>
 __device__ __forceinline__ void frot_update(FBody& B, Qt<float> inc) {
-    Qt<float> u = qt<float>(B.dq.x + inc.x, B.dq.y + inc.y, B.dq.z + inc.z, B.dq.w + inc.w);
-    float e = 2.f * (B.q0f.x * u.x + B.q0f.y * u.y + B.q0f.z * u.z + B.q0f.w * u.w) + (u.x * u.x + u.y * u.y + u.z * u.z + u.w * u.w);
-    const float u1 = 1.f + e;   // |q0 + u|^2, close to 1
-    float s = u1 * rsqrtf(u1);
-    float rm1 = __fdividef(-e, s * (1.f + s));
-    float r = 1.f + rm1;
-    B.dq = qt<float>(B.q0f.x * rm1 + u.x * r, B.q0f.y * rm1 + u.y * r, B.q0f.z * rm1 + u.z * r, B.q0f.w * rm1 + u.w * r);
+    const Qt<float> u = qt<float>(__fadd_rn(B.dq.x, inc.x), __fadd_rn(B.dq.y, inc.y), __fadd_rn(B.dq.z, inc.z), __fadd_rn(B.dq.w, inc.w));
+    const float d = __fmaf_rn(B.q0f.w, u.w, sum3(B.q0f.x, u.x, B.q0f.y, u.y, B.q0f.z, u.z));
+    const float e = __fmaf_rn(2.f, d, __fmaf_rn(u.w, u.w, sum3(u.x, u.x, u.y, u.y, u.z, u.z)));
+    const float u1 = __fadd_rn(1.f, e);   // |q0 + u|^2, close to 1
+    const float s = __fmul_rn(u1, rsqrtf(u1));
+    const float rm1 = __fdividef(-e, __fmul_rn(s, __fadd_rn(1.f, s)));
+    const float r = __fadd_rn(1.f, rm1);
+    if (JOINT)
+        B.dq = qt<float>(sum2(B.q0f.x, rm1, u.x, r), sum2(u.y, r, B.q0f.y, rm1), sum2(u.z, r, B.q0f.z, rm1), sum2(u.w, r, B.q0f.w, rm1));
+    else
+        B.dq = qt<float>(sum2(B.q0f.x, rm1, u.x, r), sum2(B.q0f.y, rm1, u.y, r), sum2(B.q0f.z, rm1, u.z, r), sum2(B.q0f.w, rm1, u.w, r));
 }
 
 // FP32 delta-form arithmetic: unit vectors from the reciprocal square root of the special-function
@@ -460,13 +423,13 @@ __device__ __forceinline__ void frot_update(FBody& B, Qt<float> inc) {
 // division in the serial Gauss-Seidel chains; squared lengths at or below 1e-36 take the IEEE path
 // (rsqrtf flushes subnormal inputs).
 __device__ __forceinline__ float funit(V3<float> v, V3<float>& n) {
-    const float c2 = v.x * v.x + v.y * v.y + v.z * v.z;
+    const float c2 = dot_f(v, v);
     if (c2 > 1e-36f) {
         const float r = rsqrtf(c2);
-        n = v3<float>(v.x * r, v.y * r, v.z * r);
-        return c2 * r;
+        n = scale_f(r, v);
+        return __fmul_rn(c2, r);
     }
-    const float c = vlen(v);
+    const float c = sqrtf(c2);
     if (c > 0.f) n = v3<float>(v.x / c, v.y / c, v.z / c);
     return c;
 }
@@ -474,82 +437,81 @@ __device__ __forceinline__ float funit(V3<float> v, V3<float>& n) {
 // The world inverse inertia applied to v at the body's current orientation, R (S (R^T v)): the
 // products the reference forms with the world tensor R S R^T (physics_util.cpp:26-63), without
 // keeping the tensor itself live through the solve (the FP32 path's register budget).
-__device__ __forceinline__ V3<float> fIinv(const FBody& B, V3<float> v) {
-    const M3<float> R = qmat3(B.q());
-    const V3<float> l = v3<float>(R.d[0][0] * v.x + R.d[1][0] * v.y + R.d[2][0] * v.z,
-                                  R.d[0][1] * v.x + R.d[1][1] * v.y + R.d[2][1] * v.z,
-                                  R.d[0][2] * v.x + R.d[1][2] * v.y + R.d[2][2] * v.z);
-    const V3<float> t = v3<float>(B.S[0] * l.x + B.S[3] * l.y + B.S[4] * l.z, B.S[3] * l.x + B.S[1] * l.y + B.S[5] * l.z,
-                                  B.S[4] * l.x + B.S[5] * l.y + B.S[2] * l.z);
-    return mmulv(R, t);
+template <bool JOINT>
+__device__ __forceinline__ V3<float> fIinv(const Duo& D, const FBody& B, V3<float> v) {
+    const M3<float> R = mat3_f(B.q(), !JOINT && D.second_right);
+    const V3<float> l = v3<float>(sum3(R.d[0][0], v.x, R.d[1][0], v.y, R.d[2][0], v.z),
+                                  JOINT ? sum3(R.d[1][1], v.y, R.d[0][1], v.x, R.d[2][1], v.z)
+                                        : sum3(R.d[0][1], v.x, R.d[1][1], v.y, R.d[2][1], v.z),
+                                  sum3(R.d[0][2], v.x, R.d[1][2], v.y, R.d[2][2], v.z));
+    const V3<float> t = v3<float>(sum3(B.S[0], l.x, B.S[3], l.y, B.S[4], l.z), sum3(B.S[3], l.x, B.S[1], l.y, B.S[5], l.z),
+                                  sum3(B.S[4], l.x, B.S[5], l.y, B.S[2], l.z));
+    return mulv_f(R, t);
 }
 
-// calculate_positional_constraint_preprocessed_data on the FP32 path: the anchors in world axes (the
-// inertia products are taken by fIinv at the same orientations, before the correction moves them)
-struct FPcpd { V3<float> r1, r2; };
-__device__ __forceinline__ FPcpd fpcpd(const FBody& a, const FBody& b, V3<float> r1_lc, V3<float> r2_lc) {
-    FPcpd p;
-    p.r1 = qrotate(a.q(), r1_lc);
-    p.r2 = qrotate(b.q(), r2_lc);
-    return p;
+// the generalised inverse mass of this lane's body for a correction along unit n at anchor r
+template <bool JOINT>
+__device__ __forceinline__ float fmass(const Duo& D, const FBody& B, V3<float> r, V3<float> n) {
+    const V3<float> c = cross_f(r, n);
+    return __fadd_rn(B.invm, dot_f(c, fIinv<JOINT>(D, B, c)));
 }
 
-__device__ __forceinline__ float fpos_dlambda(const FBody& a, const FBody& b, const FPcpd& p, float lambda_til_free, V3<float> dx) {
-    (void)lambda_til_free;
+// the angular part of a correction: q <- normalize(q + (a, 0) q / 2)
+template <bool JOINT>
+__device__ __forceinline__ void fturn(FBody& B, V3<float> a) {
+    const Qt<float> q = qmul_pure_f(a, B.q());
+    if (!B.fixed) frot_update<JOINT>(B, qt<float>(0.5f * q.x, 0.5f * q.y, 0.5f * q.z, 0.5f * q.w));
+}
+
+__device__ __forceinline__ float fpos_dlambda(const Duo& D, const FBody& B, V3<float> r, V3<float> dx) {
     V3<float> n;
     const float c = funit(dx, n);
     if (c <= 0.f) return 0.f;
-    const V3<float> c1 = vcross(p.r1, n), c2 = vcross(p.r2, n);
-    float w1 = a.invm + vdot(c1, fIinv(a, c1));
-    float w2 = b.invm + vdot(c2, fIinv(b, c2));
-    return __fdividef(-c, w1 + w2);   // contacts carry zero compliance (pbd.cpp:123,133)
+    const float w = fmass<false>(D, B, r, n);
+    return __fdividef(-c, __fadd_rn(w, D.other(w)));   // contacts carry zero compliance (pbd.cpp:123,133)
 }
 
-__device__ __forceinline__ void fpos_apply(FBody& a, FBody& b, const FPcpd& p, float dl, V3<float> dx) {
+template <bool JOINT>
+__device__ __forceinline__ void fpos_apply(const Duo& D, FBody& B, V3<float> r, float dl, V3<float> dx) {
     V3<float> n;
     const float c = funit(dx, n);
     if (c <= 0.f) return;
-    V3<float> imp = vscale(dl, n);
-    if (!a.fixed) a.dx = vadd(a.dx, vscale(a.invm, imp));
-    if (!b.fixed) b.dx = vadd(b.dx, vscale(-b.invm, imp));
-    V3<float> a1 = fIinv(a, vcross(p.r1, imp));
-    V3<float> a2 = fIinv(b, vcross(p.r2, imp));
-    Qt<float> q1 = qmul(qt<float>(a1.x, a1.y, a1.z, 0.f), a.q());
-    Qt<float> q2 = qmul(qt<float>(a2.x, a2.y, a2.z, 0.f), b.q());
-    if (!a.fixed) frot_update(a, qt<float>(0.5f * q1.x, 0.5f * q1.y, 0.5f * q1.z, 0.5f * q1.w));
-    if (!b.fixed) frot_update(b, qt<float>(-0.5f * q2.x, -0.5f * q2.y, -0.5f * q2.z, -0.5f * q2.w));
+    const V3<float> imp = scale_f(dl, n);
+    if (!B.fixed) B.dx = axpy_f(B.invm, imp, B.dx);
+    fturn<JOINT>(B, fIinv<JOINT>(D, B, cross_f(r, imp)));
 }
 
-// collision_constraint_solve (pbd.cpp:107-154) on FP32 deltas; base_ab = (float)(x0_a - x0_b)
-static __device__ void fcollision_solve(const WorldView<float>& W, FBody& a, FBody& b, V3<float> base_ab, float* c, float mus) {
-    V3<float> r1 = v3<float>(c[0], c[1], c[2]), r2 = v3<float>(c[4], c[5], c[6]), n = v3<float>(c[8], c[9], c[10]);
-    float lambda_n = c[3], lambda_t = c[7];
-    FPcpd p = fpcpd(a, b, r1, r2);
-    V3<float> d12 = vadd(vadd(base_ab, vsub(a.dx, b.dx)), vsub(p.r1, p.r2));
-    float d = vdot(d12, n);
-    if (d > 0.f) {
-        V3<float> dx = vscale(d, n);
-        float dl = fpos_dlambda(a, b, p, 0.f, dx);
-        fpos_apply(a, b, p, dl, dx);
-        lambda_n += dl;
-        p = fpcpd(a, b, r1, r2);
-        dl = fpos_dlambda(a, b, p, 0.f, dx);
-        float lt = lambda_t + dl;
-        if (lt > mus * lambda_n) {
-            // displacement since the substep began: the predict step's (pred_d, FP32 from the FP64 poses)
-            // plus the sweep's; the previous orientations' FP32 copies (prev_qf)
-            const float4 pda = W.pred_d[a.idx], pdb = W.pred_d[b.idx], qa = W.prev_qf[a.idx], qb = W.prev_qf[b.idx];
-            Qt<float> qa_prev = qt<float>(qa.x, qa.y, qa.z, qa.w), qb_prev = qt<float>(qb.x, qb.y, qb.z, qb.w);
-            V3<float> da = vadd(vadd(v3<float>(pda.x, pda.y, pda.z), a.dx), vsub(p.r1, qrotate(qa_prev, r1)));
-            V3<float> db = vadd(vadd(v3<float>(pdb.x, pdb.y, pdb.z), b.dx), vsub(p.r2, qrotate(qb_prev, r2)));
-            V3<float> dp = vsub(da, db);
-            V3<float> dpt = vsub(dp, vscale(vdot(dp, n), n));
-            fpos_apply(a, b, p, dl, dpt);
-            lambda_t += dl;
-        }
+// collision_constraint_solve (pbd.cpp:107-154) on FP32 deltas. rl: this body's anchor and multiplier
+// (the first body's lane holds lambda_n, the second's lambda_t); n and base (the predicted positions'
+// difference) seen from this body; pred_d, prev_qf: the substep's displacement and previous orientation by
+// B.idx; returns this lane's multiplier.
+static __device__ float fcollision_solve(const float4* pred_d, const float4* prev_qf, const Duo& D, FBody& B, V3<float> base, float4 rl, V3<float> n,
+                                         float mus) {
+    const V3<float> r_lc = v3<float>(rl.x, rl.y, rl.z);
+    V3<float> r = rotate_f(B.q(), r_lc, true);
+    const V3<float> gap = add_f(add_f(base, sub_f(B.dx, D.other(B.dx))), sub_f(r, D.other(r)));
+    const float d = sum3(gap.y, n.y, gap.x, n.x, gap.z, n.z);
+    if (!(d > 0.f)) return rl.w;
+    const float lo = D.other(rl.w);
+    float lambda_n = D.first(rl.w, lo), lambda_t = D.second(rl.w, lo);
+    const V3<float> dx = scale_f(d, n);
+    float dl = fpos_dlambda(D, B, r, dx);
+    fpos_apply<false>(D, B, r, dl, dx);
+    lambda_n = __fadd_rn(lambda_n, dl);
+    r = rotate_f(B.q(), r_lc, D.second_right, D.second_right);
+    dl = fpos_dlambda(D, B, r, dx);
+    const float lt = __fadd_rn(lambda_t, dl);
+    if (lt > __fmul_rn(mus, lambda_n)) {
+        // displacement since the substep began: the predict step's (pred_d, FP32 from the FP64 poses)
+        // plus the sweep's; the previous orientation's FP32 copy (prev_qf)
+        const float4 pd = pred_d[B.idx], qp = prev_qf[B.idx];
+        const V3<float> u = add_f(add_f(v3<float>(pd.x, pd.y, pd.z), B.dx),
+                                  sub_f(r, rotate_f(qt<float>(qp.x, qp.y, qp.z, qp.w), r_lc)));
+        const V3<float> dp = sub_f(u, D.other(u));
+        fpos_apply<false>(D, B, r, dl, axpy_f(-dot_f(dp, n), n, dp));
+        lambda_t = lt;
     }
-    c[3] = lambda_n;
-    c[7] = lambda_t;
+    return D.side ? lambda_t : lambda_n;
 }
 
 // --------------------------------------------------------------------------------------------
@@ -557,76 +519,79 @@ static __device__ void fcollision_solve(const WorldView<float>& W, FBody& a, FBo
 // same order of corrections as ext_solve, each applied to the FP32 deltas; joint-limit angles are
 // screened in FP32 and evaluated in FP64 (from the FP64 orientation q0 + dq) where they may act.
 __device__ __forceinline__ float fdlambda(float c, float w1, float w2, float h, float compliance, float lambda) {
-    const float til = __fdividef(compliance, h * h);
-    return __fdividef(-c - til * lambda, w1 + w2 + til);
+    const float til = __fdividef(compliance, __fmul_rn(h, h));
+    return __fdividef(__fmaf_rn(-til, lambda, -c), __fadd_rn(__fadd_rn(w1, w2), til));
 }
 
-__device__ __forceinline__ float fpos_dlambda_c(const FBody& a, const FBody& b, const FPcpd& p, float h,
-                                                float compliance, float lambda, V3<float> dx) {
+__device__ __forceinline__ float fpos_dlambda_c(const Duo& D, const FBody& B, V3<float> r, float h, float compliance, float lambda,
+                                                V3<float> dx) {
     V3<float> n;
     const float c = funit(dx, n);
     if (c <= 0.f) return 0.f;
-    const V3<float> c1 = vcross(p.r1, n), c2 = vcross(p.r2, n);
-    const float w1 = a.invm + vdot(c1, fIinv(a, c1));
-    const float w2 = b.invm + vdot(c2, fIinv(b, c2));
-    return fdlambda(c, w1, w2, h, compliance, lambda);
+    const float w = fmass<true>(D, B, r, n);
+    return fdlambda(c, w, D.other(w), h, compliance, lambda);
 }
 
-// ang_dlambda on the FP32 path
-__device__ __forceinline__ float fang_dlambda(const FBody& a, const FBody& b, float h, float compliance, float lambda, V3<float> dq) {
+// angular corrections of this lane's body (pbd_base_constraints.cpp:125-227)
+__device__ __forceinline__ float fang_dlambda(const Duo& D, const FBody& B, float h, float compliance, float lambda, V3<float> dq) {
     V3<float> n;
     const float th = funit(dq, n);
     if (th <= 0.f) return 0.f;
-    return fdlambda(th, vdot(n, fIinv(a, n)), vdot(n, fIinv(b, n)), h, compliance, lambda);
+    const float w = dot_f(n, fIinv<true>(D, B, n));
+    return fdlambda(th, w, D.other(w), h, compliance, lambda);
 }
 
-__device__ __forceinline__ void fang_apply(FBody& a, FBody& b, float dl, V3<float> dq) {
+__device__ __forceinline__ void fang_apply(const Duo& D, FBody& B, float dl, V3<float> dq) {
     V3<float> n;
     const float th = funit(dq, n);
     if (th <= 0.f) return;
-    const V3<float> imp = vscale(-dl, n);
-    const V3<float> a1 = fIinv(a, imp), a2 = fIinv(b, imp);
-    const Qt<float> q1 = qmul(qt<float>(a1.x, a1.y, a1.z, 0.f), a.q());
-    const Qt<float> q2 = qmul(qt<float>(a2.x, a2.y, a2.z, 0.f), b.q());
-    if (!a.fixed) frot_update(a, qt<float>(0.5f * q1.x, 0.5f * q1.y, 0.5f * q1.z, 0.5f * q1.w));
-    if (!b.fixed) frot_update(b, qt<float>(-0.5f * q2.x, -0.5f * q2.y, -0.5f * q2.z, -0.5f * q2.w));
+    fturn<true>(B, fIinv<true>(D, B, scale_f(-dl, n)));
 }
 
-// the FP64 orientation of a body in delta form (the predicted FP64 orientation plus the sweep's delta)
-__device__ __forceinline__ Qt<double> fq64(const WorldView<float>& W, const FBody& B) {
-    const double4_32a q = W.rot[B.idx];
-    return qt<double>(q.x + (double)B.dq.x, q.y + (double)B.dq.y, q.z + (double)B.dq.z, q.w + (double)B.dq.w);
-}
+// What the FP32 solve of one joint reads of it, besides its bodies: the axes and limits, this lane's body's
+// anchor, and the difference of the predicted positions (minus the rest offset of a positional joint).
+struct JointF {
+    int type, a1, a2, l1, l2;
+    bool limited;
+    float compliance;
+    V3<float> r1, r2, base;
+    double lo, hi, lo2, hi2;
+};
 
-// angular correction of one joint limit (limit_angle's dq, FP64) on the deltas
-__device__ __forceinline__ void flimit_apply(FBody& a, FBody& b, V3<double> dq64, float h, float* lam) {
-    const V3<float> dq = v3cast<float>(dq64);
-    V3<float> n;
-    const float th = funit(dq, n);
-    if (th <= 0.f) return;
-    const float dl = fdlambda(th, vdot(n, fIinv(a, n)), vdot(n, fIinv(b, n)), h, 0.f, *lam);
-    fang_apply(a, b, dl, dq);
-    *lam += dl;
+// A joint as the solve kernels stage it: the FP32 operands rounded at upload, and the position difference
+// formed in FP64 and rounded once per substep (the poses do not change during the position sweep).
+__device__ __forceinline__ JointF load_joint(const WorldView<float>& W, const ExtConstraint& C) {
+    JointF j;
+    j.type = C.type;
+    j.a1 = C.a1; j.a2 = C.a2; j.l1 = C.l1; j.l2 = C.l2;
+    j.limited = C.limited != 0;
+    j.compliance = C.compliance_f;
+    j.r1 = v3<float>(C.r1f[0], C.r1f[1], C.r1f[2]);
+    j.r2 = v3<float>(C.r2f[0], C.r2f[1], C.r2f[2]);
+    j.lo = C.lo; j.hi = C.hi; j.lo2 = C.lo2; j.hi2 = C.hi2;
+    const double4_32a pa = W.pos[C.e1], pb = W.pos[C.e2];
+    double x = pa.x - pb.x, y = pa.y - pb.y, z = pa.z - pb.z;
+    if (C.type == CON_POSITIONAL) { x -= C.distance[0]; y -= C.distance[1]; z -= C.distance[2]; }
+    j.base = v3<float>((float)x, (float)y, (float)z);
+    return j;
 }
 
 // FP64 evaluation of a joint limit that the FP32 screen could not rule out (rare): kind 0 the hinge
 // limit (pbd.cpp:279-298), 1 the spherical swing limit, 2 the spherical twist limit (pbd.cpp:327-378),
-// each from the FP64 orientations q0 + dq, applying its correction to a and b. Out of line, so that
-// the joint solve's common path keeps its values in registers.
-static __device__ __noinline__ void flimit64(const WorldView<float>& W, FBody& a, FBody& b, const ExtConstraint& C, float h,
-                                             float* lam, int kind) {
+// from the FP64 orientations q0 + dq of the first and the second body; true with the correction dq as
+// the first body sees it. Out of line, so that the joint solve's common path keeps its values in
+// registers; both lanes of a pair evaluate it on the same values.
+static __device__ __noinline__ bool flimit64(Qt<double> qa, Qt<double> qb, const JointF& C, int kind, V3<float>& dq) {
     const double EPS64 = 1e-50;
-    const Qt<double> qa = fq64(W, a), qb = fq64(W, b);
     V3<double> dq64;
+    bool act = false;
     if (kind == 0) {
-        if (limit_angle<double>(qaxis(qa, C.a1), qaxis(qa, C.l1), qaxis(qb, C.l2), C.lo, C.hi, dq64))
-            flimit_apply(a, b, dq64, h, &lam[2]);
+        act = limit_angle<double>(qaxis(qa, C.a1), qaxis(qa, C.l1), qaxis(qb, C.l2), C.lo, C.hi, dq64);
     } else if (kind == 1) {
         const V3<double> n1 = qaxis(qa, C.a1), n2 = qaxis(qb, C.a2);
         const V3<double> n = vcross(n1, n2);
         const double nl = vlen(n);
-        if (nl > EPS64 && limit_angle<double>(v3<double>(n.x / nl, n.y / nl, n.z / nl), n1, n2, C.lo, C.hi, dq64))
-            flimit_apply(a, b, dq64, h, &lam[1]);
+        act = nl > EPS64 && limit_angle<double>(v3<double>(n.x / nl, n.y / nl, n.z / nl), n1, n2, C.lo, C.hi, dq64);
     } else {
         const V3<double> a1 = qaxis(qa, C.a1), b1 = qaxis(qa, C.l1), a2 = qaxis(qb, C.a2), b2 = qaxis(qb, C.l2);
         V3<double> n = vadd(a1, a2);
@@ -635,102 +600,122 @@ static __device__ __noinline__ void flimit64(const WorldView<float>& W, FBody& a
             n = v3<double>(n.x / nl, n.y / nl, n.z / nl);
             const V3<double> n1 = vsub(b1, vscale(vdot(n, b1), n)), n2 = vsub(b2, vscale(vdot(n, b2), n));
             const double l1 = vlen(n1), l2 = vlen(n2);
-            if (l1 > EPS64 && l2 > EPS64 &&
-                limit_angle<double>(n, v3<double>(n1.x / l1, n1.y / l1, n1.z / l1), v3<double>(n2.x / l2, n2.y / l2, n2.z / l2),
-                                    C.lo2, C.hi2, dq64))
-                flimit_apply(a, b, dq64, h, &lam[2]);
+            act = l1 > EPS64 && l2 > EPS64 &&
+                  limit_angle<double>(n, v3<double>(n1.x / l1, n1.y / l1, n1.z / l1), v3<double>(n2.x / l2, n2.y / l2, n2.z / l2),
+                                      C.lo2, C.hi2, dq64);
         }
     }
+    if (act) dq = v3cast<float>(dq64);
+    return act;
 }
 
-// lam: the joint's Lagrange multipliers of the substep as FP32 (they start at zero every substep and
-// enter only through compliance, zero for the joints of the workloads); base: (float)(x_e1 - x_e2)
-// of the predicted positions, rounded once per substep by the cull.
-static __device__ void fext_solve(const WorldView<float>& W, const ExtConstraint& C, float4 base, float* lam, float h) {
-    FBody a = load_fbody(W, C.e1), b = load_fbody(W, C.e2);
-    const V3<float> r1 = v3<float>(C.r1f[0], C.r1f[1], C.r1f[2]);
-    const V3<float> r2 = v3<float>(C.r2f[0], C.r2f[1], C.r2f[2]);
-    const V3<float> base_ab = v3<float>(base.x, base.y, base.z);
-    auto anchor = [&](const FPcpd& p) { return vadd(vadd(base_ab, vsub(a.dx, b.dx)), vsub(p.r1, p.r2)); };
+// an axis of a body in world coordinates, FP32 with its roundings spelled out (qaxis)
+__device__ __forceinline__ V3<float> axis_f(Qt<float> q, int axis) {
+    const float x2 = 2.f * q.x, y2 = 2.f * q.y, z2 = 2.f * q.z, w = axis & 1 ? q.w : -q.w, w2 = 2.f * w;
+    if (axis < 2) return v3<float>(__fmaf_rn(-z2, q.z, __fmaf_rn(-y2, q.y, 1.f)), dif2(x2, q.y, w2, q.z), sum2(x2, q.z, w2, q.y));
+    if (axis < 4) return v3<float>(sum2(x2, q.y, w2, q.z), __fmaf_rn(-z2, q.z, __fmaf_rn(-x2, q.x, 1.f)), dif2(y2, q.z, w2, q.x));
+    return v3<float>(dif2(x2, q.z, w2, q.y), sum2(y2, q.z, w2, q.x), __fmaf_rn(-y2, q.y, __fmaf_rn(-x2, q.x, 1.f)));
+}
+
+// One joint on this lane's body B. rot: the body's predicted FP64 orientation (read only where a limit
+// has to be decided in FP64). lam: the joint's Lagrange multipliers of the substep as FP32 (they start at
+// zero every substep and enter only through compliance): zero in its first sweep; both lanes hold them.
+static __device__ void fext_solve(const Duo& D, FBody& B, const double4_32a* rot, const JointF& C, float (&lam)[3], float h) {
+    const V3<float> r_lc = D.side ? C.r2 : C.r1;
+    const V3<float> base = D.own(C.base);
+    // one positional correction along dx at anchor r
+    auto positional = [&](float compliance, V3<float> r, V3<float> dx) {
+        const float dl = fpos_dlambda_c(D, B, r, h, compliance, lam[0], dx);
+        fpos_apply<true>(D, B, r, dl, dx);
+        lam[0] = __fadd_rn(lam[0], dl);
+    };
+    auto angular = [&](float& l, float compliance, V3<float> dq) {
+        const float dl = fang_dlambda(D, B, h, compliance, l, dq);
+        fang_apply(D, B, dl, dq);
+        l = __fadd_rn(l, dl);
+    };
+    // the anchors coincide (pbd.cpp:265-276, 303-314)
+    auto attach = [&]() {
+        const V3<float> r = rotate_f(B.q(), r_lc);
+        positional(0.f, r, add_f(add_f(base, sub_f(B.dx, D.other(B.dx))), sub_f(r, D.other(r))));
+    };
+    // an axis of the first and of the second body, in both lanes
+    auto axes = [&](int k1, int k2, V3<float>& u1, V3<float>& u2) {
+        const V3<float> mine = axis_f(B.q(), D.side ? k2 : k1), theirs = D.other(mine);
+        u1 = D.first(mine, theirs);
+        u2 = D.second(mine, theirs);
+    };
+    // a limit the FP32 screen could not rule out
+    auto limit = [&](int kind) {
+        const double4_32a q4 = *rot;
+        const Qt<double> q = qt<double>(q4.x + (double)B.dq.x, q4.y + (double)B.dq.y, q4.z + (double)B.dq.z, q4.w + (double)B.dq.w);
+        const Qt<double> o = D.other(q);
+        V3<float> dq;
+        const JointF c = C;   // a copy: the call takes an address, which would keep the joint in local memory
+        if (flimit64(D.first(q, o), D.second(q, o), c, kind, dq)) angular(kind == 1 ? lam[1] : lam[2], 0.f, D.own(dq));
+    };
     switch (C.type) {
-    case CON_POSITIONAL: {  // pbd.cpp:81-97
-        const double4_32a pa = W.pos[C.e1], pb = W.pos[C.e2];
-        const V3<float> base = v3<float>((float)((pa.x - pb.x) - C.distance[0]), (float)((pa.y - pb.y) - C.distance[1]),
-                                         (float)((pa.z - pb.z) - C.distance[2]));
-        const V3<float> dx = vadd(base, vsub(a.dx, b.dx));
-        const FPcpd p = fpcpd(a, b, r1, r2);
-        const float dl = fpos_dlambda_c(a, b, p, h, C.compliance_f, lam[0], dx);
-        fpos_apply(a, b, p, dl, dx);
-        lam[0] += dl;
-    } break;
+    case CON_POSITIONAL:   // pbd.cpp:81-97
+        positional(C.compliance, rotate_f(B.q(), r_lc), add_f(base, sub_f(B.dx, D.other(B.dx))));
+        break;
     case CON_MUTUAL_ORIENTATION: {  // pbd.cpp:156-173
-        const Qt<float> aux = qmul(a.q(), qinverse(b.q()));
-        const V3<float> dq = v3<float>(2.f * aux.x, 2.f * aux.y, 2.f * aux.z);
-        const float dl = fang_dlambda(a, b, h, C.compliance_f, lam[0], dq);
-        fang_apply(a, b, dl, dq);
-        lam[0] += dl;
+        const Qt<float> mq = B.q(), oq = D.other(mq);
+        const Qt<float> aux = qmul(D.first(mq, oq), qinverse(D.second(mq, oq)));
+        angular(lam[0], C.compliance, D.own(v3<float>(2.f * aux.x, 2.f * aux.y, 2.f * aux.z)));
     } break;
     case CON_HINGE: {  // pbd.cpp:245-299
-        const V3<float> dq = vcross(qaxis(a.q(), C.a1), qaxis(b.q(), C.a2));
-        float dl = fang_dlambda(a, b, h, C.compliance_f, lam[1], dq);
-        fang_apply(a, b, dl, dq);
-        lam[1] += dl;
-        const FPcpd p = fpcpd(a, b, r1, r2);
-        const V3<float> dx = anchor(p);
-        dl = fpos_dlambda_c(a, b, p, h, 0.f, lam[0], dx);
-        fpos_apply(a, b, p, dl, dx);
-        lam[0] += dl;
-        if (C.limited && limit_may_act(qaxis(a.q(), C.a1), qaxis(a.q(), C.l1), qaxis(b.q(), C.l2), C.lo, C.hi)) {
-            flimit64(W, a, b, C, h, lam, 0);
+        V3<float> u1, u2;
+        axes(C.a1, C.a2, u1, u2);
+        angular(lam[1], C.compliance, D.own(cross_f(u1, u2)));
+        attach();
+        if (C.limited) {
+            V3<float> n1, n2;
+            axes(C.a1, C.a2, u1, u2);
+            axes(C.l1, C.l2, n1, n2);
+            if (limit_may_act(u1, n1, n2, C.lo, C.hi)) limit(0);
         }
     } break;
     case CON_SPHERICAL: {  // pbd.cpp:301-379
-        const FPcpd p = fpcpd(a, b, r1, r2);
-        const V3<float> dx = anchor(p);
-        const float dl = fpos_dlambda_c(a, b, p, h, 0.f, lam[0], dx);
-        fpos_apply(a, b, p, dl, dx);
-        lam[0] += dl;
-        {   // swing
-            const V3<float> f1 = qaxis(a.q(), C.a1), f2 = qaxis(b.q(), C.a2), fn = vcross(f1, f2);
+        attach();
+        if (!(C.lo <= -PI_REF && C.hi >= PI_REF)) {   // swing; limits at or beyond +-pi never act
+            V3<float> f1, f2;
+            axes(C.a1, C.a2, f1, f2);
+            const V3<float> fn = vcross(f1, f2);
             const float fl = vlen(fn);
-            const bool never = C.lo <= -PI_REF && C.hi >= PI_REF;   // limits at or beyond +-pi never act
-            if (!never && (fl < 1e-3f || limit_may_act(vscale(1.f / fl, fn), f1, f2, C.lo, C.hi))) {
-                flimit64(W, a, b, C, h, lam, 1);
-            }
+            if (fl < 1e-3f || limit_may_act(vscale(1.f / fl, fn), f1, f2, C.lo, C.hi)) limit(1);
         }
-        {   // twist, on the orientations after the swing correction
-            const V3<float> f1 = qaxis(a.q(), C.a1), f2 = qaxis(b.q(), C.a2);
-            const V3<float> g1 = qaxis(a.q(), C.l1), g2 = qaxis(b.q(), C.l2);
+        if (!(C.lo2 <= -PI_REF && C.hi2 >= PI_REF)) {   // twist, on the orientations after the swing correction
+            V3<float> f1, f2, g1, g2;
+            axes(C.a1, C.a2, f1, f2);
+            axes(C.l1, C.l2, g1, g2);
             V3<float> gn = vadd(f1, f2);
             const float gl = vlen(gn);
-            const bool never = C.lo2 <= -PI_REF && C.hi2 >= PI_REF;
-            bool act;
-            if (gl < 1e-3f) {
-                act = !never;
-            } else {
+            bool act = true;
+            if (gl >= 1e-3f) {
                 gn = vscale(1.f / gl, gn);
                 const V3<float> h1 = vsub(g1, vscale(vdot(gn, g1), gn)), h2 = vsub(g2, vscale(vdot(gn, g2), gn));
                 const float l1 = vlen(h1), l2 = vlen(h2);
-                act = (l1 < 1e-3f || l2 < 1e-3f) ? !never
-                                                 : limit_may_act(gn, vscale(1.f / l1, h1), vscale(1.f / l2, h2), C.lo2, C.hi2);
+                act = l1 < 1e-3f || l2 < 1e-3f || limit_may_act(gn, vscale(1.f / l1, h1), vscale(1.f / l2, h2), C.lo2, C.hi2);
             }
-            if (act) flimit64(W, a, b, C, h, lam, 2);
+            if (act) limit(2);
         }
     } break;
     default: break;
     }
-    store_fbody(W, a);
-    store_fbody(W, b);
 }
 
 // FP32 build: after predict, the FP32 copies the substep's sweeps work from (the pose, the predict
-// step's displacement and the previous orientation) and zero sweep deltas.
+// step's displacement and the previous orientation) and, for the sweeps that keep them in global memory
+// (DELTAS), zero sweep deltas.
+template <bool DELTAS = true>
 __device__ __forceinline__ void stage_body(const WorldView<float>& W, int b) {
     const double4_32a p = W.pos[b], q = W.rot[b], pp = W.prev_pos[b], pq = W.prev_rot[b];
     W.pose_f[2 * b] = make_float4((float)p.x, (float)p.y, (float)p.z, 0.f);
     W.pose_f[2 * b + 1] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
-    W.sdx[b] = make_float4(0.f, 0.f, 0.f, 0.f);
-    W.sdq[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (DELTAS) {
+        W.sdx[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+        W.sdq[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     W.pred_d[b] = make_float4((float)(p.x - pp.x), (float)(p.y - pp.y), (float)(p.z - pp.z), 0.f);
     W.prev_qf[b] = make_float4((float)pq.x, (float)pq.y, (float)pq.z, (float)pq.w);
 }
@@ -805,40 +790,75 @@ __device__ void velocity_body(const WorldView<R>& W, int b, double h) {
     W.omega[3 * b] = sgn * dq.x; W.omega[3 * b + 1] = sgn * dq.y; W.omega[3 * b + 2] = sgn * dq.z;
 }
 
-// Velocity solver for one contact (pbd.cpp:646-711); velocities of the two bodies are in registers.
-// p: the contact's preprocessed data from the current poses (anchors in world orientation, world
-// inverse inertias); a / b: inverse mass and fixed flag of the two bodies.
-template <typename R>
-struct VelBody { R invm; bool fixed; };
+// world_tensor with its roundings spelled out
+__device__ __forceinline__ M3<float> world_tensor_f(Qt<float> q, const float S[6]) {
+    const M3<float> r = mat3_f(q);
+    M3<float> x, o;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        x.d[i][0] = sum3(r.d[i][0], S[0], r.d[i][1], S[3], r.d[i][2], S[4]);
+        x.d[i][1] = sum3(r.d[i][0], S[3], r.d[i][1], S[1], r.d[i][2], S[5]);
+        x.d[i][2] = sum3(r.d[i][0], S[4], r.d[i][1], S[5], r.d[i][2], S[2]);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) o.d[i][j] = sum3(x.d[i][0], r.d[j][0], x.d[i][1], r.d[j][1], x.d[i][2], r.d[j][2]);
+    return o;
+}
 
-template <typename R, bool EXACT>
-__device__ void contact_velocity(const Pcpd<R>& p, VelBody<R> a, VelBody<R> b, const R* c, R h, R mud, R e,
-                                 V3<R>& va, V3<R>& wa, V3<R>& vb, V3<R>& wb, V3<R> pva, V3<R> pwa, V3<R> pvb, V3<R> pwb) {
-    V3<R> n = v3<R>(c[8], c[9], c[10]);
-    R lambda_n = c[3];
-    V3<R> v = vsub(vadd(va, vcross(wa, p.r1)), vadd(vb, vcross(wb, p.r2)));
-    R vn = vdot(n, v);
-    V3<R> vt = vsub(v, vscale(vn, n));
+// contact_velocity (below) in FP32 with its roundings spelled out
+__device__ __forceinline__ void fcontact_velocity(const Duo& D, V3<float> r, const M3<float>& I, V3<float> n, float invm, bool fixed,
+                                                  float lambda_n, float h, float mud, float e, V3<float>& vel, V3<float>& om,
+                                                  V3<float> pv, V3<float> pw) {
+    const V3<float> u = add_f(vel, cross_f(om, r));
+    const V3<float> v = sub_f(u, D.other(u));
+    const float vn = dot_f(n, v);
+    const V3<float> vt = axpy_f(-vn, n, v);
+    const float fn = lambda_n / h;
+    const float x1 = __fmul_rn(mud, fabsf(fn)), x2 = sqrtf(dot_f(vt, vt));
+    float fact = (x1 < x2) ? x1 : x2;
+    V3<float> dv = v3<float>(0.f, 0.f, 0.f);
+    if (vt.x != 0.f || vt.y != 0.f || vt.z != 0.f) dv = scale_f(-fact, v3<float>(vt.x / x2, vt.y / x2, vt.z / x2));
+    const V3<float> ut = add_f(pv, cross_f(pw, r));
+    const float vntil = dot_f(n, sub_f(ut, D.other(ut)));
+    const float m = __fmul_rn(-e, vntil);
+    fact = __fadd_rn(-vn, (m < 0.f) ? m : 0.f);
+    dv = axpy_f(fact, n, dv);
+    const V3<float> c = cross_f(r, n);
+    const float w = __fadd_rn(invm, dot_f(c, mulv_f(I, c)));
+    const V3<float> P = scale_f(1.0f / __fadd_rn(w, D.other(w)), dv);
+    if (!fixed) {
+        vel = D.side ? add_f(vel, scale_f(invm, P)) : axpy_f(invm, P, vel);
+        om = add_f(om, mulv_f(I, cross_f(r, P)));
+    }
+}
+
+// Velocity solver for one contact (pbd.cpp:646-711) of this lane's body: v, w its velocities, pv, pw
+// those before the velocity update, r its anchor in world orientation, I its world inverse inertia, n
+// the normal seen from it.
+template <typename R>
+__device__ __forceinline__ void contact_velocity(const Duo& D, V3<R> r, const M3<R>& I, V3<R> n, R invm, bool fixed, R lambda_n, R h,
+                                                 R mud, R e, V3<R>& vel, V3<R>& om, V3<R> pv, V3<R> pw) {
+    const V3<R> u = vadd(vel, vcross(om, r));
+    const V3<R> v = vsub(u, D.other(u));
+    const R vn = vdot(n, v);
+    const V3<R> vt = vsub(v, vscale(vn, n));
     V3<R> dv = v3<R>(0, 0, 0);
-    R fn = lambda_n / h;
-    R x1 = mud * fabs(fn), x2 = vlen(vt);
+    const R fn = lambda_n / h;
+    const R x1 = mud * fabs(fn), x2 = vlen(vt);
     R fact = (x1 < x2) ? x1 : x2;
     dv = vadd(dv, vscale(-fact, vnorm(vt)));
-    V3<R> vtil = vsub(vadd(pva, vcross(pwa, p.r1)), vadd(pvb, vcross(pwb, p.r2)));
-    R vntil = vdot(n, vtil);
-    R m = -e * vntil;
+    const V3<R> ut = vadd(pv, vcross(pw, r));
+    const R vntil = vdot(n, vsub(ut, D.other(ut)));
+    const R m = -e * vntil;
     fact = -vn + ((m < (R)0.0) ? m : (R)0.0);
     dv = vadd(dv, vscale(fact, n));
-    R w1 = a.invm + vdot(vcross(p.r1, n), mmulv(p.I1, vcross(p.r1, n)));
-    R w2 = b.invm + vdot(vcross(p.r2, n), mmulv(p.I2, vcross(p.r2, n)));
-    V3<R> P = vscale((R)1.0 / (w1 + w2), dv);
-    if (!a.fixed) {
-        va = vadd(va, vscale(a.invm, P));
-        wa = vadd(wa, mmulv(p.I1, vcross(p.r1, P)));
-    }
-    if (!b.fixed) {
-        vb = vadd(vb, vinv(vscale(b.invm, P)));
-        wb = vadd(wb, vinv(mmulv(p.I2, vcross(p.r2, P))));
+    const R w = invm + vdot(vcross(r, n), mmulv(I, vcross(r, n)));
+    const V3<R> P = vscale((R)1.0 / (w + D.other(w)), dv);
+    if (!fixed) {
+        vel = vadd(vel, vscale(invm, P));
+        om = vadd(om, mmulv(I, vcross(r, P)));
     }
 }
 

@@ -1142,95 +1142,160 @@ __device__ void narrowphase(const WorldView<R>& W, const G& g, int s, NarrowSmem
 
 // ---------------------------------------------------------------------------------------------
 // Level sweeps
-template <typename R, bool EXACT>
-__device__ void solve_node(const WorldView<R>& W, int s, int k, R h) {
+// FP32 build: one node by a lane pair (both lanes call these together)
+__device__ inline void fsolve_node(const WorldView<float>& W, const Duo& D, int s, int k, float h) {
     const int e0 = W.scene_ext[s], ne = W.scene_ext[s + 1] - e0;
     if (k < ne) {
-        if constexpr (EXACT) ext_solve<R, EXACT>(W, W.ext[e0 + k], W.ext_lambda + 4 * (size_t)(e0 + k), h);
-        else fext_solve(W, W.ext[e0 + k], W.ext_base[e0 + k], reinterpret_cast<float*>(W.ext_lambda + 4 * (size_t)(e0 + k)), h);
+        const ExtConstraint& C = W.ext[e0 + k];
+        float* lam = reinterpret_cast<float*>(W.ext_lambda + 4 * (size_t)(e0 + k));
+        const JointF j = load_joint(W, C);
+        const int me = D.side ? C.e2 : C.e1;
+        FBody B = load_fbody(W, me);
+        float l[3] = {lam[0], lam[1], lam[2]};
+        __syncwarp(D.mask);
+        fext_solve(D, B, W.rot + me, j, l, h);
+        if (D.side == 0) { lam[0] = l[0]; lam[1] = l[1]; lam[2] = l[2]; }
+        store_fbody(W, B);
         return;
     }
     const int p = W.scene_pair_cap[s] + (k - ne);
     const int nc = W.pair_ccount[p];
     if (nc == 0) return;
-    int2 pr = W.pairs[p];
-    const R mus = (W.material[4 * pr.x] + W.material[4 * pr.y]) / (R)2.0f;
-    R* c = W.contacts + 12 * (size_t)(W.scene_contact_cap[s] + W.pair_cstart[p]);
-    if constexpr (EXACT) {
-        Body<R> a = load_body(W, pr.x), b = load_body(W, pr.y);
-        for (int i = 0; i < nc; ++i) collision_solve<R, EXACT>(W, a, b, c + 12 * i, h, mus);
-        store_pose(W, a);
-        store_pose(W, b);
-    } else {
-        FBody a = load_fbody(W, pr.x), b = load_fbody(W, pr.y);
-        const float4 bb = W.pair_base[p];
-        const V3<float> base_ab = v3<float>(bb.x, bb.y, bb.z);
-        for (int i = 0; i < nc; ++i) fcollision_solve(W, a, b, base_ab, c + 12 * i, mus);
-        store_fbody(W, a);
-        store_fbody(W, b);
+    const int2 pr = W.pairs[p];
+    const int me = D.side ? pr.y : pr.x;
+    const float mus_own = W.material[4 * me];
+    const float mus = __fadd_rn(mus_own, D.other(mus_own)) / 2.0f;
+    float* c = W.contacts + 12 * (size_t)(W.scene_contact_cap[s] + W.pair_cstart[p]);
+    FBody B = load_fbody(W, me);
+    const float4 bb = W.pair_base[p];
+    const V3<float> base = D.own(v3<float>(bb.x, bb.y, bb.z));
+    // the next contact's record is fetched while the current one is solved
+    const float4* c4 = reinterpret_cast<const float4*>(c);
+    float4 rl = c4[D.side], nn = c4[2];
+    for (int i = 0; i < nc; ++i) {
+        const float4 r0 = rl;
+        const V3<float> n = D.own(v3<float>(nn.x, nn.y, nn.z));
+        if (i + 1 < nc) { rl = c4[3 * (i + 1) + D.side]; nn = c4[3 * (i + 1) + 2]; }
+        const float lam = fcollision_solve(W.pred_d, W.prev_qf, D, B, base, r0, n, mus);
+        if (lam != r0.w) c[12 * i + 4 * D.side + 3] = lam;
     }
+    store_fbody(W, B);
 }
 
-template <typename R, bool EXACT>
-__device__ void vsolve_node(const WorldView<R>& W, int s, int k, R h) {
+__device__ inline void fvsolve_node(const WorldView<float>& W, const Duo& D, int s, int k, float h) {
     const int ne = W.scene_ext[s + 1] - W.scene_ext[s];
     if (k < ne) return;
     const int p = W.scene_pair_cap[s] + (k - ne);
     const int nc = W.pair_ccount[p];
     if (nc == 0) return;
-    int2 pr = W.pairs[p];
-    const int ia = pr.x, ib = pr.y;
-    // anchors rotated by the current orientations (the FP32 build converts each orientation once)
-    Qt<R> qa, qb;
-    M3<R> Ia, Ib;
-    VelBody<R> a, b;
-    {
-        if constexpr (EXACT) {
-            double4_32a q4a = W.rot[ia], q4b = W.rot[ib];
-            qa = qcast<R>(qt<double>(q4a.x, q4a.y, q4a.z, q4a.w));
-            qb = qcast<R>(qt<double>(q4b.x, q4b.y, q4b.z, q4b.w));
-        } else {   // the FP32 copies the fold wrote: the same casts of the FP64 orientations
-            const float4 fa = W.pose_f[2 * ia + 1], fb = W.pose_f[2 * ib + 1];
-            qa = qt<R>(fa.x, fa.y, fa.z, fa.w);
-            qb = qt<R>(fb.x, fb.y, fb.z, fb.w);
-        }
-        R sa[6], sb[6];
+    const int2 pr = W.pairs[p];
+    const int me = D.side ? pr.y : pr.x;
+    // anchors rotated by the current orientation (the FP32 copy the fold wrote; the poses do not change here)
+    const float4 f = W.pose_f[2 * me + 1];
+    const Qt<float> q = qt<float>(f.x, f.y, f.z, f.w);
+    float S[6];
 #pragma unroll
-        for (int i = 0; i < 6; ++i) { sa[i] = W.inv_inertia[6 * ia + i]; sb[i] = W.inv_inertia[6 * ib + i]; }
-        Ia = world_tensor(qa, msym(sa));
-        Ib = world_tensor(qb, msym(sb));
-        a.invm = W.inv_mass[ia];
-        b.invm = W.inv_mass[ib];
-        a.fixed = W.fixed[ia] != 0;
-        b.fixed = W.fixed[ib] != 0;
-    }
-    V3<R> va = v3<R>(W.vel[3 * ia], W.vel[3 * ia + 1], W.vel[3 * ia + 2]);
-    V3<R> wa = v3<R>(W.omega[3 * ia], W.omega[3 * ia + 1], W.omega[3 * ia + 2]);
-    V3<R> vb = v3<R>(W.vel[3 * ib], W.vel[3 * ib + 1], W.vel[3 * ib + 2]);
-    V3<R> wb = v3<R>(W.omega[3 * ib], W.omega[3 * ib + 1], W.omega[3 * ib + 2]);
-    V3<R> pva = v3<R>(W.prev_vel[3 * ia], W.prev_vel[3 * ia + 1], W.prev_vel[3 * ia + 2]);
-    V3<R> pwa = v3<R>(W.prev_omega[3 * ia], W.prev_omega[3 * ia + 1], W.prev_omega[3 * ia + 2]);
-    V3<R> pvb = v3<R>(W.prev_vel[3 * ib], W.prev_vel[3 * ib + 1], W.prev_vel[3 * ib + 2]);
-    V3<R> pwb = v3<R>(W.prev_omega[3 * ib], W.prev_omega[3 * ib + 1], W.prev_omega[3 * ib + 2]);
-    const R mud = (W.material[4 * ia + 1] + W.material[4 * ib + 1]) / (R)2.0f;
-    const R e = W.material[4 * ia + 2] * W.material[4 * ib + 2];
-    const R* c = W.contacts + 12 * (size_t)(W.scene_contact_cap[s] + W.pair_cstart[p]);
+    for (int i = 0; i < 6; ++i) S[i] = W.inv_inertia[6 * me + i];
+    const M3<float> I = world_tensor_f(q, S);
+    const float invm = W.inv_mass[me];
+    const bool fixed = W.fixed[me] != 0;
+    V3<float> v = v3<float>(W.vel[3 * me], W.vel[3 * me + 1], W.vel[3 * me + 2]);
+    V3<float> w = v3<float>(W.omega[3 * me], W.omega[3 * me + 1], W.omega[3 * me + 2]);
+    const V3<float> pv = v3<float>(W.prev_vel[3 * me], W.prev_vel[3 * me + 1], W.prev_vel[3 * me + 2]);
+    const V3<float> pw = v3<float>(W.prev_omega[3 * me], W.prev_omega[3 * me + 1], W.prev_omega[3 * me + 2]);
+    const float mud_own = W.material[4 * me + 1], e_own = W.material[4 * me + 2];
+    const float mud = __fadd_rn(mud_own, D.other(mud_own)) / 2.0f;
+    const float e = __fmul_rn(e_own, D.other(e_own));
+    const float4* c4 = reinterpret_cast<const float4*>(W.contacts) + 3 * (size_t)(W.scene_contact_cap[s] + W.pair_cstart[p]);
     for (int i = 0; i < nc; ++i) {
-        const R* ci = c + 12 * i;
-        Pcpd<R> pc;   // calculate_positional_constraint_preprocessed_data (the poses do not change here)
-        pc.r1 = qrotate(qa, v3<R>(ci[0], ci[1], ci[2]));
-        pc.r2 = qrotate(qb, v3<R>(ci[4], ci[5], ci[6]));
-        pc.I1 = Ia;
-        pc.I2 = Ib;
-        contact_velocity<R, EXACT>(pc, a, b, ci, h, mud, e, va, wa, vb, wb, pva, pwa, pvb, pwb);
+        const float4 rl = c4[3 * i + D.side], nn = c4[3 * i + 2];
+        const float lo = D.other(rl.w);
+        const V3<float> r = rotate_f(q, v3<float>(rl.x, rl.y, rl.z), true);
+        fcontact_velocity(D, r, I, D.own(v3<float>(nn.x, nn.y, nn.z)), invm, fixed, D.first(rl.w, lo), h, mud, e, v, w, pv, pw);
     }
-    if (!a.fixed) {
-        W.vel[3 * ia] = va.x; W.vel[3 * ia + 1] = va.y; W.vel[3 * ia + 2] = va.z;
-        W.omega[3 * ia] = wa.x; W.omega[3 * ia + 1] = wa.y; W.omega[3 * ia + 2] = wa.z;
+    if (!fixed) {
+        W.vel[3 * me] = v.x; W.vel[3 * me + 1] = v.y; W.vel[3 * me + 2] = v.z;
+        W.omega[3 * me] = w.x; W.omega[3 * me + 1] = w.y; W.omega[3 * me + 2] = w.z;
     }
-    if (!b.fixed) {
-        W.vel[3 * ib] = vb.x; W.vel[3 * ib + 1] = vb.y; W.vel[3 * ib + 2] = vb.z;
-        W.omega[3 * ib] = wb.x; W.omega[3 * ib + 1] = wb.y; W.omega[3 * ib + 2] = wb.z;
+}
+
+// Exact build: the contacts c[0, nc) of one pair on body `me` of this lane (both lanes of the pair call these
+// together), position and velocity sweep
+__device__ inline void dsolve_pair(const WorldView<double>& W, const Duo& D, int me, double* c, int nc, double h) {
+    const double mus_own = W.material[4 * me];
+    const double mus = (mus_own + D.other(mus_own)) / 2.0;
+    Body<double> B = load_body(W, me);
+    for (int i = 0; i < nc; ++i) collision_solve(W, D, B, c + 12 * i, h, mus);
+    store_pose(W, B);
+}
+
+__device__ inline void dvsolve_pair(const WorldView<double>& W, const Duo& D, int me, const double* c, int nc, double h) {
+    // anchors rotated by the current orientation (the poses do not change here)
+    const double4_32a q4 = W.rot[me];
+    const Qt<double> q = qt<double>(q4.x, q4.y, q4.z, q4.w);
+    double sI[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) sI[i] = W.inv_inertia[6 * me + i];
+    const M3<double> I = world_tensor(q, msym(sI));
+    const double invm = W.inv_mass[me];
+    const bool fixed = W.fixed[me] != 0;
+    V3<double> v = v3<double>(W.vel[3 * me], W.vel[3 * me + 1], W.vel[3 * me + 2]);
+    V3<double> w = v3<double>(W.omega[3 * me], W.omega[3 * me + 1], W.omega[3 * me + 2]);
+    const V3<double> pv = v3<double>(W.prev_vel[3 * me], W.prev_vel[3 * me + 1], W.prev_vel[3 * me + 2]);
+    const V3<double> pw = v3<double>(W.prev_omega[3 * me], W.prev_omega[3 * me + 1], W.prev_omega[3 * me + 2]);
+    const double mud_own = W.material[4 * me + 1], e_own = W.material[4 * me + 2];
+    const double mud = (mud_own + D.other(mud_own)) / (double)2.0f;
+    const double e = e_own * D.other(e_own);
+    for (int i = 0; i < nc; ++i) {
+        const double* ci = c + 12 * i;
+        const V3<double> r = qrotate(q, v3<double>(ci[4 * D.side], ci[4 * D.side + 1], ci[4 * D.side + 2]));
+        const V3<double> n = D.own(v3<double>(ci[8], ci[9], ci[10]));
+        contact_velocity(D, r, I, n, invm, fixed, ci[3], h, mud, e, v, w, pv, pw);
+    }
+    if (!fixed) {
+        W.vel[3 * me] = v.x; W.vel[3 * me + 1] = v.y; W.vel[3 * me + 2] = v.z;
+        W.omega[3 * me] = w.x; W.omega[3 * me + 1] = w.y; W.omega[3 * me + 2] = w.z;
+    }
+}
+
+__device__ inline void dsolve_node(const WorldView<double>& W, const Duo& D, int s, int k, double h) {
+    const int e0 = W.scene_ext[s], ne = W.scene_ext[s + 1] - e0;
+    if (k < ne) {
+        ext_solve(W, D, W.ext[e0 + k], W.ext_lambda + 4 * (size_t)(e0 + k), h);
+        return;
+    }
+    const int p = W.scene_pair_cap[s] + (k - ne);
+    const int nc = W.pair_ccount[p];
+    if (nc == 0) return;
+    const int2 pr = W.pairs[p];
+    dsolve_pair(W, D, D.side ? pr.y : pr.x, W.contacts + 12 * (size_t)(W.scene_contact_cap[s] + W.pair_cstart[p]), nc, h);
+}
+
+__device__ inline void dvsolve_node(const WorldView<double>& W, const Duo& D, int s, int k, double h) {
+    const int ne = W.scene_ext[s + 1] - W.scene_ext[s];
+    if (k < ne) return;
+    const int p = W.scene_pair_cap[s] + (k - ne);
+    const int nc = W.pair_ccount[p];
+    if (nc == 0) return;
+    const int2 pr = W.pairs[p];
+    dvsolve_pair(W, D, D.side ? pr.y : pr.x, W.contacts + 12 * (size_t)(W.scene_contact_cap[s] + W.pair_cstart[p]), nc, h);
+}
+
+// The nodes [lo, hi) of a level by a group's threads, a lane pair per node, consecutive nodes in different
+// warps (a warp runs as long as its longest node). alike: both bodies of a contact round alike.
+template <typename R, bool EXACT, bool VELOCITY>
+__device__ __forceinline__ void sweep_level(const WorldView<R>& W, int s, const int* nodes, int lo, int hi, int rank, int size, R h,
+                                            bool alike = false) {
+    Duo D = duo_of_lane();
+    if (alike) D.second_right = false;
+    for (int i = lo + ((rank & 31) >> 1) * (size >> 5) + (rank >> 5); i < hi; i += size >> 1) {
+        if constexpr (EXACT) {
+            if (VELOCITY) dvsolve_node(W, D, s, nodes[i], h);
+            else dsolve_node(W, D, s, nodes[i], h);
+        } else {
+            if (VELOCITY) fvsolve_node(W, D, s, nodes[i], h);
+            else fsolve_node(W, D, s, nodes[i], h);
+        }
     }
 }
 
@@ -1253,10 +1318,7 @@ __device__ void sweep_levels(const WorldView<R>& W, const G& g, int s, R hR) {
     while (l < L) {
         int cnt = lstart[l + 1] - lstart[l];
         if (g.nblocks() == 1 || cnt > solo) {
-            for (int i = lstart[l] + g.rank(); i < lstart[l + 1]; i += g.size()) {
-                if (VELOCITY) vsolve_node<R, EXACT>(W, s, v.nodes[i], hR);
-                else solve_node<R, EXACT>(W, s, v.nodes[i], hR);
-            }
+            sweep_level<R, EXACT, VELOCITY>(W, s, v.nodes, lstart[l], lstart[l + 1], g.rank(), g.size(), hR);
             g.sync();
             ++l;
             continue;
@@ -1265,16 +1327,32 @@ __device__ void sweep_levels(const WorldView<R>& W, const G& g, int s, R hR) {
         while (l2 < L && lstart[l2 + 1] - lstart[l2] <= solo) ++l2;
         if (g.block() == 0) {
             for (int k = l; k < l2; ++k) {
-                for (int i = lstart[k] + (int)threadIdx.x; i < lstart[k + 1]; i += blockDim.x) {
-                    if (VELOCITY) vsolve_node<R, EXACT>(W, s, v.nodes[i], hR);
-                    else solve_node<R, EXACT>(W, s, v.nodes[i], hR);
-                }
+                sweep_level<R, EXACT, VELOCITY>(W, s, v.nodes, lstart[k], lstart[k + 1], (int)threadIdx.x, (int)blockDim.x, hR, true);
                 __syncthreads();
             }
         }
         g.sync();
         l = l2;
     }
+}
+
+// predict and the substep's FP32 copies of one body (phase-major form)
+template <typename R, bool EXACT, bool DELTAS>
+__device__ __forceinline__ void predict_stage(const WorldView<R>& W, int b, double h) {
+    predict_body<R, EXACT>(W, b, h);
+    if constexpr (EXACT) {
+        const double4_32a p = W.pos[b], q = W.rot[b];
+        W.pose_f[2 * b] = make_float4((float)p.x, (float)p.y, (float)p.z, 0.f);
+        W.pose_f[2 * b + 1] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
+    } else {
+        stage_body<DELTAS>(W, b);
+    }
+}
+
+// the work counters of a substep's narrowphase (phase-major form), and the substep count
+template <typename R>
+__device__ __forceinline__ void reset_narrow_queue(const WorldView<R>& W) {
+    W.queue[2] = 0; W.queue[3] = 0; W.queue[4] += 1; W.queue[5] = 0; W.queue[7] = 0;
 }
 
 template <typename R, bool EXACT, class G>
@@ -1332,7 +1410,6 @@ __device__ void step_scene(const WorldView<R>& W, const G& g, int s, const StepP
                 const int2 pr = W.pairs[pb + p];
                 W.pair_base[pb + p] = fbase4(W, pr.x, pr.y);
             }
-            for (int e = e0 + g.rank(); e < e1; e += g.size()) W.ext_base[e] = fbase4(W, W.ext[e].e1, W.ext[e].e2);
             g.sync();
         }
         mark(PH_NARROW);
