@@ -161,7 +161,7 @@ struct rp_world {
     DevBuf d_rec, d_slot_entity;                   // the records on the device; entity of each body slot
     cudaEvent_t ev_rec = nullptr;                  // the last record upload (h_rec is refilled after it)
     double adj_prof[6] = {0, 0, 0, 0, 0, 0};      // last adjoint's slowest scene (rp_adjoint_profile)
-    DevBuf d_pose_f, d_body_scene, d_col_body, d_scene_order, d_gjk_list, d_hit_list, d_work_list, d_work_state, d_work_simplex, d_work_epa, d_queue, d_work_off, d_work_face, d_fallback, d_tstamp, d_tlist, d_single_hull, d_pair_base, d_solve_scenes;
+    DevBuf d_pose_f, d_body_scene, d_col_body, d_scene_order, d_gjk_list, d_hit_list, d_work_list, d_work_state, d_work_simplex, d_work_epa, d_queue, d_work_off, d_work_face, d_fallback, d_tstamp, d_tlist, d_single_hull, d_pair_base, d_solve_scenes, d_hull_ref, d_topo_rec;
     int mode = RP_MODE_AUTO;          // RP_MODE_*: how a frame is launched
     int solo_nodes = 512;             // tunable: grid sweeps run levels up to this size on one CTA
     int cta_from = 0;                 // tunable: batched sweeps give a whole CTA to scenes of this cost or more (0: none)
@@ -384,6 +384,64 @@ rp_status build_device(rp_world* w) {
         shapes.push_back(sh);
     }
     fstart.push_back((int32_t)felem.size());
+    // byte records of each distinct topology for the narrowphase's warp kernels (HullRef, rp_world.h)
+    std::vector<uint8_t> rec;
+    std::vector<HullRef> hull_recs(w->hulls.size());
+    {
+        std::map<int32_t, HullRef> done;   // by Shape::elem_off (one per topology)
+        for (size_t h = 0; h < w->hulls.size(); ++h) {
+            const Hull& H = *w->hulls[h];
+            HullRef r;
+            std::memset(&r, 0, sizeof(r));
+            if (H.nv() <= 64) {
+                auto it = done.find(shapes[h].elem_off);
+                if (it == done.end()) {
+                    auto emit = [&](size_t rows, auto&& bytes_of, int32_t& first, int32_t& stride) {
+                        std::vector<std::vector<uint8_t>> all;
+                        size_t longest = 1;
+                        for (size_t i = 0; i < rows; ++i) {
+                            all.push_back(bytes_of(i));
+                            longest = std::max(longest, all.back().size());
+                        }
+                        stride = (int32_t)((longest + 127) / 128);
+                        first = (int32_t)(rec.size() / 128);
+                        for (auto& b : all) {
+                            b.resize((size_t)stride * 128, 0);
+                            rec.insert(rec.end(), b.begin(), b.end());
+                        }
+                    };
+                    emit((size_t)H.nv(), [&](size_t v) {
+                        std::vector<uint8_t> b{(uint8_t)H.v2f[v].size(), (uint8_t)H.v2n[v].size()};
+                        for (int f : H.v2f[v]) b.push_back((uint8_t)f);
+                        for (int u : H.v2n[v]) b.push_back((uint8_t)u);
+                        return b;
+                    }, r.vrec, r.vstride);
+                    emit((size_t)H.nf(), [&](size_t f) {
+                        std::vector<uint8_t> b{(uint8_t)H.faces[f].size(), (uint8_t)H.f2n[f].size()};
+                        for (auto v : H.faces[f]) b.push_back((uint8_t)v);
+                        for (int g : H.f2n[f]) b.push_back((uint8_t)g);
+                        for (int g : H.f2n[f]) b.push_back((uint8_t)H.faces[(size_t)g][0]);
+                        return b;
+                    }, r.frec, r.fstride);
+                    done.emplace(shapes[h].elem_off, r);
+                } else {
+                    r = it->second;
+                }
+            }
+            r.nv = shapes[h].nv;
+            r.face_off = shapes[h].face_off;
+            hull_recs[h] = r;
+        }
+    }
+    // a hull whose counts do not fit the records' bytes takes the general narrowphase path
+    std::vector<uint8_t> recordable(w->hulls.size(), 0);
+    for (size_t h = 0; h < w->hulls.size(); ++h) {
+        const Hull& H = *w->hulls[h];
+        bool ok = H.nv() <= 64 && H.nf() <= 255;
+        for (const auto* rows : {&H.faces, &H.v2f, &H.v2n, &H.f2n})
+            for (const auto& r : *rows) ok = ok && r.size() <= 255;
+        recordable[h] = ok;
+    }
     // colliders, transformed-geometry offsets
     std::vector<Collider> cols;
     std::vector<int32_t> col_start(N + 1, 0);
@@ -565,6 +623,19 @@ rp_status build_device(rp_world* w) {
             single[slot] = col_start[slot + 1] - c == 1 && cols[(size_t)c].type == COL_HULL &&
                            shapes[(size_t)cols[(size_t)c].shape].nv <= 64;
         }
+        std::vector<HullRef> refs(std::max<size_t>(N, 1));
+        for (size_t slot = 0; slot < N; ++slot) {
+            if (!single[slot]) continue;
+            const Collider& c = cols[(size_t)col_start[slot]];
+            const size_t h = (size_t)w->bodies[(size_t)w->slot_to_entity[slot]].cols[0].hull;
+            if (!recordable[h]) { single[slot] = 0; continue; }
+            refs[slot] = hull_recs[h];
+            refs[slot].tv_off = c.tv_off;
+            refs[slot].tn_off = c.tn_off;
+        }
+        RP_CUDA(upload(w->d_hull_ref, refs, st));
+        rec.resize(rec.size() + 512, 0);   // lanes past a record's end read on
+        RP_CUDA(upload(w->d_topo_rec, rec, st));
         RP_CUDA(upload(w->d_single_hull, single, st));
         RP_CUDA(w->d_pose_f.ensure(std::max<size_t>(N, 1) * 32));
         for (DevBuf* b : {&w->d_sdx, &w->d_sdq, &w->d_pred_d, &w->d_prev_qf}) {
@@ -573,8 +644,8 @@ rp_status build_device(rp_world* w) {
         }
         RP_CUDA(w->d_work_list.ensure(std::max<size_t>(P, 1) * 4));
         RP_CUDA(w->d_work_state.ensure(std::max<size_t>(P, 1) * 4));
-        RP_CUDA(w->d_gjk_list.ensure(std::max<size_t>(P, 1) * 4));
-        RP_CUDA(w->d_hit_list.ensure(std::max<size_t>(P, 1) * 4));
+        RP_CUDA(w->d_gjk_list.ensure(std::max<size_t>(P, 1) * 16));
+        RP_CUDA(w->d_hit_list.ensure(std::max<size_t>(P, 1) * 16));
         RP_CUDA(w->d_work_simplex.ensure(std::max<size_t>(P, 1) * 16 * R));
         RP_CUDA(w->d_work_epa.ensure(std::max<size_t>(P, 1) * 4 * 8));
         RP_CUDA(w->d_work_off.ensure(std::max<size_t>(P, 1) * 16));
@@ -761,8 +832,10 @@ WorldView<R> make_view(rp_world* w) {
     V.single_hull = w->d_single_hull.as<uint8_t>();
     V.work_list = w->d_work_list.as<int32_t>();
     V.work_state = w->d_work_state.as<int32_t>();
-    V.gjk_list = w->d_gjk_list.as<int32_t>();
-    V.hit_list = w->d_hit_list.as<int32_t>();
+    V.gjk_list = w->d_gjk_list.as<int4>();
+    V.hull_ref = w->d_hull_ref.as<HullRef>();
+    V.topo_rec = w->d_topo_rec.as<uint8_t>();
+    V.hit_list = w->d_hit_list.as<int4>();
     V.work_simplex = w->d_work_simplex.as<R>();
     V.work_epa = w->d_work_epa.as<double>();
     V.work_off = w->d_work_off.as<float4>();

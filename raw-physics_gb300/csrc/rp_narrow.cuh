@@ -163,9 +163,9 @@ struct ColView {
 // A face normal of a hull rotated by the body's FP64 orientation (collider_update's normal
 // transform, collider.cpp:425-429), for the FP32 build's FP64 reference-face decision.
 template <typename R>
-__device__ __forceinline__ V3<double> face_normal64(const WorldView<R>& W, const ColView<R>& c, int f) {
-    const double* n = W.face_normal + 3 * (c.shape->face_off + f);
-    const double4_32a q = W.rot[c.body];
+__device__ __forceinline__ V3<double> face_normal64(const WorldView<R>& W, int face, int body) {
+    const double* n = W.face_normal + 3 * face;
+    const double4_32a q = W.rot[body];
     return vnorm_fast(mmulv(qmat3(qt<double>(q.x, q.y, q.z, q.w)), v3<double>(n[0], n[1], n[2])));
 }
 
@@ -349,12 +349,11 @@ __device__ __forceinline__ bool same_bits(double a, double b) { return __double_
 // and would end false at the iteration cap. Brent's cycle detection (one saved state, saved
 // again at power-of-two distances, kept in `saved`, 16 values in shared memory) stops such runs
 // early with the same result; the iteration count returned is then below 100 and `cycled` is set.
-template <typename R>
-__device__ bool gjk_collides(const ColView<R>& c1, const ColView<R>& c2, Simplex<R>& s, int& iters,
-                             long long& support_cycles, R* saved, bool& cycled) {
+template <typename R, class Mink>
+__device__ bool gjk_run(const Mink& mink, Simplex<R>& s, int& iters, long long& support_cycles, R* saved, bool& cycled) {
     const int lane = (int)lane_id();
     long long t0 = clock64();
-    s.a = support_mink(c1, c2, v3<R>(0, 0, 1));
+    s.a = mink(v3<R>(0, 0, 1));
     s.b = s.c = s.d = v3<R>(0, 0, 0);
     s.num = 1;
     V3<R> dir = vscale((R)-1.0, s.a);
@@ -362,7 +361,7 @@ __device__ bool gjk_collides(const ColView<R>& c1, const ColView<R>& c2, Simplex
     int power = 1, lam = 0;
     for (int i = 0; i < 100; ++i) {
         iters = i + 1;
-        V3<R> p = support_mink(c1, c2, dir);
+        V3<R> p = mink(dir);
         support_cycles += clock64() - t0;
         if (vdot(p, dir) < (R)0) return false;
         if (s.num == 1) { s.b = s.a; s.a = p; }
@@ -386,6 +385,19 @@ __device__ bool gjk_collides(const ColView<R>& c1, const ColView<R>& c2, Simplex
         t0 = clock64();
     }
     return false;
+}
+
+// the support of two colliders of any kind, the form gjk_run and epa take
+template <typename R>
+struct ColMink {
+    const ColView<R>& a;
+    const ColView<R>& b;
+    __device__ __forceinline__ V3<R> operator()(V3<R> d) const { return support_mink(a, b, d); }
+};
+template <typename R>
+__device__ bool gjk_collides(const ColView<R>& c1, const ColView<R>& c2, Simplex<R>& s, int& iters,
+                             long long& support_cycles, R* saved, bool& cycled) {
+    return gjk_run(ColMink<R>{c1, c2}, s, iters, support_cycles, saved, cycled);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -469,8 +481,8 @@ __device__ __forceinline__ void epa_add_edge_warp(EdgeRegs<R>& E, int& ne, int x
 }
 
 // Returns true when converged; normal and penetration are then set (FP64).
-template <typename R>
-__device__ bool epa(NarrowSmem<R>& sm, const ColView<R>& c1, const ColView<R>& c2, const Simplex<R>& s,
+template <typename R, class Mink>
+__device__ bool epa(NarrowSmem<R>& sm, const Mink& mink, const Simplex<R>& s,
                     V3<double>& out_n, double& out_pen, int& iters) {
     const unsigned lane = lane_id();
     if (lane == 0) {
@@ -495,7 +507,7 @@ __device__ bool epa(NarrowSmem<R>& sm, const ColView<R>& c1, const ColView<R>& c
     double min_d = md;
     for (int it = 0; it < 100; ++it) {
         iters = it + 1;
-        V3<R> sp = support_mink(c1, c2, v3cast<R>(min_n));
+        V3<R> sp = mink(v3cast<R>(min_n));
         V3<double> spd = v3cast<double>(sp);
         double d = vdot(min_n, spd);
         if (fabs(d - min_d) < 0.0001) {
@@ -626,8 +638,8 @@ __device__ __forceinline__ void epa_face_f32(const V3<float>* poly, int npoly, u
 // face_out (optional): when FP32 decides the termination, lane 0 writes the final face's three
 // points and its FP32 normal there (12 floats) and *deferred is set, leaving the FP64 normal and depth
 // to a thread-per-pair kernel (k_epa_finish) instead of the warp; otherwise they are computed here.
-template <typename R>
-__device__ bool epa_fast(NarrowSmem<R>& smr, const ColView<R>& c1, const ColView<R>& c2, const Simplex<R>& s,
+template <typename R, class Mink>
+__device__ bool epa_fast(NarrowSmem<R>& smr, const Mink& mink, const Simplex<R>& s,
                          V3<double>& out_n, double& out_pen, int& iters, long long* support_cycles = nullptr,
                          float* face_out = nullptr, bool* deferred = nullptr) {
     static_assert(sizeof(EpaFastSmem<R>) <= sizeof(typename NarrowSmem<R>::U), "EPA scratch must fit the union");
@@ -660,7 +672,7 @@ __device__ bool epa_fast(NarrowSmem<R>& smr, const ColView<R>& c1, const ColView
         iters = it + 1;
         V3<float> min_n = mi == 0x7fffffff ? v3<float>(0.f, 0.f, 0.f) : sm.fn[mi];
         const long long ts = clock64();
-        V3<float> sp = v3cast<float>(support_mink(c1, c2, v3cast<R>(min_n)));
+        V3<float> sp = v3cast<float>(mink(v3cast<R>(min_n)));
         if (support_cycles) *support_cycles += clock64() - ts;
         // Termination test (epa.cpp:153-160) with the FP64 outcome: |<n, s> - d| < 1e-4 for the
         // closest face. FP32 decides it when the FP32 gap is farther from 1e-4 than its error bound
@@ -918,6 +930,55 @@ __device__ void push_contact(NarrowSmem<R>& sm, const PairFrame<R, EXACT>& fr, V
 template <typename R>
 __device__ __forceinline__ int csr_len(const int32_t* start, int row) { return start[row + 1] - start[row]; }
 
+// the closest points of two skew lines p1 + t dd1, p2 + u dd2 (clipping.cpp:210-239); false when parallel
+template <typename R>
+__device__ __forceinline__ bool skew_points(V3<R> p1, V3<R> dd1, V3<R> p2, V3<R> dd2, V3<R>& l1, V3<R>& l2) {
+    R nA = dd1.x * dd2.x + dd1.y * dd2.y + dd1.z * dd2.z;
+    R nB = dd2.x * dd2.x + dd2.y * dd2.y + dd2.z * dd2.z;
+    R mA = -dd1.x * dd1.x - dd1.y * dd1.y - dd1.z * dd1.z;
+    R mB = -dd2.x * dd1.x - dd2.y * dd1.y - dd2.z * dd1.z;
+    R rA = -dd1.x * p2.x + dd1.x * p1.x - dd1.y * p2.y + dd1.y * p1.y - dd1.z * p2.z + dd1.z * p1.z;
+    R rB = -dd2.x * p2.x + dd2.x * p1.x - dd2.y * p2.y + dd2.y * p1.y - dd2.z * p2.z + dd2.z * p1.z;
+    R den = (nA * mB) - (nB * mA);
+    bool ok = den != (R)0;
+    R nn = ok ? ((rA * mB) - (rB * mA)) / den : (R)0;
+    R mm = ok ? ((nA * rB) - (nB * rA)) / den : (R)0;
+    l1 = vadd(p1, vscale(mm, dd1));
+    l2 = vadd(p2, vscale(nn, dd2));
+    return ok;
+}
+
+// The contacts of a clipped incident polygon: its points below the reference plane, each with its projection
+template <typename R, bool EXACT>
+__device__ __forceinline__ void clipped_contacts(NarrowSmem<R>& sm, const PairFrame<R, EXACT>& fr, const V3<R>* poly, int n, bool ref1,
+                                                 V3<R> ref_n, V3<R> ref_p, V3<R> normal) {
+    const unsigned lane = lane_id();
+    // contacts from the kept points (clipping.cpp:302-327)
+    for (int base = 0; base < n; base += WARP) {
+        int k = base + (int)lane;
+        bool pred = false;
+        V3<R> c1 = v3<R>(0, 0, 0), c2 = v3<R>(0, 0, 0);
+        if (k < n) {
+            V3<R> pt = poly[k];
+            R dd = vdot(vscale((R)-1.0, ref_n), ref_p);
+            V3<R> cp = vsub(pt, vscale(vdot(ref_n, pt) + dd, ref_n));
+            V3<R> diff = vsub(pt, cp);
+            R pen;
+            if (ref1) {
+                pen = vdot(diff, normal);
+                c1 = vsub(pt, vscale(pen, normal));
+                c2 = pt;
+            } else {
+                pen = -vdot(diff, normal);
+                c1 = pt;
+                c2 = vadd(pt, vscale(pen, normal));
+            }
+            pred = pen < (R)0.0;
+        }
+        push_contact(sm, fr, c1, c2, normal, pred);
+    }
+}
+
 // convex_convex_contact_manifold (clipping.cpp:249-341)
 template <typename R, bool EXACT>
 __device__ void convex_convex_manifold(NarrowSmem<R>& sm, const WorldView<R>& W, const ColView<R>& h1, const ColView<R>& h2,
@@ -979,21 +1040,9 @@ __device__ void convex_convex_manifold(NarrowSmem<R>& sm, const WorldView<R>& W,
     R d1 = vdot(n1, normal), d2 = vdot(n2, inv_n), de = vdot(edge_normal, normal);
     if (de > d1 + (R)0.0001 && de > d2 + (R)0.0001) {
         // collision_distance_between_skew_lines (clipping.cpp:210-239)
-        V3<R> p1 = sp1, dd1 = vsub(cv_vertex(h1, ei), p1);
-        V3<R> p2 = sp2, dd2 = vsub(cv_vertex(h2, ej), p2);
-        R nA = dd1.x * dd2.x + dd1.y * dd2.y + dd1.z * dd2.z;
-        R nB = dd2.x * dd2.x + dd2.y * dd2.y + dd2.z * dd2.z;
-        R mA = -dd1.x * dd1.x - dd1.y * dd1.y - dd1.z * dd1.z;
-        R mB = -dd2.x * dd1.x - dd2.y * dd1.y - dd2.z * dd1.z;
-        R rA = -dd1.x * p2.x + dd1.x * p1.x - dd1.y * p2.y + dd1.y * p1.y - dd1.z * p2.z + dd1.z * p1.z;
-        R rB = -dd2.x * p2.x + dd2.x * p1.x - dd2.y * p2.y + dd2.y * p1.y - dd2.z * p2.z + dd2.z * p1.z;
-        R den = (nA * mB) - (nB * mA);
-        bool ok = den != (R)0;
+        V3<R> l1, l2;
+        const bool ok = skew_points(sp1, vsub(cv_vertex(h1, ei), sp1), sp2, vsub(cv_vertex(h2, ej), sp2), l1, l2);
         if (!ok && lane == 0) atomicOr(&sm.status, (int)(ST_DEGENERATE | ST_DEG_SKEW));
-        R nn = ok ? ((rA * mB) - (rB * mA)) / den : (R)0;
-        R mm = ok ? ((nA * rB) - (nB * rA)) / den : (R)0;
-        V3<R> l1 = vadd(p1, vscale(mm, dd1));
-        V3<R> l2 = vadd(p2, vscale(nn, dd2));
         push_contact(sm, fr, l1, l2, normal, ok && lane == 0);
         return;
     }
@@ -1007,7 +1056,7 @@ __device__ void convex_convex_manifold(NarrowSmem<R>& sm, const WorldView<R>& W,
         // one lane evaluates it (FP64 on GB300 issues at 1/64 of the FP32 rate) and broadcasts it
         int r = 0;
         if (lane == 0) {
-            const V3<double> m1 = face_normal64(W, h1, f1), m2 = face_normal64(W, h2, f2);
+            const V3<double> m1 = face_normal64(W, h1.shape->face_off + f1, h1.body), m2 = face_normal64(W, h2.shape->face_off + f2, h2.body);
             r = vdot(m1, normal64) > vdot(m2, vinv(normal64)) ? 1 : 0;
         }
         ref1 = __shfl_sync(0xffffffffu, r, 0) != 0;
@@ -1045,30 +1094,7 @@ __device__ void convex_convex_manifold(NarrowSmem<R>& sm, const WorldView<R>& W,
         if (m >= 0) { n = m; cur ^= 1; }
     }
     if (st && lane == 0) atomicOr(&sm.status, (int)st);
-    // contacts from the kept points (clipping.cpp:302-327)
-    for (int base = 0; base < n; base += WARP) {
-        int k = base + (int)lane;
-        bool pred = false;
-        V3<R> c1 = v3<R>(0, 0, 0), c2 = v3<R>(0, 0, 0);
-        if (k < n) {
-            V3<R> pt = sm.u.clip.buf[cur][k];
-            R dd = vdot(vscale((R)-1.0, ref_n), ref_p);
-            V3<R> cp = vsub(pt, vscale(vdot(ref_n, pt) + dd, ref_n));
-            V3<R> diff = vsub(pt, cp);
-            R pen;
-            if (ref1) {
-                pen = vdot(diff, normal);
-                c1 = vsub(pt, vscale(pen, normal));
-                c2 = pt;
-            } else {
-                pen = -vdot(diff, normal);
-                c1 = pt;
-                c2 = vadd(pt, vscale(pen, normal));
-            }
-            pred = pen < (R)0.0;
-        }
-        push_contact(sm, fr, c1, c2, normal, pred);
-    }
+    clipped_contacts<R, EXACT>(sm, fr, sm.u.clip.buf[cur], n, ref1, ref_n, ref_p, normal);
 }
 
 // clipping_get_contact_manifold (clipping.cpp:343-370)
@@ -1121,8 +1147,8 @@ __device__ void collider_contacts(NarrowSmem<R>& sm, const WorldView<R>& W, cons
     V3<double> n;
     double pen;
     bool ok;
-    if constexpr (EXACT || !kEpaFast) ok = epa(sm, c1, c2, s, n, pen, ei);
-    else ok = epa_fast(sm, c1, c2, s, n, pen, ei);
+    if constexpr (EXACT || !kEpaFast) ok = epa(sm, ColMink<R>{c1, c2}, s, n, pen, ei);
+    else ok = epa_fast(sm, ColMink<R>{c1, c2}, s, n, pen, ei);
     const long long t2 = clock64();
     if (counters && lane_id() == 0) {
         atomicAdd(&counters[1], (unsigned long long)ei);

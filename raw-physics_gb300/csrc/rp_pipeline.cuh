@@ -25,6 +25,7 @@
 #pragma once
 #include "rp_step.cuh"
 #include "rp_scene.cuh"
+#include "rp_hullpair.cuh"
 #include "rp_launch.h"
 
 namespace rp {
@@ -32,11 +33,9 @@ namespace rp {
 constexpr int PIPE_BLOCK = 256;
 constexpr int PIPE_WARPS = PIPE_BLOCK / 32;
 
-// Shared memory of one warp in k_gjk: the two staged hulls and the cycle-detection state.
+// Shared memory of one warp in k_gjk: the cycle-detection state.
 template <typename R>
 struct GjkSmem {
-    V3<R> va[STAGE_V];
-    V3<R> vb[STAGE_V];
     R saved[16];
 };
 
@@ -53,33 +52,37 @@ struct WarpTally {
     }
 };
 
-// Views of a pair of single-hull bodies in the pair frame of pair_contacts (FP32 build: body a's
-// origin; exact build: world coordinates), staging both hulls' vertices in shared memory. The FP32
-// build reads the pair's FP32 offset (work_off, rounded from the FP64 poses by k_cull) and the FP32
-// orientations of the predict phase (pose_f), which equal the casts of the FP64 values: no FP64
-// arithmetic or conversion runs in the warp.
+// The pair frame of two single-hull bodies (FP32 build: body a's origin; exact build: world coordinates) and
+// body b's offset in it. The FP32 build reads the pair's FP32 offset (work_off, rounded from the FP64 poses by
+// k_cull) and the FP32 orientations of the predict phase (pose_f), which equal the casts of the FP64
+// values: no FP64 arithmetic or conversion runs in the warp.
 template <typename R, bool EXACT>
-__device__ void single_views(const WorldView<R>& W, V3<R>* stage_a, V3<R>* stage_b, int a, int b, int k, ColView<R>& va,
-                             ColView<R>& vb, PairFrame<R, EXACT>& fr) {
+__device__ __forceinline__ V3<R> pair_offset(const WorldView<R>& W, int k) {
+    if constexpr (EXACT) {
+        return v3<R>(0, 0, 0);
+    } else {
+        const float4 o = W.work_off[k];
+        return v3<R>(o.x, o.y, o.z);
+    }
+}
+template <typename R, bool EXACT>
+__device__ __forceinline__ PairFrame<R, EXACT> pair_frame(const WorldView<R>& W, int a, int b, V3<R> offb) {
+    PairFrame<R, EXACT> fr;
     fr.raw = false;
-    V3<R> offa = v3<R>(0, 0, 0), offb;
     if constexpr (EXACT) {
         double4_32a pa = W.pos[a], pb = W.pos[b], qa4 = W.rot[a], qb4 = W.rot[b];
-        offb = v3<R>(0, 0, 0);
         fr.x1 = v3<R>((R)pa.x, (R)pa.y, (R)pa.z);
         fr.x2 = v3<R>((R)pb.x, (R)pb.y, (R)pb.z);
         fr.q1inv = qinverse(qt<R>((R)qa4.x, (R)qa4.y, (R)qa4.z, (R)qa4.w));
         fr.q2inv = qinverse(qt<R>((R)qb4.x, (R)qb4.y, (R)qb4.z, (R)qb4.w));
     } else {
-        const float4 o = W.work_off[k], qa = W.pose_f[2 * a + 1], qb = W.pose_f[2 * b + 1];
-        offb = v3<R>(o.x, o.y, o.z);
-        fr.x1 = offa;
+        const float4 qa = W.pose_f[2 * a + 1], qb = W.pose_f[2 * b + 1];
+        fr.x1 = v3<R>(0, 0, 0);
         fr.x2 = offb;
         fr.q1inv = qinverse(qt<R>(qa.x, qa.y, qa.z, qa.w));
         fr.q2inv = qinverse(qt<R>(qb.x, qb.y, qb.z, qb.w));
     }
-    va = make_view<R, EXACT>(W, W.col_start[a], EXACT ? fr.x1 : offa, offa, stage_a, a);
-    vb = make_view<R, EXACT>(W, W.col_start[b], EXACT ? fr.x2 : offb, offb, stage_b, b);
+    return fr;
 }
 
 // True when both bodies have exactly one collider, a hull whose vertices fit the staging area.
@@ -228,7 +231,7 @@ __global__ void __launch_bounds__(PIPE_BLOCK) k_velocity(WorldView<R> W, int nbo
 // Narrowphase kernels
 // Appends `item` (valid where `take`) to list[*count ...] with one atomic per CTA: a block-wide
 // scan of the flags, then thread 0 reserves the block's range. Every thread of the block calls it.
-__device__ __forceinline__ void block_append(int32_t* list, int32_t* count, bool take, int item, int* smem, int* base_smem) {
+__device__ __forceinline__ void block_append(int4* list, int32_t* count, bool take, int4 item, int* smem, int* base_smem) {
     int total;
     const int incl = block_incl_scan(take ? 1 : 0, smem, total);
     if (threadIdx.x == 0) *base_smem = total ? atomicAdd(count, total) : 0;
@@ -252,10 +255,12 @@ __global__ void __launch_bounds__(PIPE_BLOCK) k_cull(WorldView<R> W, int enabled
         int state = WS_NONE;
         bool gjk = false;
         int ta = -1, tb = -1;
+        int4 item = make_int4(k, 0, 0, 0);
         if (k < n) {
             const int gp = W.work_list[k];
             const int2 pr = W.pairs[gp];
             const int a = pr.x, b = pr.y;
+            item = make_int4(k, gp, a, b);
             const bool live = !((W.fixed[a] || !W.active[a]) && (W.fixed[b] || !W.active[b]));
             if (live && enabled) {
                 if (!single_hulls(W, a, b)) state = WS_GENERAL;
@@ -292,8 +297,8 @@ __global__ void __launch_bounds__(PIPE_BLOCK) k_cull(WorldView<R> W, int enabled
             if (ta >= 0) W.tlist[base++] = ta;
             if (tb >= 0) W.tlist[base] = tb;
         }
-        block_append(W.gjk_list, &W.queue[2], gjk, k, scan_smem, &base_smem);
-        block_append(W.hit_list, &W.queue[3], state == WS_GENERAL, k, scan_smem, &base_smem);
+        block_append(W.gjk_list, &W.queue[2], gjk, item, scan_smem, &base_smem);
+        block_append(W.hit_list, &W.queue[3], state == WS_GENERAL, item, scan_smem, &base_smem);
     }
     for (int o = 16; o > 0; o >>= 1) apart += __shfl_xor_sync(0xffffffffu, apart, o);
     if ((threadIdx.x & 31) == 0 && apart && W.counters) atomicAdd(&W.counters[11], apart);
@@ -310,21 +315,19 @@ __global__ void __launch_bounds__(PIPE_BLOCK, 3) k_gjk(WorldView<R> W) {
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     const int n = W.queue[2];
     WarpTally t;   // GJK iterations, cap hits, cycles, support cycles, cycle exits, -, GJK runs
-    int pending = 0, mine = 0;
+    int pending = 0;
+    int4 mine = make_int4(0, 0, 0, 0);
     for (int j = gw; j < n; j += nw) {
-        const int k = W.gjk_list[j];
-        const int gp = W.work_list[k];
-        const int2 pr = W.pairs[gp];
-        const int a = pr.x, b = pr.y;
-        ColView<R> va, vb;
-        PairFrame<R, EXACT> fr;
-        single_views<R, EXACT>(W, sm.va, sm.vb, a, b, k, va, vb, fr);
+        const int4 item = W.gjk_list[j];
+        const int k = item.x, gp = item.y;
+        const RegHull<R> ra = load_reghull(W, W.hull_ref[item.z], v3<R>(0, 0, 0));
+        const RegHull<R> rb = load_reghull(W, W.hull_ref[item.w], pair_offset<R, EXACT>(W, k));
         Simplex<R> sx;
         int gi = 0;
         long long tsup = 0;
         bool cycled = false;
         const long long t0 = clock64();
-        const bool hit = gjk_collides(va, vb, sx, gi, tsup, sm.saved, cycled);
+        const bool hit = gjk_run(RegMink<R>{ra, rb}, sx, gi, tsup, sm.saved, cycled);
         t.v[0] += gi;
         t.v[1] += gi >= 100;
         t.v[2] += clock64() - t0;
@@ -338,7 +341,7 @@ __global__ void __launch_bounds__(PIPE_BLOCK, 3) k_gjk(WorldView<R> W) {
 #pragma unroll
             for (int i = 0; i < 12; ++i)
                 if (lane == i) out[i] = comp[i];
-            if (lane == pending) mine = k;
+            if (lane == pending) mine = item;
             if (++pending == 32) {
                 int base = 0;
                 if (lane == 0) base = atomicAdd(&W.queue[3], 32);
@@ -373,17 +376,15 @@ __global__ void __launch_bounds__(PIPE_BLOCK, EXACT ? 2 : 3) k_epa(WorldView<R> 
     const int n = W.queue[3];
     WarpTally t;   // EPA iterations, EPA calls, EPA cycles, EPA cap hits
     for (int j = gw; j < n; j += nw) {
-        const int k = W.hit_list[j];
+        const int4 item = W.hit_list[j];
+        const int k = item.x;
         if (W.work_state[k] != WS_HIT) continue;
         {
-            const int gp = W.work_list[k];
-            const int2 pr = W.pairs[gp];
-            const int a = pr.x, b = pr.y;
+            const int gp = item.y, a = item.z, b = item.w;
             if (lane == 0) { sm.status = 0; }
             const long long tv = clock64();
-            ColView<R> va, vb;
-            PairFrame<R, EXACT> fr;
-            single_views<R, EXACT>(W, sm.va, sm.vb, a, b, k, va, vb, fr);
+            const RegHull<R> ra = load_reghull(W, W.hull_ref[a], v3<R>(0, 0, 0));
+            const RegHull<R> rb = load_reghull(W, W.hull_ref[b], pair_offset<R, EXACT>(W, k));
             const R* in = W.work_simplex + 16 * (size_t)k;
             Simplex<R> sx;
             sx.a = v3<R>(in[0], in[1], in[2]);
@@ -398,8 +399,8 @@ __global__ void __launch_bounds__(PIPE_BLOCK, EXACT ? 2 : 3) k_epa(WorldView<R> 
             long long tsup = 0;
             bool deferred = false;
             bool ok;
-            if constexpr (EXACT || !kEpaFast) ok = epa(sm, va, vb, sx, nrm, pen, ei);
-            else ok = epa_fast(sm, va, vb, sx, nrm, pen, ei, &tsup, W.work_face + 12 * (size_t)k, &deferred);
+            if constexpr (EXACT || !kEpaFast) ok = epa(sm, RegMink<R>{ra, rb}, sx, nrm, pen, ei);
+            else ok = epa_fast(sm, RegMink<R>{ra, rb}, sx, nrm, pen, ei, &tsup, W.work_face + 12 * (size_t)k, &deferred);
             t.v[0] += ei;
             t.v[1] += 1;
             t.v[2] += clock64() - t0;
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(PIPE_BLOCK) k_epa_finish(WorldView<R> W) {
     if (frame_abandoned(W.status)) return;
     const int n = W.queue[3];
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        const int k = W.hit_list[j];
+        const int k = W.hit_list[j].x;
         if (W.work_state[k] != WS_EPA_FACE) continue;
         float* f = W.work_face + 12 * (size_t)k;
         V3<double> n64;
@@ -480,13 +481,12 @@ __global__ void __launch_bounds__(PIPE_BLOCK, (GENERAL || EXACT) ? 2 : 3) k_mani
     const int n = W.queue[3];
     WarpTally t;   // contacts, manifold cycles
     for (int j = gw; j < n; j += nw) {
-        const int k = W.hit_list[j];
+        const int4 item = W.hit_list[j];
+        const int k = item.x;
         const int st = W.work_state[k];
         if (st != (GENERAL ? WS_GENERAL : WS_EPA_OK)) continue;
         {
-            const int gp = W.work_list[k];
-            const int2 pr = W.pairs[gp];
-            const int a = pr.x, b = pr.y;
+            const int gp = item.y, a = item.z, b = item.w;
             const int s = W.body_scene[a];
             const long long t0 = clock64();
             long long t1 = t0;
@@ -495,18 +495,22 @@ __global__ void __launch_bounds__(PIPE_BLOCK, (GENERAL || EXACT) ? 2 : 3) k_mani
             } else {
                 if (lane == 0) { sm.ncontacts = 0; sm.status = 0; }
                 __syncwarp();
-                ColView<R> va, vb;
-                PairFrame<R, EXACT> fr;
-                single_views<R, EXACT>(W, sm.va, sm.vb, a, b, k, va, vb, fr);
+                const V3<R> offb = pair_offset<R, EXACT>(W, k);
+                const HullRef ha = W.hull_ref[a], hb = W.hull_ref[b];
+                const RegHull<R> ra = load_reghull(W, ha, v3<R>(0, 0, 0)), rb = load_reghull(W, hb, offb);
+                const PairFrame<R, EXACT> fr = pair_frame<R, EXACT>(W, a, b, offb);
+                sm.va[lane] = ra.v0; sm.va[lane + 32] = ra.v1;
+                sm.vb[lane] = rb.v0; sm.vb[lane + 32] = rb.v1;
+                __syncwarp();
                 const double* e = W.work_epa + 4 * (size_t)k;
                 const V3<double> n64 = v3<double>(e[0], e[1], e[2]);
                 t1 = clock64();
                 if constexpr (EXACT) {
-                    contact_manifold<R, EXACT>(sm, W, va, vb, v3cast<R>(n64), n64, (R)e[3], fr);
+                    hull_manifold<R, EXACT>(sm, W, ra, rb, ha, hb, a, b, v3cast<R>(n64), n64, fr);
                 } else {
-                    // the FP32 normal and depth stored beside the FP64 ones (no conversion in the warp)
+                    // the FP32 normal stored beside the FP64 one (no conversion in the warp)
                     const float* f = W.work_face + 12 * (size_t)k;
-                    contact_manifold<R, EXACT>(sm, W, va, vb, v3<R>(f[0], f[1], f[2]), n64, (R)f[3], fr);
+                    hull_manifold<R, EXACT>(sm, W, ra, rb, ha, hb, a, b, v3<R>(f[0], f[1], f[2]), n64, fr);
                 }
             }
             const long long t2 = clock64();

@@ -88,6 +88,19 @@ struct Collider {
     int32_t tn_off;
 };
 
+// What the narrowphase's warp kernels read of a body whose only collider is a hull of at most 64 vertices
+// (single_hull): its transformed geometry and the topology records of its hull. A vertex record holds
+// {faces n, neighbours m, n face indices, m vertex indices} (vertex_to_faces, vertex_to_neighbors), a face
+// record {vertices n, neighbour faces m, n vertex indices, m face indices, the first vertex of each neighbour
+// face}, one byte each; records start on 128-byte lines, every record of a kind `stride` lines long.
+struct __align__(16) HullRef {
+    int32_t tv_off, tn_off;      // transformed vertices / normals
+    int32_t nv;
+    int32_t face_off;            // into face_normal (FP64 local normals)
+    int32_t vrec, frec;          // first line of the vertex / face records
+    int32_t vstride, fstride;    // lines per record
+};
+
 template <typename R>
 struct WorldView {
     // ---- batch layout --------------------------------------------------------------------
@@ -191,8 +204,11 @@ struct WorldView {
                                  //     (the narrowphase warp kernels' case)
     int32_t* work_list;          // [pair capacity] global pair slots narrowphased this frame
     int32_t* work_state;         // [pair capacity] per work item: WS_* below
-    int32_t* gjk_list;           // [pair capacity] work items needing GJK this substep (queue[2] of them)
-    int32_t* hit_list;           // [pair capacity] work items needing a manifold this substep (queue[3])
+    const HullRef* hull_ref;     // [bodies] of single_hull bodies
+    const uint8_t* topo_rec;     // topology records of the distinct topologies (HullRef)
+    int4* gjk_list;              // [pair capacity] work items needing GJK this substep (queue[2] of them):
+                                 //     work item, pair slot, the two bodies
+    int4* hit_list;              // [pair capacity] work items needing a manifold this substep (queue[3])
     R* work_simplex;             // [16 * pair capacity] GJK simplex of a hit (a, b, c, d)
     double* work_epa;            // [4 * pair capacity] EPA normal (FP64) and penetration of a hit
     float4* pair_base;           // [pair capacity] FP32 build: (float)(x_a - x_b) of a pair slot's predicted
