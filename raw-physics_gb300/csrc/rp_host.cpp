@@ -633,6 +633,8 @@ rp_status build_device(rp_world* w) {
             refs[slot].tv_off = c.tv_off;
             refs[slot].tn_off = c.tn_off;
         }
+        w->dims.pair_cap = (int)P;
+        w->dims.general = std::any_of(single.begin(), single.begin() + (ptrdiff_t)N, [](uint8_t x) { return !x; }) ? 1 : 0;
         RP_CUDA(upload(w->d_hull_ref, refs, st));
         rec.resize(rec.size() + 512, 0);   // lanes past a record's end read on
         RP_CUDA(upload(w->d_topo_rec, rec, st));

@@ -104,6 +104,42 @@ struct Rec {
     }
 };
 
+// One Sutherland-Hodgman pass (sh_pass, without its all-inside shortcut): a lane per polygon edge, the output
+// places from two ballots. Returns the output count.
+template <typename R, bool REMOVE_ONLY>
+__device__ __forceinline__ int clip_pass(const V3<R>* in, int n, V3<R>* out, V3<R> pn, V3<R> pp, int& status) {
+    const unsigned lane = lane_id(), below = (1u << lane) - 1u;
+    int carry = 0;
+    for (int base = 0; base < n; base += WARP) {
+        const int j = base + (int)lane;
+        bool first = false, second = false;   // the edge emits its crossing (or end point), then its end point
+        V3<R> o0 = v3<R>(0, 0, 0), end = v3<R>(0, 0, 0);
+        if (j < n) {
+            end = in[j];
+            const bool ei = in_plane(pn, pp, end);
+            o0 = end;
+            first = ei;
+            if (!REMOVE_ONLY) {
+                const V3<R> start = in[j == 0 ? n - 1 : j - 1];
+                const bool si = in_plane(pn, pp, start);
+                V3<R> t;
+                if (si != ei && plane_edge(pn, pp, start, end, t)) {
+                    o0 = t;
+                    first = true;
+                    second = ei;
+                }
+            }
+        }
+        const unsigned m1 = __ballot_sync(0xffffffffu, first), m2 = REMOVE_ONLY ? 0u : __ballot_sync(0xffffffffu, second);
+        const int pos = carry + __popc(m1 & below) + __popc(m2 & below);
+        if (first) { if (pos < CLIP_MAX) out[pos] = o0; else status |= ST_CLIP_OVERFLOW; }
+        if (second) { if (pos + 1 < CLIP_MAX) out[pos + 1] = end; else status |= ST_CLIP_OVERFLOW; }
+        carry += __popc(m1) + __popc(m2);
+    }
+    __syncwarp();
+    return carry < CLIP_MAX ? carry : CLIP_MAX;
+}
+
 // convex_convex_contact_manifold (clipping.cpp:249-341) of two register hulls; sm.va / sm.vb hold the staged
 // vertices (pair frame) for the per-lane lookups.
 template <typename R, bool EXACT>
@@ -159,22 +195,14 @@ __device__ void hull_manifold(NarrowSmem<R>& sm, const WorldView<R>& W, const Re
         }
     }
     warp_argmax_first(bestE, bestK);
-    V3<R> edge_normal = v3<R>(0, 0, 0);
-    int ei = 0, ej = 0;
-    if (bestK != 0x7fffffff) {
-        const int k = bestK >> 1;
-        ei = w1[2 + nf1 + k / nn2];
-        ej = w2[2 + nf2 + k % nn2];
-        V3<R> e1 = vsub(sp1, sm.va[ei]);
-        V3<R> e2 = vsub(sp2, sm.vb[ej]);
-        edge_normal = vnorm(vcross(e1, e2));
-        if (bestK & 1) edge_normal = vinv(edge_normal);
-    }
-    R d1 = vdot(n1, normal), d2 = vdot(n2, inv_n), de = vdot(edge_normal, normal);
+    const bool edges = bestK != 0x7fffffff;
+    const R d1 = vdot(n1, normal), d2 = vdot(n2, inv_n), de = edges ? bestE : (R)0;
     if (de > d1 + (R)0.0001 && de > d2 + (R)0.0001) {
         // collision_distance_between_skew_lines (clipping.cpp:210-239)
+        const int k = edges ? bestK >> 1 : 0;
+        const V3<R> q1 = sm.va[w1[2 + nf1 + (edges ? k / nn2 : 0)]], q2 = sm.vb[w2[2 + nf2 + (edges ? k % nn2 : 0)]];
         V3<R> l1, l2;
-        const bool ok = skew_points(sp1, vsub(sm.va[ei], sp1), sp2, vsub(sm.vb[ej], sp2), l1, l2);
+        const bool ok = skew_points(sp1, vsub(edges ? q1 : sm.va[0], sp1), sp2, vsub(edges ? q2 : sm.vb[0], sp2), l1, l2);
         if (!ok && lane == 0) atomicOr(&sm.status, (int)(ST_DEGENERATE | ST_DEG_SKEW));
         push_contact(sm, fr, l1, l2, normal, ok && lane == 0);
         return;
@@ -182,14 +210,23 @@ __device__ void hull_manifold(NarrowSmem<R>& sm, const WorldView<R>& W, const Re
     bool ref1 = d1 > d2;
     // screen in FP32: |d1 - d2| below 1e-5 (within the float subtraction's rounding: 1.1e-5 covers it)
     if (!EXACT && fabsf((float)d1 - (float)d2) < 1.1e-5f) {
-        // nearly parallel faces: the reference face is decided from FP64 normals by one lane
-        // (see convex_convex_manifold)
-        int r = 0;
-        if (lane == 0) {
-            const V3<double> m1 = face_normal64(W, ha.face_off + f1, body_a), m2 = face_normal64(W, hb.face_off + f2, body_b);
-            r = vdot(m1, normal64) > vdot(m2, vinv(normal64)) ? 1 : 0;
+        // Nearly parallel faces: the reference decides d1 > d2 in FP64, below FP32 resolution of the dot products.
+        // For unit vectors 1 - <m, n> = |m - n|^2 / 2, which FP32 resolves far better near zero: with each
+        // vector within e of its FP64 value, |m - n|^2 is within 2 e |m - n| + e^2. e = 2e-6 covers the FP32
+        // normals (about 5e-7 off). The FP64 comparison (7500 cycles of one lane, 30 % of this kernel before)
+        // is left for faces parallel to within about 1e-5 rad, one face a lane.
+        const V3<R> u1 = vsub(n1, normal), u2 = vadd(n2, normal);
+        const R q1 = vdot(u1, u1), q2 = vdot(u2, u2), e = (R)2e-6;
+        if (fabsf((float)(q1 - q2)) > (float)((R)2 * e * (sqrtf((float)q1) + sqrtf((float)q2)) + (R)4 * e * e)) {
+            ref1 = q1 < q2;
+        } else {
+            double d = 0.0;
+            if (lane < 2) {
+                const V3<double> m = face_normal64(W, lane ? hb.face_off + f2 : ha.face_off + f1, lane ? body_b : body_a);
+                d = vdot(m, lane ? vinv(normal64) : normal64);
+            }
+            ref1 = __shfl_sync(0xffffffffu, d, 0) > __shfl_sync(0xffffffffu, d, 1);
         }
-        ref1 = __shfl_sync(0xffffffffu, r, 0) != 0;
     }
     // incident polygon and boundary planes (build_boundary_planes, clipping.cpp:121-134)
     const Rec rr = ref1 ? r1 : r2, ri = ref1 ? r2 : r1;
@@ -221,23 +258,22 @@ __device__ void hull_manifold(NarrowSmem<R>& sm, const WorldView<R>& W, const Re
             bool out = false;
             if (k < npl) {
                 const V3<R> pn = sm.u.clip.pn[k], pp = sm.u.clip.pp[k];
-                for (int j = 0; j < n; ++j) out = out || !in_plane(pn, pp, sm.u.clip.buf[cur][j]);
+                for (int j = 0; j < n; ++j) out |= !in_plane(pn, pp, sm.u.clip.buf[cur][j]);
             }
             todo &= __ballot_sync(0xffffffffu, out);
             if (!todo) break;
             const int p = base + __ffs(todo) - 1;
-            const int m = sh_pass(sm.u.clip.buf[cur], n, sm.u.clip.buf[cur ^ 1], sm.u.clip.pn[p], sm.u.clip.pp[p], false, st);
-            if (m >= 0) { n = m; cur ^= 1; }
+            n = clip_pass<R, false>(sm.u.clip.buf[cur], n, sm.u.clip.buf[cur ^ 1], sm.u.clip.pn[p], sm.u.clip.pp[p], st);
+            cur ^= 1;
             // the planes after p see the new polygon
             todo = (npl - base >= 32 ? 0xffffffffu : (1u << (npl - base)) - 1u) & ~((2u << (p - base)) - 1u);
         }
     }
-    const int rf = ref1 ? f1 : f2;
-    const V3<R> ref_n = vinv(rn[rf]);
+    const V3<R> ref_n = vinv(ref1 ? n1 : n2);
     const V3<R> ref_p = rv[rr[2]];
     if (n > 0) {
-        const int m = sh_pass(sm.u.clip.buf[cur], n, sm.u.clip.buf[cur ^ 1], ref_n, ref_p, true, st);
-        if (m >= 0) { n = m; cur ^= 1; }
+        n = clip_pass<R, true>(sm.u.clip.buf[cur], n, sm.u.clip.buf[cur ^ 1], ref_n, ref_p, st);
+        cur ^= 1;
     }
     if (st && lane == 0) atomicOr(&sm.status, (int)st);
     clipped_contacts<R, EXACT>(sm, fr, sm.u.clip.buf[cur], n, ref1, ref_n, ref_p, normal);

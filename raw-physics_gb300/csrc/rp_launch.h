@@ -20,6 +20,8 @@ struct PipeConfig {
 };
 struct PipeDims {
     int nbodies = 0, ncolliders = 0, next = 0, num_scenes = 0;
+    int pair_cap = 0;    // pair slots of the world
+    int general = 0;     // some body is not a single hull of at most 64 vertices
     int node_words = 0;  // words of the node bitmap (node capacity / 32 + 1)
     int grid_mode = 0;   // one large scene: cooperative setup and sweeps
     // scene-resident solves (k_solve) in place of the sweep, velocity and predict kernels: the scenes in two

@@ -27,6 +27,7 @@
 #include "rp_scene.cuh"
 #include "rp_hullpair.cuh"
 #include "rp_launch.h"
+#include <algorithm>
 
 namespace rp {
 
@@ -971,6 +972,9 @@ struct PipeLauncher {
             return cudaEventRecord(marks->ev[marks->n++], st);
         };
         const double h = P.dt / P.num_substeps;
+        // no more blocks than the pair scratch can give work to: a small world's kernels are launch and latency
+        const int by_thread = std::max(1, std::min(c.cull_blocks, (d.pair_cap + PIPE_BLOCK - 1) / PIPE_BLOCK));
+        const int warp_blocks = std::max(1, (d.pair_cap + PIPE_WARPS - 1) / PIPE_WARPS);
         const int body_blocks = (d.nbodies + d.next + PIPE_BLOCK - 1) / PIPE_BLOCK + 1;
         const int col_blocks = (d.ncolliders * c.transform_group + PIPE_BLOCK - 1) / PIPE_BLOCK + 1;
         if ((e = mark(-1)) != cudaSuccess) return e;
@@ -985,27 +989,29 @@ struct PipeLauncher {
                 if ((e = mark(PH_PREDICT)) != cudaSuccess) return e;
             }
             if (P.enable_collisions || sub == 0 || !d.solve) {   // without collisions it only empties the pairs' contacts
-                k_cull<R><<<c.cull_blocks, PIPE_BLOCK, 0, st>>>(W, P.enable_collisions);
+                k_cull<R><<<by_thread, PIPE_BLOCK, 0, st>>>(W, P.enable_collisions);
                 if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(PH_NARROW)) != cudaSuccess) return e;
             }
             if (P.enable_collisions) {
                 k_transform<R, EXACT><<<col_blocks, PIPE_BLOCK, 0, st>>>(W, c.transform_group);
                 if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(PH_TRANSFORM)) != cudaSuccess) return e;
-                k_gjk<R, EXACT><<<c.gjk_blocks, PIPE_BLOCK, gjk_smem(), st>>>(W);
+                k_gjk<R, EXACT><<<std::min(c.gjk_blocks, warp_blocks), PIPE_BLOCK, gjk_smem(), st>>>(W);
                 if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(PH_GJK)) != cudaSuccess) return e;
-                k_epa<R, EXACT><<<c.epa_blocks, PIPE_BLOCK, narrow_smem(), st>>>(W);
+                k_epa<R, EXACT><<<std::min(c.epa_blocks, warp_blocks), PIPE_BLOCK, narrow_smem(), st>>>(W);
                 if ((e = cudaGetLastError()) != cudaSuccess) return e;
                 if (!EXACT) {
-                    k_epa_finish<R><<<c.cull_blocks, PIPE_BLOCK, 0, st>>>(W);
+                    k_epa_finish<R><<<by_thread, PIPE_BLOCK, 0, st>>>(W);
                     if ((e = cudaGetLastError()) != cudaSuccess) return e;
                 }
                 if ((e = mark(PH_EPA)) != cudaSuccess) return e;
-                k_manifold<R, EXACT, false><<<c.manifold_blocks, PIPE_BLOCK, narrow_smem(), st>>>(W);
+                k_manifold<R, EXACT, false><<<std::min(c.manifold_blocks, warp_blocks), PIPE_BLOCK, narrow_smem(), st>>>(W);
                 if ((e = cudaGetLastError()) != cudaSuccess) return e;
-                k_manifold<R, EXACT, true><<<c.general_blocks, PIPE_BLOCK, narrow_smem(), st>>>(W);
-                if ((e = cudaGetLastError()) != cudaSuccess) return e;
+                if (d.general) {   // compound bodies, spheres or large hulls in the world
+                    k_manifold<R, EXACT, true><<<std::min(c.general_blocks, warp_blocks), PIPE_BLOCK, narrow_smem(), st>>>(W);
+                    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+                }
                 if (!EXACT) {
-                    k_fallback<R><<<c.sms, 32, fallback_smem(), st>>>(W);
+                    k_fallback<R><<<std::min(c.sms, std::max(1, d.pair_cap)), 32, fallback_smem(), st>>>(W);
                     if ((e = cudaGetLastError()) != cudaSuccess) return e;
                 }
                 if ((e = mark(PH_MANIFOLD)) != cudaSuccess) return e;
@@ -1033,11 +1039,13 @@ struct PipeLauncher {
         return cudaSuccess;
     }
 
+    static int narrow_launches(const PipeDims& d) { return (EXACT ? 5 : 7) + (d.general ? 1 : 0); }
+
     static int launches_per_frame(const StepParams& P, const PipeDims& d) {
         if (d.solve)
             return 2 + (P.enable_collisions ? 0 : 1) +
-                   P.num_substeps * ((P.enable_collisions ? (EXACT ? 6 : 8) : 0) + (d.solve_count[0] > 0) + (d.solve_count[1] > 0));
-        const int per_sub = 2 + (P.enable_collisions ? (EXACT ? 6 : 8) : 1) + P.num_pos_iters + 1;
+                   P.num_substeps * ((P.enable_collisions ? narrow_launches(d) : 0) + (d.solve_count[0] > 0) + (d.solve_count[1] > 0));
+        const int per_sub = 2 + (P.enable_collisions ? narrow_launches(d) : 1) + P.num_pos_iters + 1;
         return 1 + P.num_substeps * per_sub;
     }
 };
