@@ -1,6 +1,6 @@
 // The collision half of the adjoint substep (rp_adjoint.cuh): broad phase and islands of a frame,
 // hull transforms, GJK, EPA, contact-manifold clipping, the contact constraint solve and the
-// velocity solver, for one scene on one thread.
+// velocity solver. A pair, a contact, a body is the work of one thread.
 //
 // Every function is written once for both passes. The scalar pass (S = double) repeats the all-FP64
 // step's arithmetic operation for operation, so its trajectory is the FP64 step's. The taped pass
@@ -30,15 +30,20 @@ __device__ inline bool g_broad_hit(const double* xi, const double* xj, double ri
     return __dsqrt_rn(d2) <= __dadd_rn(__dadd_rn(ri, rj), 0.1);
 }
 
+// by one warp
 __device__ inline int g_broad(const AdjointScene& sc, const AdjGeom& G, const double* st, int2* pairs) {
+    const int lane = threadIdx.x & 31;
     int n = 0;
     for (int i = 0; i < sc.nb; ++i)
-        for (int j = i + 1; j < sc.nb; ++j) {
-            if (!g_broad_hit(st + 13 * i, st + 13 * j, G.radius[sc.body0 + i], G.radius[sc.body0 + j])) continue;
-            if (n < sc.pair_cap) pairs[n] = make_int2(i, j);
-            else sc.status[0] |= ADJ_ST_PAIRS;
-            ++n;
+        for (int j0 = i + 1; j0 < sc.nb; j0 += 32) {
+            const int j = j0 + lane;
+            const bool hit = j < sc.nb && g_broad_hit(st + 13 * i, st + 13 * j, G.radius[sc.body0 + i], G.radius[sc.body0 + j]);
+            const unsigned mask = __ballot_sync(0xffffffffu, hit);
+            const int at = n + __popc(mask & ((1u << lane) - 1u));
+            if (hit && at < sc.pair_cap) pairs[at] = make_int2(i, j);
+            n += __popc(mask);
         }
+    if (n > sc.pair_cap && lane == 0) atomicOr(sc.status, ADJ_ST_PAIRS);
     return min(n, sc.pair_cap);
 }
 
@@ -102,10 +107,9 @@ struct GScene {
     V3<double>* tvv;          // their values
     V3<double>* tnv;
     GCon<S>* con;
-    int ncon;
+    int ncon, con_cap;
     GClip<S>* clip;
     GEpa* epa;
-    int* stamp;               // substep counter shared by both passes (bodies transformed in a substep carry its number)
 };
 
 template <typename S>
@@ -117,11 +121,12 @@ struct GHull {
     const V3<double>* tnv;
 };
 
-// collider_update (collider.cpp:409-446) for every hull of body i. The model matrix is translation
+// collider_update (collider.cpp:409-446) for every hull of body i: its vertices and faces first,
+// first + step and so on. The model matrix is translation
 // times rotation with a (0 0 0 1) last row, so the reference's 4x4 product and divide by w reduce,
 // operation for operation, to (v.x R00 + v.y R01) + v.z R02 + x and (R00 n.x + R01 n.y) + R02 n.z.
 template <typename S>
-__device__ __noinline__ void g_transform(const AdjointScene& sc, const AdjGeom& G, const GBody<S>& B, int i, GScene<S>& X) {
+__device__ __noinline__ void g_transform(const AdjointScene& sc, const AdjGeom& G, const GBody<S>& B, int i, GScene<S>& X, int first, int step) {
     const M3<S> R = qmat3(B.q);
     const int slot = sc.body0 + i;
     for (int c = G.col_start[slot]; c < G.col_start[slot + 1]; ++c) {
@@ -129,7 +134,7 @@ __device__ __noinline__ void g_transform(const AdjointScene& sc, const AdjGeom& 
         if (col.type != COL_HULL) continue;
         const Shape sh = G.shapes[col.shape];
         const int tv = col.tv_off - sc.tv0, tn = col.tn_off - sc.tn0;
-        for (int k = 0; k < sh.nv; ++k) {
+        for (int k = first; k < sh.nv; k += step) {
             const double* v = G.shape_verts + 3 * (sh.vert_off + k);
             const S vx = S(v[0]), vy = S(v[1]), vz = S(v[2]);
             const V3<S> t = v3<S>(vx * R.d[0][0] + vy * R.d[0][1] + vz * R.d[0][2] + B.x.x,
@@ -138,7 +143,7 @@ __device__ __noinline__ void g_transform(const AdjointScene& sc, const AdjGeom& 
             X.tv[tv + k] = t;
             X.tvv[tv + k] = vval(t);
         }
-        for (int k = 0; k < sh.nf; ++k) {
+        for (int k = first; k < sh.nf; k += step) {
             const double* nn = G.face_normal + 3 * (sh.face_off + k);
             const S nx = S(nn[0]), ny = S(nn[1]), nz = S(nn[2]);
             const V3<S> t = vnorm(v3<S>(R.d[0][0] * nx + R.d[0][1] * ny + R.d[0][2] * nz,
@@ -397,8 +402,7 @@ template <typename S>
 __device__ void g_push_contact(const AdjointScene& sc, GScene<S>& X, const GBody<S>& A, const GBody<S>& B, int ia, int ib,
                                const V3<S>& p1, const V3<S>& p2, const V3<S>& n, int& npair) {
     // clipping_contact_to_collision_constraint (pbd.cpp:408-424); at most CMAX per body pair
-    if (npair >= CMAX) { sc.status[0] |= ADJ_ST_CONTACTS; return; }
-    if (X.ncon >= sc.contact_cap) { sc.status[0] |= ADJ_ST_CONTACTS; return; }
+    if (npair >= CMAX || X.ncon >= X.con_cap) { atomicOr(sc.status, ADJ_ST_CONTACTS); return; }
     GCon<S>& c = X.con[X.ncon++];
     ++npair;
     c.r1 = qrotate(qinverse(A.q), vsub(p1, A.x));
@@ -472,7 +476,7 @@ __device__ __noinline__ void g_manifold(const AdjointScene& sc, const AdjGeom& G
         const S rA = -dd1.x * p2.x + dd1.x * p1.x - dd1.y * p2.y + dd1.y * p1.y - dd1.z * p2.z + dd1.z * p1.z;
         const S rB = -dd2.x * p2.x + dd2.x * p1.x - dd2.y * p2.y + dd2.y * p1.y - dd2.z * p2.z + dd2.z * p1.z;
         const S den = (nA * mB) - (nB * mA);
-        if (val(den) == 0.0) { sc.status[0] |= ADJ_ST_NARROW; return; }
+        if (val(den) == 0.0) { atomicOr(sc.status, ADJ_ST_NARROW); return; }
         const S nn = ((rA * mB) - (rB * mA)) / den;
         const S mm = ((nA * rB) - (nB * rA)) / den;
         const V3<S> l1 = vadd(p1, vscale(mm, dd1));
@@ -512,7 +516,7 @@ __device__ __noinline__ void g_manifold(const AdjointScene& sc, const AdjGeom& G
         const int m = g_sh_pass(C.buf[cur], n, C.buf[cur ^ 1], ref_n, ref_p, true, overflow);
         if (m >= 0) { n = m; cur ^= 1; }
     }
-    if (overflow) sc.status[0] |= ADJ_ST_NARROW;
+    if (overflow) atomicOr(sc.status, ADJ_ST_NARROW);
     // contacts from the kept points (clipping.cpp:302-327)
     for (int k = 0; k < n; ++k) {
         const V3<S> pt = C.buf[cur][k];
@@ -542,7 +546,7 @@ __device__ __noinline__ void g_pair_contacts(const AdjointScene& sc, const AdjGe
     for (int ca = G.col_start[sa]; ca < G.col_start[sa + 1]; ++ca)
         for (int cb = G.col_start[sb]; cb < G.col_start[sb + 1]; ++cb) {
             const Collider c1 = G.colliders[ca], c2 = G.colliders[cb];
-            if (c1.type != COL_HULL || c2.type != COL_HULL) { sc.status[0] |= ADJ_ST_UNSUPPORTED; continue; }
+            if (c1.type != COL_HULL || c2.type != COL_HULL) { atomicOr(sc.status, ADJ_ST_UNSUPPORTED); continue; }
             GHull<S> h1, h2;
             h1.sh = G.shapes[c1.shape];
             h2.sh = G.shapes[c2.shape];
@@ -557,7 +561,7 @@ __device__ __noinline__ void g_pair_contacts(const AdjointScene& sc, const AdjGe
             int npoly = 0;
             bool overflow = false;
             if (!g_epa(*X.epa, h1, h2, s, ix, face, npoly, overflow)) {
-                if (overflow) sc.status[0] |= ADJ_ST_NARROW;
+                if (overflow) atomicOr(sc.status, ADJ_ST_NARROW);
                 continue;
             }
             const V3<S> normal = g_epa_normal(*X.epa, face, npoly, h1, h2);

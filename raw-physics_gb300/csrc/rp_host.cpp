@@ -18,6 +18,7 @@
 #include <map>
 #include <memory>
 #include <thread>
+#include <type_traits>
 #include <string>
 #include <vector>
 
@@ -155,7 +156,7 @@ struct rp_world {
     DevBuf d_node_vpred, d_node_vlevel, d_vlevel_count, d_vlevel_fill, d_vlevel_nodes, d_scene_vlevels, d_act_list, d_act_count;
 
     // phase-major pipeline
-    DevBuf d_adj_scenes, d_adj_data, d_adj_ext;   // adjoint scratch
+    DevBuf d_adj_scenes, d_adj_workers, d_adj_data, d_adj_ext;   // adjoint scratch
     HostBuf h_state;                               // pinned staging of the body state (rp_state_set / _get)
     HostBuf h_rec;                                 // pinned staging of the state records (device-side packing)
     DevBuf d_rec, d_slot_entity;                   // the records on the device; entity of each body slot
@@ -2011,6 +2012,8 @@ rp_status rp_autotune(rp_world* w, double dt, uint32_t substeps, uint32_t iters,
     return s != RP_OK ? s : r;
 }
 
+constexpr size_t ADJ_TAPE_BYTES = (size_t)8 << 30;   // scratch of the substeps an adjoint tapes at once
+
 rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint32_t iters, int32_t collisions,
                                 uint32_t frames, uint32_t checkpoint_every, const int32_t* loss_entity, const double* target,
                                 double* loss_out, double* grad_v, double* grad_w, double* grad_mass, double* grad_friction) {
@@ -2081,16 +2084,18 @@ rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint3
     const size_t K = checkpoint_every;
     const size_t body_d = adjoint_body_bytes(false), body_a = adjoint_body_bytes(true), var = adjoint_var_bytes();
     const size_t con_d = adjoint_contact_bytes(false), con_a = adjoint_contact_bytes(true);
-    const size_t clip_d = adjoint_clip_bytes(false), clip_a = adjoint_clip_bytes(true), epa = adjoint_epa_bytes();
+    const size_t clip_d = adjoint_clip_bytes(false), clip_a = adjoint_clip_bytes(true), epa_d = adjoint_epa_bytes(false), epa_a = adjoint_epa_bytes(true);
     struct Off {
-        size_t ckpt, seg, work, deact, active, aseg, pairs, npairs, uf, awake, stamp, tvd, tnd, tva, tna, tvv, tnv, cond, cona,
-            clipd, clipa, epa, grad, ginv, gmu, loss, status, prof, bd, ba, lamd, lama, tab, td, tadj;
-        int cap, pcap, ccap;
+        size_t ckpt, seg, deact, active, aseg, pairs, npairs, uf, awake, stamp, nlev, tvd, tnd, cond, stage, clipd, epa, grad, ginv,
+            gmu, loss, status, prof, bd, lamd, worker;
+        int ncap, mcap, pcap, ccap;
     };
     std::vector<Off> off((size_t)S);
     // the tape of one substep: bodies, joints, and with collisions the hull transforms, narrowphase
-    // and contact solves; an overflow doubles it and runs again
+    // and contact solves; an overflow makes it four times as long and runs again
     size_t tape_scale = 1;
+    int sms = 1;
+    RP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, w->device));
     rp_status result = RP_OK;
     for (int attempt = 0; attempt < 3; ++attempt) {
         size_t total = 0;
@@ -2105,11 +2110,11 @@ rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint3
             Off& o = off[(size_t)s];
             o.pcap = (int)std::min<size_t>(nb * (nb - 1) / 2 + 1, 16 * nb + 64);
             o.ccap = collisions ? (int)(32 * nb + 256) : 1;
-            const size_t cap = (600 * nb + 2500 * ne * iters + (collisions ? 8000 * nb * iters : 0) + 4096) * tape_scale;
-            o.cap = (int)std::min<size_t>((size_t)1 << 30, cap);
+            const size_t cap = (300 * nb + 1000 * ne * iters + (collisions ? 4000 * nb * iters : 0) + 4096) * tape_scale;
+            o.ncap = (int)std::min<size_t>((size_t)1 << 28, cap);
+            o.mcap = (int)std::min<size_t>((size_t)1 << 30, 4 * cap);
             o.ckpt = take(((frames + K - 1) / K + 1) * 15 * nb * 8);
             o.seg = take((K * substeps + 1) * stride);
-            o.work = take(stride);
             o.deact = take(nb * 8);
             o.active = take(nb);
             o.aseg = take(K * nb);
@@ -2118,17 +2123,13 @@ rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint3
             o.uf = take(nb * 4);
             o.awake = take(nb);
             o.stamp = take(nb * 4);
+            o.nlev = take((ne + (size_t)o.ccap) * 4);
             o.tvd = take(ntv * 24 + 8);
             o.tnd = take(ntn * 24 + 8);
-            o.tva = take(ntv * 3 * var + var);
-            o.tna = take(ntn * 3 * var + var);
-            o.tvv = take(ntv * 24 + 8);
-            o.tnv = take(ntn * 24 + 8);
             o.cond = take((size_t)o.ccap * con_d);
-            o.cona = take((size_t)o.ccap * con_a);
+            o.stage = take(collisions ? adjoint_stage_bytes() : 8);
             o.clipd = take(collisions ? clip_d : 8);
-            o.clipa = take(collisions ? clip_a : 8);
-            o.epa = take(collisions ? epa : 8);
+            o.epa = take(collisions ? epa_d : 8);
             o.grad = take(stride);
             o.ginv = take(nb * 8);
             o.gmu = take(2 * nb * 8);
@@ -2136,13 +2137,62 @@ rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint3
             o.status = take(8);
             o.prof = take(6 * 8);
             o.bd = take(nb * body_d);
-            o.ba = take(nb * body_a);
             o.lamd = take(4 * ne * 8 + 8);
-            o.lama = take(4 * ne * var + var);
-            o.tab = take((size_t)o.cap * 8);
-            o.td = take((size_t)o.cap * 16);
-            o.tadj = take((size_t)o.cap * 8);
         }
+        // One worker's scratch of scene s from byte `at` on (in *a when given); its size
+        auto worker = [&](int s, char* at, AdjointWorker* a) -> size_t {
+            const Off& o = off[(size_t)s];
+            const int b0 = w->scene_body[(size_t)s];
+            const size_t nb = (size_t)(w->scene_body[(size_t)s + 1] - b0);
+            const size_t ne = (size_t)(ext_start[(size_t)s + 1] - ext_start[(size_t)s]);
+            const size_t ntv = (size_t)(tv_of[(size_t)b0 + nb] - tv_of[(size_t)b0]);
+            const size_t ntn = (size_t)(tn_of[(size_t)b0 + nb] - tn_of[(size_t)b0]);
+            const size_t nc = (size_t)o.ncap, mc = (size_t)o.mcap;
+            size_t used = 0;
+            auto part = [&](auto*& p, size_t bytes) {
+                if (a) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(at + used);
+                used += (bytes + 255) & ~(size_t)255;
+            };
+            AdjointWorker none;
+            AdjointWorker& v = a ? *a : none;
+            part(v.bodies, nb * body_a);
+            part(v.lam, 4 * ne * var + var);
+            part(v.tv, ntv * 3 * var + var);
+            part(v.tn, ntn * 3 * var + var);
+            part(v.tv_val, ntv * 24 + 8);
+            part(v.tn_val, ntn * 24 + 8);
+            part(v.con, (size_t)o.ccap * con_a);
+            part(v.clip, collisions ? clip_a : 8);
+            part(v.epa, collisions ? epa_a : 8);
+            part(v.stamp, nb * 4);
+            part(v.out, 13 * nb * 4);
+            part(v.edge, mc * 8);
+            part(v.partial, mc * 8);
+            part(v.level, nc * 4);
+            part(v.pos, nc * 4);
+            part(v.level_start, (nc + 2) * 4);
+            part(v.child_start, (nc + 2) * 4);
+            part(v.cursor, nc * 4);
+            part(v.child, mc * 4);
+            part(v.child_partial, mc * 8);
+            part(v.adj, nc * 8);
+            part(v.counts, 8);
+            part(v.cycles, 8);
+            v.ncap = o.ncap;
+            v.mcap = o.mcap;
+            return used;
+        };
+        // Substeps taped at once, of each scene: enough for four blocks on every SM (a block is one thread's
+        // serial work), no more than a segment has, within ADJ_TAPE_BYTES of scratch; the groups of a segment
+        // are of one size as nearly as can be.
+        size_t each = 0;
+        for (int s = 0; s < S; ++s) each += worker(s, nullptr, nullptr);
+        const int nsub = (int)(std::min<size_t>(K, frames) * substeps);
+        int G = std::max(1, std::min(nsub, 4 * sms / S));
+        while (G > 1 && each * (size_t)G > ADJ_TAPE_BYTES) --G;
+        const int groups = (nsub + G - 1) / G;
+        G = (nsub + groups - 1) / groups;
+        for (int s = 0; s < S; ++s) off[(size_t)s].worker = take((size_t)G * worker(s, nullptr, nullptr));
         const size_t inputs = (13 + 1 + 12 + 3 + 6 + 1) * N * 8 + 2 * N + 256;
         RP_CUDA(w->d_adj_data.ensure(total + inputs + 1024));
         RP_CUDA(w->d_adj_ext.ensure(std::max<size_t>(ext.size(), 1) * sizeof(ExtConstraint)));
@@ -2170,6 +2220,8 @@ rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint3
         if (!ext.empty())
             RP_CUDA(cudaMemcpyAsync(w->d_adj_ext.p, ext.data(), ext.size() * sizeof(ExtConstraint), cudaMemcpyHostToDevice,
                                     w->stream));
+        RP_CUDA(w->d_adj_workers.ensure((size_t)S * (size_t)G * sizeof(AdjointWorker)));
+        std::vector<AdjointWorker> workers((size_t)S * (size_t)G);
         std::vector<AdjointScene> scenes((size_t)S);
         for (int s = 0; s < S; ++s) {
             AdjointScene& a = scenes[(size_t)s];
@@ -2198,7 +2250,6 @@ rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint3
             a.contact_cap = o.ccap;
             a.checkpoints = (double*)(base + o.ckpt);
             a.segment = (double*)(base + o.seg);
-            a.work = (double*)(base + o.work);
             a.deact = (double*)(base + o.deact);
             a.active = (uint8_t*)(base + o.active);
             a.active_seg = (uint8_t*)(base + o.aseg);
@@ -2209,14 +2260,10 @@ rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint3
             a.stamp = (int*)(base + o.stamp);
             a.tv_d = base + o.tvd;
             a.tn_d = base + o.tnd;
-            a.tv_a = base + o.tva;
-            a.tn_a = base + o.tna;
-            a.tv_val = (double*)(base + o.tvv);
-            a.tn_val = (double*)(base + o.tnv);
+            a.node_level = (int*)(base + o.nlev);
             a.con_d = base + o.cond;
-            a.con_a = base + o.cona;
+            a.stage_d = base + o.stage;
             a.clip_d = base + o.clipd;
-            a.clip_a = base + o.clipa;
             a.epa = base + o.epa;
             a.grad_state = (double*)(base + o.grad);
             a.grad_invm = (double*)(base + o.ginv);
@@ -2225,15 +2272,14 @@ rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint3
             a.status = (int*)(base + o.status);
             a.prof = (long long*)(base + o.prof);
             a.bodies_d = base + o.bd;
-            a.bodies_a = base + o.ba;
             a.lam_d = (double*)(base + o.lamd);
-            a.lam_a = base + o.lama;
-            a.tape_ab = (int2*)(base + o.tab);
-            a.tape_d = (double2*)(base + o.td);
-            a.tape_adj = (double*)(base + o.tadj);
-            a.tape_cap = o.cap;
+            const size_t bytes = worker(s, nullptr, nullptr);
+            for (int k = 0; k < G; ++k)
+                worker(s, base + o.worker + (size_t)k * bytes, &workers[(size_t)s * (size_t)G + (size_t)k]);
         }
         RP_CUDA(cudaMemcpyAsync(w->d_adj_scenes.p, scenes.data(), scenes.size() * sizeof(AdjointScene),
+                                cudaMemcpyHostToDevice, w->stream));
+        RP_CUDA(cudaMemcpyAsync(w->d_adj_workers.p, workers.data(), workers.size() * sizeof(AdjointWorker),
                                 cudaMemcpyHostToDevice, w->stream));
         AdjointParams P;
         P.dt = dt;
@@ -2253,8 +2299,10 @@ rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint3
         P.geom.csr_data = w->d_csr_data.as<int32_t>();
         P.geom.col_start = w->d_col_start.as<int32_t>();
         P.geom.radius = w->d_radius.as<double>();
-        RP_CUDA(adjoint_launch(w->d_adj_scenes.as<AdjointScene>(), S, P, w->stream));
-        w->launches++;
+        int launches = 0;
+        RP_CUDA(adjoint_launch(w->d_adj_scenes.as<AdjointScene>(), S, w->d_adj_workers.as<AdjointWorker>(), G, P, w->stream,
+                               &launches));
+        w->launches += launches;
         // results
         std::vector<double> g(13 * N), gi(N), gmu(2 * N);
         std::vector<int> status((size_t)S, 0);

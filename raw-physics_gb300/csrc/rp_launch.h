@@ -55,7 +55,7 @@ struct PipeMarks {
     int pipe_launches_##SUF(const StepParams& P, const PipeDims& d);                                          \
     size_t pipe_solve_smem_##SUF(int bodies, int joints);
 
-// Adjoint of the substep (rp_adjoint.cu): one scene per thread.
+// Adjoint of the substep (rp_adjoint.cu): a block per scene, and a worker per substep taped at once.
 struct AdjGeom {                           // the world's collider geometry (FP64), shared by all scenes
     const Collider* colliders;
     const Shape* shapes;
@@ -94,8 +94,7 @@ struct AdjointScene {
     int tv0, tn0, ntv, ntn;                // the scene's transformed vertices / normals (global offset, count)
     int pair_cap, contact_cap;
     double* checkpoints;                   // [(frames / K + 1) * 15 nb]: state, deactivation time, awake flag
-    double* segment;                       // [(K * substeps + 1) * 13 nb]
-    double* work;                          // [13 nb]
+    double* segment;                       // [(K * substeps + 1) * 13 nb] start states of the segment's substeps
     double* deact;                         // [nb]
     uint8_t* active;                       // [nb]
     uint8_t* active_seg;                   // [K nb] awake flags of each frame of the segment
@@ -103,13 +102,13 @@ struct AdjointScene {
     int* npairs;                           // [K]
     int* uf;                               // [nb] union-find parents
     uint8_t* awake;                        // [nb]
-    int* stamp;                            // [nb] substep of the body's last hull transform
+    int* stamp;                            // [nb] scratch of the scalar substep
+    int* node_level;                       // [ne + contact_cap] levels of its solves
     void* tv_d; void* tn_d;                // transformed vertices / normals, scalar pass
-    void* tv_a; void* tn_a;                // taped pass
-    double* tv_val; double* tn_val;        // their values (every decision is taken on these)
-    void* con_d; void* con_a;              // [contact_cap] contact constraints of the substep
-    void* clip_d; void* clip_a;            // clipping buffers
-    void* epa;                             // EPA polytope
+    void* con_d;                           // [contact_cap] contact constraints of the substep
+    void* stage_d;                         // [warps CMAX] contacts of a round of pairs
+    void* clip_d;                          // [warps] clipping buffers
+    void* epa;                             // [warps] EPA polytopes
     double* grad_state;                    // [13 nb] adjoint of the state (ends as d loss / d start)
     double* grad_invm;                     // [nb]
     double* grad_mu;                       // [2 nb] static, dynamic friction
@@ -118,21 +117,44 @@ struct AdjointScene {
     long long* prof;                       // [6] SM cycles: forward, segment recompute, taped substeps, reverse
                                            //     sweeps; largest and total tape entries of a substep
     void* bodies_d;                        // nb bodies of the scalar pass
-    void* bodies_a;                        // nb bodies of the taped pass
     double* lam_d;                         // [4 ne]
-    void* lam_a;                           // [4 ne] taped lambdas
-    int2* tape_ab;
-    double2* tape_d;
-    double* tape_adj;
-    int tape_cap;
 };
-cudaError_t adjoint_launch(AdjointScene* d_scenes, int nscenes, const AdjointParams& P, cudaStream_t st);
+// Scratch of one taped substep
+struct AdjointWorker {
+    void* bodies;                          // nb bodies of the taped pass
+    void* lam;                             // [4 ne] taped lambdas
+    void* tv; void* tn;                    // transformed vertices / normals
+    double* tv_val; double* tn_val;        // their values (every decision is taken on these)
+    void* con;                             // [contact_cap]
+    void* clip;
+    void* epa;
+    int* stamp;                            // [nb] bodies whose hulls are transformed
+    int* out;                              // [13 nb] tape entries of the end state
+    int2* edge;                            // [mcap] parent, child
+    double* partial;                       // [mcap] d child / d parent
+    int* level;                            // [ncap]
+    int* pos;                              // [ncap] place in the reverse sweep's order
+    int* level_start;                      // [ncap + 1] first place of a level, highest level first
+    int* child_start;                      // [ncap + 1] first child edge of a place
+    int* cursor;                           // [ncap]
+    int* child;                            // [mcap] places of the children
+    double* child_partial;                 // [mcap]
+    double* adj;                           // [ncap] adjoints by place
+    int* counts;                           // [2] entries (-1: corrupt), levels
+    long long* cycles;                     // [1]
+    int ncap, mcap;
+};
+// workers: G per scene, in scene order; *launches counts the kernels
+cudaError_t adjoint_launch(const AdjointScene* scenes, int nscenes, const AdjointWorker* workers, int G, const AdjointParams& P,
+                           cudaStream_t st, int* launches);
 size_t adjoint_body_bytes(bool tape);
 size_t adjoint_var_bytes();
-// scratch sizes of the contact pipeline: contact record, clipping buffers (per pass), EPA polytope
+// scratch sizes of the contact pipeline: contact record, a round's contacts, and of the taped pass (a worker)
+// or the scalar pass (a block) the clipping buffers and EPA polytopes
 size_t adjoint_contact_bytes(bool tape);
 size_t adjoint_clip_bytes(bool tape);
-size_t adjoint_epa_bytes();
+size_t adjoint_stage_bytes();
+size_t adjoint_epa_bytes(bool tape);
 
 // colliders_update (collider.cpp:409-446) of every hull collider at its body's current pose, in FP64
 // with the reference's arithmetic (built with -fmad=false in rp_kernels_f64.cu): world-space vertices
