@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(PIPE_BLOCK) k_predict(WorldView<R> W, int nbod
     if (frame_abandoned(W.status)) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
     for (int b = t; b < nbodies; b += n) {
-        predict_stage<R, EXACT, true>(W, b, h);
+        predict_body<R, EXACT, true, true>(W, b, h);
     }
     for (int e = t; e < next; e += n)
         for (int k = 0; k < 4; ++k) W.ext_lambda[4 * (size_t)e + k] = 0.0;
@@ -948,7 +948,7 @@ struct PipeLauncher {
         auto launch = [&](int k, cudaStream_t s, int reset) -> cudaError_t {
             const SolveRoom room = solve_room(d.solve_bodies[k], d.solve_joints[k]);
             k_solve<R, EXACT><<<d.solve_count[k], k == 0 ? SOLVE_BLOCK : SOLVE_BLOCK / 2, solve_smem<R>(room), s>>>(
-                W, d.solve_scenes + (k ? d.solve_count[0] : 0), room, h, P.num_pos_iters, alike, predict, reset);
+                W, d.solve_scenes + (k ? d.solve_count[0] : 0), room, h, 1.0 / h, P.num_pos_iters, alike, predict, reset);
             return cudaGetLastError();
         };
         if (d.solve_count[0] == 0) return launch(1, st, 1);

@@ -135,7 +135,7 @@ __device__ __noinline__ void solve_scene_general(const WorldView<R>& W, int s, d
 // which records the schedules for rp_last_schedule instead); reset: this launch also zeroes the
 // next substep's narrowphase counters.
 template <typename R, bool EXACT>
-__global__ void __launch_bounds__(SOLVE_BLOCK, 2) k_solve(WorldView<R> W, const int32_t* scenes, SolveRoom room, double h, int iters,
+__global__ void __launch_bounds__(SOLVE_BLOCK, 2) k_solve(WorldView<R> W, const int32_t* scenes, SolveRoom room, double h, double inv_h, int iters,
                                                           int alike, int predict, int reset) {
     if (frame_abandoned(W.status)) return;
     extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -330,22 +330,41 @@ __global__ void __launch_bounds__(SOLVE_BLOCK, 2) k_solve(WorldView<R> W, const 
             }
         }
     }
-    // velocity update
+    // velocity update: the corrections into the FP64 pose, then the velocities of awake bodies from it
     for (int b = tid; b < nb; b += nt) {
         const int g = b0 + b;
-        if constexpr (EXACT) {
-            velocity_body<R, EXACT>(W, g, h);
-        } else {
+        double4_32a p = W.pos[g], q = W.rot[g];
+        const double4_32a pp = W.prev_pos[g], pq = W.prev_rot[g];
+        const bool moves = !fixed[b] && W.active[g];
+        V3<R> v = v3<R>(W.vel[3 * g], W.vel[3 * g + 1], W.vel[3 * g + 2]);
+        V3<R> w = v3<R>(W.omega[3 * g], W.omega[3 * g + 1], W.omega[3 * g + 2]);
+        V3<R> pv = v3<R>(W.prev_vel[3 * g], W.prev_vel[3 * g + 1], W.prev_vel[3 * g + 2]);
+        V3<R> pw = v3<R>(W.prev_omega[3 * g], W.prev_omega[3 * g + 1], W.prev_omega[3 * g + 2]);
+        if constexpr (!EXACT) {
             const float4 dx = general ? W.sdx[g] : s_dx[b], dq = general ? W.sdq[g] : s_dq[b];
-            const float invm = s_dx[b].w, rest = s_pd[b].w;
-            const float4 q = fold_pose(W, g, dx, dq, s_q[b]);
-            velocity_body<R, EXACT>(W, g, h);
-            if (general) W.pose_f[2 * g + 1] = q;
-            s_q[b] = q;
-            s_dq[b] = make_float4(W.vel[3 * g], W.vel[3 * g + 1], W.vel[3 * g + 2], 0.f);
-            s_pd[b] = make_float4(W.omega[3 * g], W.omega[3 * g + 1], W.omega[3 * g + 2], rest);
-            s_pq[b] = make_float4(W.prev_vel[3 * g], W.prev_vel[3 * g + 1], W.prev_vel[3 * g + 2], 0.f);
-            s_dx[b] = make_float4(W.prev_omega[3 * g], W.prev_omega[3 * g + 1], W.prev_omega[3 * g + 2], invm);
+            if (fold_pose(p, q, dx, dq)) {
+                W.pos[g] = p;
+                W.rot[g] = q;
+                s_q[b] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
+            }
+            if (general) W.pose_f[2 * g + 1] = s_q[b];
+        }
+        if (moves) {
+            pv = v;
+            pw = w;
+            W.prev_vel[3 * g] = v.x; W.prev_vel[3 * g + 1] = v.y; W.prev_vel[3 * g + 2] = v.z;
+            W.prev_omega[3 * g] = w.x; W.prev_omega[3 * g + 1] = w.y; W.prev_omega[3 * g + 2] = w.z;
+            velocity_values<R, EXACT>(p, q, pp, pq, inv_h, v, w);
+            if (EXACT || general) {   // otherwise stored after the velocity sweep
+                W.vel[3 * g] = v.x; W.vel[3 * g + 1] = v.y; W.vel[3 * g + 2] = v.z;
+                W.omega[3 * g] = w.x; W.omega[3 * g + 1] = w.y; W.omega[3 * g + 2] = w.z;
+            }
+        }
+        if constexpr (!EXACT) {
+            s_dq[b] = make_float4(v.x, v.y, v.z, 0.f);
+            s_pd[b] = make_float4(w.x, w.y, w.z, s_pd[b].w);
+            s_pq[b] = make_float4(pv.x, pv.y, pv.z, 0.f);
+            s_dx[b] = make_float4(pw.x, pw.y, pw.z, s_dx[b].w);
         }
     }
     __syncthreads();
@@ -404,7 +423,7 @@ __global__ void __launch_bounds__(SOLVE_BLOCK, 2) k_solve(WorldView<R> W, const 
     if (!predict) return;
     if (tid == 0) W.contact_count[s] = 0;
     if (reset && blockIdx.x == 0 && tid == 0) reset_narrow_queue(W);
-    for (int b = tid; b < nb; b += nt) predict_stage<R, EXACT, false>(W, b0 + b, h);
+    for (int b = tid; b < nb; b += nt) predict_body<R, EXACT, true, false>(W, b0 + b, h);
 }
 
 }  // namespace rp

@@ -92,9 +92,10 @@ __device__ __forceinline__ Duo duo_of_lane() {
 // one FP64 Newton step (relative error ~1e-14), instead of an FP64 square root and four FP64
 // divisions, which GB300 executes at a small fraction of its FP32 rate.
 __device__ __forceinline__ Qt<double> qnormalize_fast(Qt<double> q) {
-    double n2 = q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
+    // (roundings spelled out: every kernel that normalises gives the same bits)
+    const double n2 = __fma_rn(q.w, q.w, __fma_rn(q.z, q.z, __fma_rn(q.x, q.x, __dmul_rn(q.y, q.y))));
     double r = (double)rsqrtf((float)n2);
-    r = r * (1.5 - 0.5 * n2 * r * r);
+    r = __dmul_rn(r, __fma_rn(-__dmul_rn(__dmul_rn(0.5, n2), r), r, 1.5));
     return qt<double>(q.x * r, q.y * r, q.z * r, q.w * r);
 }
 
@@ -382,20 +383,23 @@ __device__ __forceinline__ float4 fbase4(const WorldView<float>& W, int a, int b
 }
 
 
-// The position sweep's corrections d, q into the FP64 pose (x += dx, q = normalize(q + dq)), and the
-// FP32 orientation copy the velocity sweep reads (returned; q0 before); bodies the sweep did not touch keep
-// their pose.
-__device__ __forceinline__ float4 fold_pose(const WorldView<float>& W, int b, float4 d, float4 q, float4 q0) {
-    if (d.x == 0.f && d.y == 0.f && d.z == 0.f && q.x == 0.f && q.y == 0.f && q.z == 0.f && q.w == 0.f) return q0;
-    const double4_32a p4 = W.pos[b], q4 = W.rot[b];
+// The position sweep's corrections d, q into the FP64 pose (x += dx, q = normalize(q + dq)); false for a body
+// the sweep did not touch, which keeps its pose.
+__device__ __forceinline__ bool fold_pose(double4_32a& p4, double4_32a& q4, float4 d, float4 q) {
+    if (d.x == 0.f && d.y == 0.f && d.z == 0.f && q.x == 0.f && q.y == 0.f && q.z == 0.f && q.w == 0.f) return false;
     const Qt<double> nq = qnormalize_fast(qt<double>(q4.x + (double)q.x, q4.y + (double)q.y, q4.z + (double)q.z,
                                                      q4.w + (double)q.w));
-    W.pos[b] = make_double4_32a(p4.x + (double)d.x, p4.y + (double)d.y, p4.z + (double)d.z, 0.0);
-    W.rot[b] = make_double4_32a(nq.x, nq.y, nq.z, nq.w);
-    return make_float4((float)nq.x, (float)nq.y, (float)nq.z, (float)nq.w);
+    p4 = make_double4_32a(p4.x + (double)d.x, p4.y + (double)d.y, p4.z + (double)d.z, 0.0);
+    q4 = make_double4_32a(nq.x, nq.y, nq.z, nq.w);
+    return true;
 }
+// for one body in global memory, with the FP32 orientation copy the velocity sweep reads
 __device__ __forceinline__ void fold_body(const WorldView<float>& W, int b) {
-    W.pose_f[2 * b + 1] = fold_pose(W, b, W.sdx[b], W.sdq[b], W.pose_f[2 * b + 1]);
+    double4_32a p = W.pos[b], q = W.rot[b];
+    if (!fold_pose(p, q, W.sdx[b], W.sdq[b])) return;
+    W.pos[b] = p;
+    W.rot[b] = q;
+    W.pose_f[2 * b + 1] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
 }
 
 // JOINT in the functions below: the contact solve and the joint solves fuse some of their sums in
@@ -704,40 +708,11 @@ static __device__ void fext_solve(const Duo& D, FBody& B, const double4_32a* rot
     }
 }
 
-// FP32 build: after predict, the FP32 copies the substep's sweeps work from (the pose, the predict
-// step's displacement and the previous orientation) and, for the sweeps that keep them in global memory
-// (DELTAS), zero sweep deltas.
-template <bool DELTAS = true>
-__device__ __forceinline__ void stage_body(const WorldView<float>& W, int b) {
-    const double4_32a p = W.pos[b], q = W.rot[b], pp = W.prev_pos[b], pq = W.prev_rot[b];
-    W.pose_f[2 * b] = make_float4((float)p.x, (float)p.y, (float)p.z, 0.f);
-    W.pose_f[2 * b + 1] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
-    if (DELTAS) {
-        W.sdx[b] = make_float4(0.f, 0.f, 0.f, 0.f);
-        W.sdq[b] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    W.pred_d[b] = make_float4((float)(p.x - pp.x), (float)(p.y - pp.y), (float)(p.z - pp.z), 0.f);
-    W.prev_qf[b] = make_float4((float)pq.x, (float)pq.y, (float)pq.z, (float)pq.w);
-}
-
-// --------------------------------------------------------------------------------------------
-// Predict (pbd.cpp:537-577) for one body
+// Predict (pbd.cpp:537-577): the pose x, q and velocities v, w of an awake body after a step h under force F and
+// torque T.
 template <typename R, bool EXACT>
-__device__ void predict_body(const WorldView<R>& W, int b, double h) {
-    double4_32a p = W.pos[b], q4 = W.rot[b];
-    W.prev_pos[b] = p;
-    W.prev_rot[b] = q4;
-    if (W.fixed[b] || !W.active[b]) return;
-    V3<double> x = v3<double>(p.x, p.y, p.z);
-    Qt<double> q = qt<double>(q4.x, q4.y, q4.z, q4.w);
-    V3<R> v = v3<R>(W.vel[3 * b], W.vel[3 * b + 1], W.vel[3 * b + 2]);
-    V3<R> w = v3<R>(W.omega[3 * b], W.omega[3 * b + 1], W.omega[3 * b + 2]);
-    V3<R> F = v3<R>((R)W.force[3 * b], (R)W.force[3 * b + 1], (R)W.force[3 * b + 2]);
-    V3<R> T = v3<R>((R)W.torque[3 * b], (R)W.torque[3 * b + 1], (R)W.torque[3 * b + 2]);
-    R invm = W.inv_mass[b];
-    R si[6], sI[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) { si[i] = W.inv_inertia[6 * b + i]; sI[i] = W.inertia[6 * b + i]; }
+__device__ __forceinline__ void predict_values(V3<double>& x, Qt<double>& q, V3<R>& v, V3<R>& w, V3<R> F, V3<R> T, R invm,
+                                               const R (&si)[6], const R (&sI)[6], double h) {
     R hR = (R)h;
     v = vadd(v, vscale(hR * invm, F));
     if (EXACT) x = vadd(x, v3cast<double>(vscale(hR, v)));
@@ -756,38 +731,82 @@ __device__ void predict_body(const WorldView<R>& W, int b, double h) {
         q.z = q.z + (double)(s * qd.z); q.w = q.w + (double)(s * qd.w);
         q = qnormalize_fast(q);
     }
-    W.pos[b] = make_double4_32a(x.x, x.y, x.z, 0.0);
-    W.rot[b] = make_double4_32a(q.x, q.y, q.z, q.w);
-    W.vel[3 * b] = v.x; W.vel[3 * b + 1] = v.y; W.vel[3 * b + 2] = v.z;
-    W.omega[3 * b] = w.x; W.omega[3 * b + 1] = w.y; W.omega[3 * b + 2] = w.z;
 }
 
-// PBD velocity update (pbd.cpp:623-643) for one body
+// Predict for one body, and with STAGE the copies the substep's phases work from: the FP32 pose, and in the
+// FP32 build the predict step's displacement, the previous orientation and, for the sweeps that keep them
+// in global memory (DELTAS), zero sweep deltas. Every load is issued before the first use.
+template <typename R, bool EXACT, bool STAGE, bool DELTAS>
+__device__ __forceinline__ void predict_body(const WorldView<R>& W, int b, double h) {
+    const double4_32a p = W.pos[b], q4 = W.rot[b];
+    const bool moves = !W.fixed[b] && W.active[b];
+    V3<R> v = v3<R>(W.vel[3 * b], W.vel[3 * b + 1], W.vel[3 * b + 2]);
+    V3<R> w = v3<R>(W.omega[3 * b], W.omega[3 * b + 1], W.omega[3 * b + 2]);
+    const V3<R> F = v3<R>((R)W.force[3 * b], (R)W.force[3 * b + 1], (R)W.force[3 * b + 2]);
+    const V3<R> T = v3<R>((R)W.torque[3 * b], (R)W.torque[3 * b + 1], (R)W.torque[3 * b + 2]);
+    const R invm = W.inv_mass[b];
+    R si[6], sI[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) { si[i] = W.inv_inertia[6 * b + i]; sI[i] = W.inertia[6 * b + i]; }
+    V3<double> x = v3<double>(p.x, p.y, p.z);
+    Qt<double> q = qt<double>(q4.x, q4.y, q4.z, q4.w);
+    W.prev_pos[b] = p;
+    W.prev_rot[b] = q4;
+    if (moves) {
+        predict_values<R, EXACT>(x, q, v, w, F, T, invm, si, sI, h);
+        W.pos[b] = make_double4_32a(x.x, x.y, x.z, 0.0);
+        W.rot[b] = make_double4_32a(q.x, q.y, q.z, q.w);
+        W.vel[3 * b] = v.x; W.vel[3 * b + 1] = v.y; W.vel[3 * b + 2] = v.z;
+        W.omega[3 * b] = w.x; W.omega[3 * b + 1] = w.y; W.omega[3 * b + 2] = w.z;
+    }
+    if (!STAGE) return;
+    W.pose_f[2 * b] = make_float4((float)x.x, (float)x.y, (float)x.z, 0.f);
+    W.pose_f[2 * b + 1] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
+    if constexpr (!EXACT) {
+        if (DELTAS) {
+            W.sdx[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+            W.sdq[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        W.pred_d[b] = make_float4((float)(x.x - p.x), (float)(x.y - p.y), (float)(x.z - p.z), 0.f);
+        W.prev_qf[b] = make_float4((float)q4.x, (float)q4.y, (float)q4.z, (float)q4.w);
+    }
+}
+
+// PBD velocity update (pbd.cpp:623-643): the velocities of a body that went from pose pp, pq4 to p, q4 in a
+// substep; inv_h = 1 / h.
+template <typename R, bool EXACT>
+__device__ __forceinline__ void velocity_values(double4_32a p, double4_32a q4, double4_32a pp, double4_32a pq4, double inv_h, V3<R>& v,
+                                                V3<R>& w) {
+    V3<double> dx = vsub(v3<double>(p.x, p.y, p.z), v3<double>(pp.x, pp.y, pp.z));
+    if constexpr (EXACT) {
+        v = vscale(inv_h, dx);
+        Qt<double> dq = qmul(qt<double>(q4.x, q4.y, q4.z, q4.w), qinverse(qt<double>(pq4.x, pq4.y, pq4.z, pq4.w)));
+        const double two = 2.0 * inv_h;   // the reference's 2 / h: the same double
+        w = (dq.w >= 0.0) ? vscale(two, v3<double>(dq.x, dq.y, dq.z)) : vscale(-two, v3<double>(dq.x, dq.y, dq.z));
+    } else {
+        // only the pose differences are formed in FP64. With q = q_prev + d,
+        // q * q_prev^-1 = (0, 0, 0, |q_prev|^2) + d * q_prev^-1, so its vector part is d * q_prev^-1.
+        const R ih = (R)inv_h;
+        v = vscale(ih, v3cast<R>(dx));
+        // (differences of rounded poses, not fused with the normalisation they come from)
+        Qt<R> d = qt<R>((R)__dsub_rn(q4.x, pq4.x), (R)__dsub_rn(q4.y, pq4.y), (R)__dsub_rn(q4.z, pq4.z), (R)__dsub_rn(q4.w, pq4.w));
+        Qt<R> qpi = qinverse(qt<R>((R)pq4.x, (R)pq4.y, (R)pq4.z, (R)pq4.w));
+        Qt<R> dq = qmul(d, qpi);
+        R sgn = ((R)1 + dq.w >= (R)0) ? (R)2 * ih : (R)-2 * ih;
+        w = v3<R>(sgn * dq.x, sgn * dq.y, sgn * dq.z);
+    }
+}
+
+// for one body, from global memory
 template <typename R, bool EXACT>
 __device__ void velocity_body(const WorldView<R>& W, int b, double h) {
     if (W.fixed[b] || !W.active[b]) return;
 #pragma unroll
     for (int i = 0; i < 3; ++i) { W.prev_vel[3 * b + i] = W.vel[3 * b + i]; W.prev_omega[3 * b + i] = W.omega[3 * b + i]; }
-    double4_32a p = W.pos[b], pp = W.prev_pos[b], q4 = W.rot[b], pq4 = W.prev_rot[b];
-    V3<double> dx = vsub(v3<double>(p.x, p.y, p.z), v3<double>(pp.x, pp.y, pp.z));
-    if (EXACT) {
-        V3<double> v = vscale(1.0 / h, dx);
-        Qt<double> dq = qmul(qt<double>(q4.x, q4.y, q4.z, q4.w), qinverse(qt<double>(pq4.x, pq4.y, pq4.z, pq4.w)));
-        V3<double> w = (dq.w >= 0.0) ? vscale(2.0 / h, v3<double>(dq.x, dq.y, dq.z)) : vscale(-2.0 / h, v3<double>(dq.x, dq.y, dq.z));
-        W.vel[3 * b] = (R)v.x; W.vel[3 * b + 1] = (R)v.y; W.vel[3 * b + 2] = (R)v.z;
-        W.omega[3 * b] = (R)w.x; W.omega[3 * b + 1] = (R)w.y; W.omega[3 * b + 2] = (R)w.z;
-        return;
-    }
-    // FP32 build: only the pose differences are formed in FP64. With q = q_prev + d,
-    // q * q_prev^-1 = (0, 0, 0, |q_prev|^2) + d * q_prev^-1, so its vector part is d * q_prev^-1.
-    const R inv_h = (R)(1.0 / h);
-    V3<R> v = vscale(inv_h, v3cast<R>(dx));
-    Qt<R> d = qt<R>((R)(q4.x - pq4.x), (R)(q4.y - pq4.y), (R)(q4.z - pq4.z), (R)(q4.w - pq4.w));
-    Qt<R> qpi = qinverse(qt<R>((R)pq4.x, (R)pq4.y, (R)pq4.z, (R)pq4.w));
-    Qt<R> dq = qmul(d, qpi);
-    R sgn = ((R)1 + dq.w >= (R)0) ? (R)2 * inv_h : (R)-2 * inv_h;
+    V3<R> v, w;
+    velocity_values<R, EXACT>(W.pos[b], W.rot[b], W.prev_pos[b], W.prev_rot[b], 1.0 / h, v, w);
     W.vel[3 * b] = v.x; W.vel[3 * b + 1] = v.y; W.vel[3 * b + 2] = v.z;
-    W.omega[3 * b] = sgn * dq.x; W.omega[3 * b + 1] = sgn * dq.y; W.omega[3 * b + 2] = sgn * dq.z;
+    W.omega[3 * b] = w.x; W.omega[3 * b + 1] = w.y; W.omega[3 * b + 2] = w.z;
 }
 
 // world_tensor with its roundings spelled out

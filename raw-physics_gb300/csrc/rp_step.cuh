@@ -1336,19 +1336,6 @@ __device__ void sweep_levels(const WorldView<R>& W, const G& g, int s, R hR) {
     }
 }
 
-// predict and the substep's FP32 copies of one body (phase-major form)
-template <typename R, bool EXACT, bool DELTAS>
-__device__ __forceinline__ void predict_stage(const WorldView<R>& W, int b, double h) {
-    predict_body<R, EXACT>(W, b, h);
-    if constexpr (EXACT) {
-        const double4_32a p = W.pos[b], q = W.rot[b];
-        W.pose_f[2 * b] = make_float4((float)p.x, (float)p.y, (float)p.z, 0.f);
-        W.pose_f[2 * b + 1] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
-    } else {
-        stage_body<DELTAS>(W, b);
-    }
-}
-
 // the work counters of a substep's narrowphase (phase-major form), and the substep count
 template <typename R>
 __device__ __forceinline__ void reset_narrow_queue(const WorldView<R>& W) {
@@ -1379,8 +1366,7 @@ __device__ void step_scene(const WorldView<R>& W, const G& g, int s, const StepP
     const int e0 = W.scene_ext[s], e1 = W.scene_ext[s + 1];
     for (int sub = 0; sub < P.num_substeps; ++sub) {
         for (int b = b0 + g.rank(); b < b1; b += g.size()) {
-            predict_body<R, EXACT>(W, b, h);
-            if constexpr (!EXACT) stage_body(W, b);
+            predict_body<R, EXACT, !EXACT, true>(W, b, h);
         }
         for (int e = e0 + g.rank(); e < e1; e += g.size())
             for (int k = 0; k < 4; ++k) W.ext_lambda[4 * (size_t)e + k] = 0.0;
