@@ -164,7 +164,7 @@ struct rp_world {
     double adj_prof[6] = {0, 0, 0, 0, 0, 0};      // last adjoint's slowest scene (rp_adjoint_profile)
     DevBuf d_pose_f, d_body_scene, d_col_body, d_scene_order, d_gjk_list, d_hit_list, d_work_list, d_work_state, d_work_simplex, d_work_epa, d_queue, d_work_off, d_work_face, d_fallback, d_tstamp, d_tlist, d_single_hull, d_pair_base, d_solve_scenes, d_hull_ref, d_topo_rec;
     int mode = RP_MODE_AUTO;          // RP_MODE_*: how a frame is launched
-    int solo_nodes = 512;             // tunable: grid sweeps run levels up to this size on one CTA
+    int solo_nodes = 0;               // tunable: grid sweeps run levels up to this size on one CTA (0: the default)
     int cta_from = 0;                 // tunable: batched sweeps give a whole CTA to scenes of this cost or more (0: none)
     std::vector<int64_t> order_cost;  // sweep cost of the scenes in scene_order (decreasing)
     int cta_scenes = 0;               // how many leading scenes of scene_order that is
@@ -1965,7 +1965,9 @@ rp_status rp_autotune(rp_world* w, double dt, uint32_t substeps, uint32_t iters,
         w->layout_gen++;   // recapture the frame graph with the new launch shapes
     };
     const int cta0 = w->pipe.sweep_cta ? 1 : w->cta_from;
-    int best[4] = {RP_MODE_PHASED, 4, cta0, 512};
+    const bool fp64 = w->precision == RP_PRECISION_FP64;
+    const int group0 = transform_group_for(fp64, w->dims.ncolliders, w->num_sms), solo0 = fp64 ? SOLO_NODES_FP64 : SOLO_NODES;
+    int best[4] = {RP_MODE_PHASED, group0, cta0, solo0};
     float best_ms = 0.f;
     // each candidate timed twice (the faster run counts); a later candidate replaces the best only
     // when it is at least 1 % faster, so timing noise does not move the choice off the default
@@ -1983,23 +1985,23 @@ rp_status rp_autotune(rp_world* w, double dt, uint32_t substeps, uint32_t iters,
         return RP_OK;
     };
     // coordinate search: launch mode, then the hull-transform group, then the sweep layout
-    s = consider(RP_MODE_PHASED, 4, cta0, 512);
-    if (s == RP_OK) s = consider(RP_MODE_PERSISTENT, 4, cta0, 512);
+    s = consider(RP_MODE_PHASED, group0, cta0, solo0);
+    if (s == RP_OK) s = consider(RP_MODE_PERSISTENT, group0, cta0, solo0);
     if (s == RP_OK && best[0] == RP_MODE_PHASED) {
-        for (int g : {8, 16, 32})
-            if (s == RP_OK) s = consider(RP_MODE_PHASED, g, cta0, 512);
+        for (int g : {4, 8, 16, 32})
+            if (s == RP_OK && g != group0) s = consider(RP_MODE_PHASED, g, cta0, solo0);
         const int g = best[1];
         if (w->grid_mode) {
-            for (int solo : {128, 256, 1024, 2048})
+            for (int solo : {fp64 ? 64 : 128, 256, 1024, 2048})
                 if (s == RP_OK) s = consider(RP_MODE_PHASED, g, cta0, solo);
         } else {
             // the sweeps' scene assignment: every scene a warp, every scene a CTA, or the largest a CTA
             for (int cta : {0, 1, 96, 160, 256, 384})
-                if (s == RP_OK && cta != cta0) s = consider(RP_MODE_PHASED, g, cta, 512);
+                if (s == RP_OK && cta != cta0) s = consider(RP_MODE_PHASED, g, cta, solo0);
         }
     } else if (s == RP_OK && w->grid_mode) {
-        for (int solo : {128, 256, 1024, 2048})
-            if (s == RP_OK) s = consider(RP_MODE_PERSISTENT, 4, 0, solo);
+        for (int solo : {fp64 ? 64 : 128, 256, 1024, 2048})
+            if (s == RP_OK) s = consider(RP_MODE_PERSISTENT, group0, 0, solo);
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

@@ -7,12 +7,16 @@
 namespace rp {
 
 // Launch shapes of the phase-major pipeline, chosen once per device (occupancy) and per world.
+// Threads per collider in the hull transform: a warp while every SM has room for the colliders' warps at once,
+// and always in FP64, whose time is the instructions of a warp; else four.
+inline int transform_group_for(bool fp64, int colliders, int sms) { return fp64 || colliders <= 16 * sms ? 32 : 4; }
+
 struct PipeConfig {
     int sms = 0;
     int cull_blocks = 0, gjk_blocks = 0, epa_blocks = 0, manifold_blocks = 0, general_blocks = 0;
     int setup_grid_blocks = 0, sweep_grid_blocks = 0, vsweep_grid_blocks = 0, sweep_warp_blocks = 0;
     // tunable (rp_autotune): the schedule does not depend on them (FP64 results identical, FP32 to rounding)
-    int transform_group = 4;     // threads per collider in the hull transform
+    int transform_group = 0;     // threads per collider in the hull transform; 0: transform_group_for
     int sweep_cta = 0;           // batched sweeps: one CTA per scene instead of one warp per scene
     // a second stream and its fork / join events: the two size classes of k_solve run side by side
     cudaStream_t side = nullptr;

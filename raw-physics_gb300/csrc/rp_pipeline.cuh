@@ -185,8 +185,11 @@ template <typename R, bool EXACT>
 __global__ void __launch_bounds__(PIPE_BLOCK) k_predict(WorldView<R> W, int nbodies, int next, double h) {
     if (frame_abandoned(W.status)) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
-    for (int b = t; b < nbodies; b += n) {
-        predict_body<R, EXACT, true, true>(W, b, h);
+    if constexpr (EXACT) {
+        const Oct O = oct_of_lane();
+        for (int b = t >> 2; b < nbodies; b += n >> 2) oct_predict(W, O, b, h);
+    } else {
+        for (int b = t; b < nbodies; b += n) predict_body<R, EXACT, true, true>(W, b, h);
     }
     for (int e = t; e < next; e += n)
         for (int k = 0; k < 4; ++k) W.ext_lambda[4 * (size_t)e + k] = 0.0;
@@ -200,8 +203,8 @@ __global__ void __launch_bounds__(PIPE_BLOCK) k_predict(WorldView<R> W, int nbod
 
 // The hulls of the bodies k_cull listed for this substep (tlist: bodies of the pairs that go on to
 // GJK or the general path; the narrowphase reads no other transformed hull), `group` threads per
-// collider (a power of two up to 32; 4 by default: the typical hull has 8-64 vertices, so a whole
-// warp per collider would leave most lanes idle).
+// collider (a power of two up to 32; the typical hull has 8-64 vertices, so a whole warp per collider
+// leaves lanes idle where there are more colliders than warps).
 template <typename R, bool EXACT>
 __global__ void __launch_bounds__(PIPE_BLOCK) k_transform(WorldView<R> W, int group) {
     if (frame_abandoned(W.status)) return;
@@ -222,9 +225,14 @@ template <typename R, bool EXACT>
 __global__ void __launch_bounds__(PIPE_BLOCK) k_velocity(WorldView<R> W, int nbodies, double h) {
     if (frame_abandoned(W.status)) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
-    for (int b = t; b < nbodies; b += n) {
-        if constexpr (!EXACT) fold_body(W, b);   // the position sweep's corrections into the FP64 pose
-        velocity_body<R, EXACT>(W, b, h);
+    if constexpr (EXACT) {
+        const Oct O = oct_of_lane();
+        for (int b = t >> 2; b < nbodies; b += n >> 2) oct_velocity(W, O, b, 1.0 / h);
+    } else {
+        for (int b = t; b < nbodies; b += n) {
+            fold_body(W, b);   // the position sweep's corrections into the FP64 pose
+            velocity_body<R, EXACT>(W, b, h);
+        }
     }
 }
 
@@ -975,8 +983,9 @@ struct PipeLauncher {
         // no more blocks than the pair scratch can give work to: a small world's kernels are launch and latency
         const int by_thread = std::max(1, std::min(c.cull_blocks, (d.pair_cap + PIPE_BLOCK - 1) / PIPE_BLOCK));
         const int warp_blocks = std::max(1, (d.pair_cap + PIPE_WARPS - 1) / PIPE_WARPS);
-        const int body_blocks = (d.nbodies + d.next + PIPE_BLOCK - 1) / PIPE_BLOCK + 1;
-        const int col_blocks = (d.ncolliders * c.transform_group + PIPE_BLOCK - 1) / PIPE_BLOCK + 1;
+        const int body_blocks = (d.nbodies * (EXACT ? 4 : 1) + d.next + PIPE_BLOCK - 1) / PIPE_BLOCK + 1;
+        const int group = c.transform_group ? c.transform_group : transform_group_for(EXACT, d.ncolliders, c.sms);
+        const int col_blocks = (d.ncolliders * group + PIPE_BLOCK - 1) / PIPE_BLOCK + 1;
         if ((e = mark(-1)) != cudaSuccess) return e;
         if (d.grid_mode) e = coop(k_setup_grid<R>, c.setup_grid_blocks, BLOCK, st, W, P.dt);
         else k_setup_cta<R><<<d.num_scenes, BLOCK, 0, st>>>(W, P.dt), e = cudaGetLastError();
@@ -993,7 +1002,7 @@ struct PipeLauncher {
                 if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(PH_NARROW)) != cudaSuccess) return e;
             }
             if (P.enable_collisions) {
-                k_transform<R, EXACT><<<col_blocks, PIPE_BLOCK, 0, st>>>(W, c.transform_group);
+                k_transform<R, EXACT><<<col_blocks, PIPE_BLOCK, 0, st>>>(W, group);
                 if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(PH_TRANSFORM)) != cudaSuccess) return e;
                 k_gjk<R, EXACT><<<std::min(c.gjk_blocks, warp_blocks), PIPE_BLOCK, gjk_smem(), st>>>(W);
                 if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(PH_GJK)) != cudaSuccess) return e;

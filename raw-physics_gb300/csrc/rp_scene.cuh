@@ -227,7 +227,9 @@ __global__ void __launch_bounds__(SOLVE_BLOCK, 2) k_solve(WorldView<R> W, const 
     }
     const bool general = sh.general != 0;
     Duo D = duo_of_lane();
-    const int nw = nt >> 5, first = ((tid & 31) >> 1) * nw + (tid >> 5), step = nt >> 1;
+    const Oct O = oct_of_lane();
+    constexpr int LANES = EXACT ? 8 : 2;   // of a node
+    const int nw = nt >> 5, first = (tid & 31) / LANES * nw + (tid >> 5), step = nt / LANES;
     const float4* contacts4 = reinterpret_cast<const float4*>(W.contacts);
     if (general) {
         solve_scene_general<R, EXACT, false>(W, s, h, iters);
@@ -266,7 +268,7 @@ __global__ void __launch_bounds__(SOLVE_BLOCK, 2) k_solve(WorldView<R> W, const 
                 }
             }
         }
-        // lane pairs take a level's nodes, consecutive nodes in different warps (a warp runs as long as its
+        // lane pairs (exact build: eight lanes) take a level's nodes, consecutive nodes in different warps (a warp runs as long as its
         // longest node)
         for (int it = 0; it < iters; ++it) {
             int lo = 0;
@@ -278,11 +280,11 @@ __global__ void __launch_bounds__(SOLVE_BLOCK, 2) k_solve(WorldView<R> W, const 
                     if constexpr (EXACT) {
                         if (r.pair < 0) {
                             double* lam = W.ext_lambda + 4 * (size_t)(e0 + r.cstart);
-                            if (it == 0 && D.side == 0) { lam[0] = 0.0; lam[1] = 0.0; lam[2] = 0.0; }
-                            __syncwarp(D.mask);
-                            ext_solve(W, D, W.ext[e0 + r.cstart], lam, h);
+                            if (it == 0 && O.lead()) { lam[0] = 0.0; lam[1] = 0.0; lam[2] = 0.0; }
+                            __syncwarp(O.oct);
+                            ext_solve(W, O, W.ext[e0 + r.cstart], lam, h);
                         } else {
-                            dsolve_pair(W, D, b0 + (D.side ? r.b : r.a), W.contacts + 12 * (size_t)r.cstart, r.nc, h);
+                            dsolve_pair(W, O, b0 + (O.side ? r.b : r.a), W.contacts + 12 * (size_t)r.cstart, r.nc, h);
                         }
                     } else {
                         const int me = D.side ? r.b : r.a;
@@ -331,7 +333,9 @@ __global__ void __launch_bounds__(SOLVE_BLOCK, 2) k_solve(WorldView<R> W, const 
         }
     }
     // velocity update: the corrections into the FP64 pose, then the velocities of awake bodies from it
-    for (int b = tid; b < nb; b += nt) {
+    if constexpr (EXACT) {
+        for (int b = tid >> 2; b < nb; b += nt >> 2) oct_velocity(W, O, b0 + b, inv_h);
+    } else for (int b = tid; b < nb; b += nt) {
         const int g = b0 + b;
         double4_32a p = W.pos[g], q = W.rot[g];
         const double4_32a pp = W.prev_pos[g], pq = W.prev_rot[g];
@@ -340,32 +344,28 @@ __global__ void __launch_bounds__(SOLVE_BLOCK, 2) k_solve(WorldView<R> W, const 
         V3<R> w = v3<R>(W.omega[3 * g], W.omega[3 * g + 1], W.omega[3 * g + 2]);
         V3<R> pv = v3<R>(W.prev_vel[3 * g], W.prev_vel[3 * g + 1], W.prev_vel[3 * g + 2]);
         V3<R> pw = v3<R>(W.prev_omega[3 * g], W.prev_omega[3 * g + 1], W.prev_omega[3 * g + 2]);
-        if constexpr (!EXACT) {
-            const float4 dx = general ? W.sdx[g] : s_dx[b], dq = general ? W.sdq[g] : s_dq[b];
-            if (fold_pose(p, q, dx, dq)) {
-                W.pos[g] = p;
-                W.rot[g] = q;
-                s_q[b] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
-            }
-            if (general) W.pose_f[2 * g + 1] = s_q[b];
+        const float4 dx = general ? W.sdx[g] : s_dx[b], dq = general ? W.sdq[g] : s_dq[b];
+        if (fold_pose(p, q, dx, dq)) {
+            W.pos[g] = p;
+            W.rot[g] = q;
+            s_q[b] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
         }
+        if (general) W.pose_f[2 * g + 1] = s_q[b];
         if (moves) {
             pv = v;
             pw = w;
             W.prev_vel[3 * g] = v.x; W.prev_vel[3 * g + 1] = v.y; W.prev_vel[3 * g + 2] = v.z;
             W.prev_omega[3 * g] = w.x; W.prev_omega[3 * g + 1] = w.y; W.prev_omega[3 * g + 2] = w.z;
             velocity_values<R, EXACT>(p, q, pp, pq, inv_h, v, w);
-            if (EXACT || general) {   // otherwise stored after the velocity sweep
+            if (general) {   // otherwise stored after the velocity sweep
                 W.vel[3 * g] = v.x; W.vel[3 * g + 1] = v.y; W.vel[3 * g + 2] = v.z;
                 W.omega[3 * g] = w.x; W.omega[3 * g + 1] = w.y; W.omega[3 * g + 2] = w.z;
             }
         }
-        if constexpr (!EXACT) {
-            s_dq[b] = make_float4(v.x, v.y, v.z, 0.f);
-            s_pd[b] = make_float4(w.x, w.y, w.z, s_pd[b].w);
-            s_pq[b] = make_float4(pv.x, pv.y, pv.z, 0.f);
-            s_dx[b] = make_float4(pw.x, pw.y, pw.z, s_dx[b].w);
-        }
+        s_dq[b] = make_float4(v.x, v.y, v.z, 0.f);
+        s_pd[b] = make_float4(w.x, w.y, w.z, s_pd[b].w);
+        s_pq[b] = make_float4(pv.x, pv.y, pv.z, 0.f);
+        s_dx[b] = make_float4(pw.x, pw.y, pw.z, s_dx[b].w);
     }
     __syncthreads();
     if (general) {
@@ -377,9 +377,9 @@ __global__ void __launch_bounds__(SOLVE_BLOCK, 2) k_solve(WorldView<R> W, const 
             const int hi = sh.cnt[1][l];
             for (int i = lo + first; i < hi; i += step) {
                 const NodeRec r = rec[ord[room.nodes + i]];
-                const int me = D.side ? r.b : r.a;
+                const int me = (EXACT ? O.side : D.side) ? r.b : r.a;
                 if constexpr (EXACT) {
-                    dvsolve_pair(W, D, b0 + me, W.contacts + 12 * (size_t)r.cstart, r.nc, h);
+                    dvsolve_pair(W, O, b0 + me, W.contacts + 12 * (size_t)r.cstart, r.nc, h);
                 } else {
                     const float4* c4 = contacts4 + 3 * (size_t)r.cstart;
                     float4 rl = c4[D.side], nn4 = c4[2];
@@ -423,7 +423,11 @@ __global__ void __launch_bounds__(SOLVE_BLOCK, 2) k_solve(WorldView<R> W, const 
     if (!predict) return;
     if (tid == 0) W.contact_count[s] = 0;
     if (reset && blockIdx.x == 0 && tid == 0) reset_narrow_queue(W);
-    for (int b = tid; b < nb; b += nt) predict_body<R, EXACT, true, false>(W, b0 + b, h);
+    if constexpr (EXACT) {
+        for (int b = tid >> 2; b < nb; b += nt >> 2) oct_predict(W, O, b0 + b, h);
+    } else {
+        for (int b = tid; b < nb; b += nt) predict_body<R, EXACT, true, false>(W, b0 + b, h);
+    }
 }
 
 }  // namespace rp

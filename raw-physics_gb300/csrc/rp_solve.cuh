@@ -1,11 +1,11 @@
 // XPBD constraint solves, integration and velocity passes on the device.
 //
 // Two lanes of a warp solve one solver node (a broad-phase pair with its contacts, or one external
-// joint), one lane per body (Duo): each lane loads its body into registers, applies the corrections in
-// the reference's order and writes it back once; nodes of one level never share a non-fixed body, so no
-// two lanes write the same body. The corrections of the two bodies differ only in sign, so the second
-// body's lane works on negated vectors (separation, normal, impulse): negation is exact, every product
-// and sum rounds as in the one-thread form, and both lanes take the same branches.
+// joint) in FP32, one lane per body (Duo; the FP64 solves are in rp_exact.cuh): each lane loads its body into
+// registers, applies the corrections in the reference's order and writes it back once; nodes of one level
+// never share a non-fixed body, so no two lanes write the same body. The corrections of the two bodies differ
+// only in sign, so the second body's lane works on negated vectors (separation, normal, impulse): negation is
+// exact, every product and sum rounds as in the one-thread form, and both lanes take the same branches.
 // What bounds a node is the instruction stream of one warp with two active lanes: a contact is
 // about a thousand dependent instructions in the one-thread form. Half of them belong to each body,
 // so the lane pair halves the stream.
@@ -112,85 +112,6 @@ __device__ __forceinline__ void q_add_normalize(Qt<double>& q, Qt<R> d, double s
     }
 }
 
-// --------------------------------------------------------------------------------------------
-// Exact build: positional corrections (pbd_base_constraints.cpp:6-123) of this lane's body. r: the
-// anchor in world axes, I: the body's world inverse inertia, dx: the separation seen from this body.
-__device__ __forceinline__ double pos_dlambda(const Duo& D, const Body<double>& B, V3<double> r, const M3<double>& I, double h,
-                                              double compliance, double lambda, V3<double> dx) {
-    const double c = vlen(dx);
-    if (c <= Tiny<double>::v) return 0.0;
-    const V3<double> n = v3<double>(dx.x / c, dx.y / c, dx.z / c);
-    const double w = B.invm + vdot(vcross(r, n), mmulv(I, vcross(r, n)));
-    const double til = compliance / (h * h);
-    return (-c - til * lambda) / (w + D.other(w) + til);
-}
-
-__device__ __forceinline__ void pos_apply(Body<double>& B, V3<double> r, const M3<double>& I, double dl, V3<double> dx) {
-    const double c = vlen(dx);
-    if (c <= Tiny<double>::v) return;
-    const V3<double> n = v3<double>(dx.x / c, dx.y / c, dx.z / c);
-    const V3<double> imp = vscale(dl, n);
-    const V3<double> a = mmulv(I, vcross(r, imp));
-    const Qt<double> dq = qmul(qt<double>(a.x, a.y, a.z, 0.0), B.q);
-    if (!B.fixed) {
-        B.x = vadd(B.x, vscale(B.invm, imp));
-        q_add_normalize(B.q, dq, 0.5);
-    }
-}
-
-// Angular corrections (pbd_base_constraints.cpp:125-227); dq seen from this body
-__device__ __forceinline__ double ang_dlambda(const Duo& D, const M3<double>& I, double h, double compliance, double lambda,
-                                              V3<double> dq) {
-    const double th = vlen(dq);
-    if (th <= Tiny<double>::v) return 0.0;
-    const V3<double> n = v3<double>(dq.x / th, dq.y / th, dq.z / th);
-    const double w = vdot(n, mmulv(I, n));
-    const double til = compliance / (h * h);
-    return (-th - til * lambda) / (w + D.other(w) + til);
-}
-
-__device__ __forceinline__ void ang_apply(Body<double>& B, const M3<double>& I, double dl, V3<double> dq) {
-    const double th = vlen(dq);
-    if (th <= Tiny<double>::v) return;
-    const V3<double> n = v3<double>(dq.x / th, dq.y / th, dq.z / th);
-    const V3<double> a = mmulv(I, vscale(-dl, n));
-    const Qt<double> q1 = qmul(qt<double>(a.x, a.y, a.z, 0.0), B.q);
-    if (!B.fixed) q_add_normalize(B.q, q1, 0.5);
-}
-
-// collision_constraint_solve (pbd.cpp:107-154). c points at the contact record
-// {r1_lc, lambda_n, r2_lc, lambda_t, normal, -}.
-static __device__ void collision_solve(const WorldView<double>& W, const Duo& D, Body<double>& B, double* c, double h, double mus) {
-    const V3<double> r_lc = v3<double>(c[4 * D.side], c[4 * D.side + 1], c[4 * D.side + 2]);
-    const V3<double> n = D.own(v3<double>(c[8], c[9], c[10]));
-    V3<double> r = qrotate(B.q, r_lc);
-    const V3<double> p0 = vadd(B.x, r);
-    const double d = vdot(vsub(p0, D.other(p0)), n);
-    if (!(d > 0.0)) return;
-    double lambda_n = c[3], lambda_t = c[7];
-    const V3<double> dx = vscale(d, n);
-    M3<double> I = world_tensor(B.q, B.Iinv);
-    double dl = pos_dlambda(D, B, r, I, h, 0.0, lambda_n, dx);
-    pos_apply(B, r, I, dl, dx);
-    lambda_n += dl;
-    r = qrotate(B.q, r_lc);
-    I = world_tensor(B.q, B.Iinv);
-    dl = pos_dlambda(D, B, r, I, h, 0.0, lambda_t, dx);
-    const double lt = lambda_t + dl;
-    if (lt > mus * lambda_n) {
-        // p1 - p1_til - (p2 - p2_til) with p_til from the previous pose (pbd.cpp:142-148)
-        const double4_32a x4 = W.prev_pos[B.idx], q4 = W.prev_rot[B.idx];
-        const V3<double> pt = vadd(v3<double>(x4.x, x4.y, x4.z), qrotate(qt<double>(q4.x, q4.y, q4.z, q4.w), r_lc));
-        const V3<double> u = vsub(vadd(B.x, r), pt);
-        const V3<double> dp = vsub(u, D.other(u));
-        pos_apply(B, r, I, dl, vsub(dp, vscale(vdot(dp, n), n)));
-        lambda_t += dl;
-    }
-    // both lanes hold the same multipliers: each writes one
-    __syncwarp(D.mask);
-    c[D.side ? 7 : 3] = D.side ? lambda_t : lambda_n;
-}
-
 // limit_angle (pbd.cpp:175-217)
 // Joint limits are evaluated in FP64 in both builds (the axes come from the FP64 orientations):
 // asin's slope diverges at |s| -> 1, so at a +-90 degree limit an FP32 s (error 1e-7) would move
@@ -231,102 +152,6 @@ __device__ __forceinline__ bool limit_may_act(V3<float> n, V3<float> n1, V3<floa
     if (phi > pi) phi -= 2.f * pi;
     if (phi < -pi) phi += 2.f * pi;
     return !(phi >= (float)lo + 0.01f && phi <= (float)hi - 0.01f);
-}
-
-// one joint limit of the exact build: the angle between n1 (first body) and n2 (second body) about n,
-// clamped to [lo, hi] (limit_angle), corrected with a zero-compliance angular solve
-__device__ __forceinline__ void limit_solve(const Duo& D, Body<double>& B, V3<double> n, V3<double> n1, V3<double> n2, double lo,
-                                            double hi, double h, double* lam) {
-    if (lo <= -PI_REF && hi >= PI_REF) return;   // the wrapped angle can never leave limits at or beyond +-pi
-    V3<double> dq;
-    if (!limit_angle<double>(n, n1, n2, lo, hi, dq)) return;
-    dq = D.own(dq);
-    const M3<double> I = world_tensor(B.q, B.Iinv);
-    const double l = *lam;
-    const double dl = ang_dlambda(D, I, h, 0.0, l, dq);
-    ang_apply(B, I, dl, dq);
-    __syncwarp(D.mask);
-    if (D.side == 0) *lam = l + dl;
-}
-
-// External constraints of the exact build (pbd.cpp:81-379), one lane per body
-static __device__ void ext_solve(const WorldView<double>& W, const Duo& D, const ExtConstraint& C, double* lam, double h) {
-    Body<double> B = load_body(W, D.side ? C.e2 : C.e1);
-    const double* rl = D.side ? C.r2 : C.r1;
-    const V3<double> r_lc = v3<double>(rl[0], rl[1], rl[2]);
-    // one positional correction with lambda lam[k]
-    auto positional = [&](int k, double compliance, V3<double> r, V3<double> dx) {
-        const M3<double> I = world_tensor(B.q, B.Iinv);
-        const double l = lam[k];
-        const double dl = pos_dlambda(D, B, r, I, h, compliance, l, dx);
-        pos_apply(B, r, I, dl, dx);
-        __syncwarp(D.mask);
-        if (D.side == 0) lam[k] = l + dl;
-    };
-    auto angular = [&](int k, V3<double> dq) {
-        const M3<double> I = world_tensor(B.q, B.Iinv);
-        const double l = lam[k];
-        const double dl = ang_dlambda(D, I, h, C.compliance, l, dq);
-        ang_apply(B, I, dl, dq);
-        __syncwarp(D.mask);
-        if (D.side == 0) lam[k] = l + dl;
-    };
-    // an axis of the first and of the second body, in both lanes
-    auto axes = [&](int k1, int k2, V3<double>& u1, V3<double>& u2) {
-        const V3<double> mine = qaxis(B.q, D.side ? k2 : k1), theirs = D.other(mine);
-        u1 = D.first(mine, theirs);
-        u2 = D.second(mine, theirs);
-    };
-    switch (C.type) {
-    case CON_POSITIONAL: {  // pbd.cpp:81-97
-        const V3<double> dist = D.own(v3<double>(C.distance[0], C.distance[1], C.distance[2]));
-        positional(0, C.compliance, qrotate(B.q, r_lc), vsub(vsub(B.x, D.other(B.x)), dist));
-    } break;
-    case CON_MUTUAL_ORIENTATION: {  // pbd.cpp:156-173
-        const Qt<double> oq = D.other(B.q);
-        const Qt<double> aux = qmul(D.first(B.q, oq), qinverse(D.second(B.q, oq)));
-        angular(0, D.own(v3<double>(2.0 * aux.x, 2.0 * aux.y, 2.0 * aux.z)));
-    } break;
-    case CON_HINGE: {  // pbd.cpp:245-299
-        V3<double> u1, u2;
-        axes(C.a1, C.a2, u1, u2);
-        angular(1, D.own(vcross(u1, u2)));
-        const V3<double> r = qrotate(B.q, r_lc), p = vadd(B.x, r);
-        positional(0, 0.0, r, vsub(p, D.other(p)));
-        if (C.limited) {
-            V3<double> n1, n2;
-            axes(C.l1, C.l2, n1, n2);
-            axes(C.a1, C.a2, u1, u2);
-            limit_solve(D, B, u1, n1, n2, C.lo, C.hi, h, lam + 2);
-        }
-    } break;
-    case CON_SPHERICAL: {  // pbd.cpp:301-379
-        const double EPS64 = 1e-50;
-        const V3<double> r = qrotate(B.q, r_lc), p = vadd(B.x, r);
-        positional(0, 0.0, r, vsub(p, D.other(p)));
-        V3<double> n1, n2;
-        axes(C.a1, C.a2, n1, n2);
-        V3<double> n = vcross(n1, n2);
-        double nl = vlen(n);
-        if (nl > EPS64) limit_solve(D, B, v3<double>(n.x / nl, n.y / nl, n.z / nl), n1, n2, C.lo, C.hi, h, lam + 1);
-        V3<double> a1, a2, b1, b2;   // on the orientations after the swing correction
-        axes(C.a1, C.a2, a1, a2);
-        axes(C.l1, C.l2, b1, b2);
-        n = vadd(a1, a2);
-        nl = vlen(n);
-        if (nl > EPS64) {
-            n = v3<double>(n.x / nl, n.y / nl, n.z / nl);
-            n1 = vsub(b1, vscale(vdot(n, b1), n));
-            n2 = vsub(b2, vscale(vdot(n, b2), n));
-            const double l1 = vlen(n1), l2 = vlen(n2);
-            if (l1 > EPS64 && l2 > EPS64)
-                limit_solve(D, B, n, v3<double>(n1.x / l1, n1.y / l1, n1.z / l1), v3<double>(n2.x / l2, n2.y / l2, n2.z / l2), C.lo2,
-                            C.hi2, h, lam + 2);
-        }
-    } break;
-    default: break;
-    }
-    store_pose(W, B);
 }
 
 // --------------------------------------------------------------------------------------------
@@ -826,7 +651,9 @@ __device__ __forceinline__ M3<float> world_tensor_f(Qt<float> q, const float S[6
     return o;
 }
 
-// contact_velocity (below) in FP32 with its roundings spelled out
+// Velocity solver for one contact (pbd.cpp:646-711) of this lane's body, its roundings spelled out: vel, om its
+// velocities, pv, pw those before the velocity update, r its anchor in world orientation, I its world inverse
+// inertia, n the normal seen from it.
 __device__ __forceinline__ void fcontact_velocity(const Duo& D, V3<float> r, const M3<float>& I, V3<float> n, float invm, bool fixed,
                                                   float lambda_n, float h, float mud, float e, V3<float>& vel, V3<float>& om,
                                                   V3<float> pv, V3<float> pw) {
@@ -850,34 +677,6 @@ __device__ __forceinline__ void fcontact_velocity(const Duo& D, V3<float> r, con
     if (!fixed) {
         vel = D.side ? add_f(vel, scale_f(invm, P)) : axpy_f(invm, P, vel);
         om = add_f(om, mulv_f(I, cross_f(r, P)));
-    }
-}
-
-// Velocity solver for one contact (pbd.cpp:646-711) of this lane's body: v, w its velocities, pv, pw
-// those before the velocity update, r its anchor in world orientation, I its world inverse inertia, n
-// the normal seen from it.
-template <typename R>
-__device__ __forceinline__ void contact_velocity(const Duo& D, V3<R> r, const M3<R>& I, V3<R> n, R invm, bool fixed, R lambda_n, R h,
-                                                 R mud, R e, V3<R>& vel, V3<R>& om, V3<R> pv, V3<R> pw) {
-    const V3<R> u = vadd(vel, vcross(om, r));
-    const V3<R> v = vsub(u, D.other(u));
-    const R vn = vdot(n, v);
-    const V3<R> vt = vsub(v, vscale(vn, n));
-    V3<R> dv = v3<R>(0, 0, 0);
-    const R fn = lambda_n / h;
-    const R x1 = mud * fabs(fn), x2 = vlen(vt);
-    R fact = (x1 < x2) ? x1 : x2;
-    dv = vadd(dv, vscale(-fact, vnorm(vt)));
-    const V3<R> ut = vadd(pv, vcross(pw, r));
-    const R vntil = vdot(n, vsub(ut, D.other(ut)));
-    const R m = -e * vntil;
-    fact = -vn + ((m < (R)0.0) ? m : (R)0.0);
-    dv = vadd(dv, vscale(fact, n));
-    const R w = invm + vdot(vcross(r, n), mmulv(I, vcross(r, n)));
-    const V3<R> P = vscale((R)1.0 / (w + D.other(w)), dv);
-    if (!fixed) {
-        vel = vadd(vel, vscale(invm, P));
-        om = vadd(om, mmulv(I, vcross(r, P)));
     }
 }
 

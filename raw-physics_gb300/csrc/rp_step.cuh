@@ -23,6 +23,7 @@
 #include "rp_world.h"
 #include "rp_narrow.cuh"
 #include "rp_solve.cuh"
+#include "rp_exact.cuh"
 #include <type_traits>
 
 namespace rp {
@@ -888,14 +889,24 @@ __device__ void transform_collider(const WorldView<R>& W, const Collider& col, i
     V3<R>* tn = (V3<R>*)(W.tnorms) + col.tn_off;
     if (EXACT) {
         const double4_32a p4 = W.pos[b], q4 = W.rot[b];
-        M4<double> M = model_matrix(qt<double>(q4.x, q4.y, q4.z, q4.w), v3<double>(p4.x, p4.y, p4.z));
+        // util_get_model_matrix_no_scale and the point transform (util.cpp:60-74, collider.cpp:414-422) without the
+        // products with the matrices' constant ones and zeros, which change no bit: 69 FP64 instructions for the
+        // matrix and 18 a vertex instead of 150 and 41
+        M3<double> M = qmat3(qt<double>(q4.x, q4.y, q4.z, q4.w));
+        const double t[3] = {p4.x, p4.y, p4.z};
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) M.d[i][j] = M.d[i][j] + t[i] * 0.0;
+        const V3<double> o = v3<double>(0.0 + t[0], 0.0 + t[1], 0.0 + t[2]);
         for (int i = lane; i < sh.nv; i += nsub) {
             const double* v = W.shape_verts + 3 * (sh.vert_off + i);
-            tv[i] = v3cast<R>(m4_point(M, v3<double>(v[0], v[1], v[2])));
+            const V3<double> m = mmulv(M, v3<double>(v[0], v[1], v[2]));
+            tv[i] = v3cast<R>(vadd(m, o));
         }
         for (int i = lane; i < sh.nf; i += nsub) {
             const double* nrm = W.face_normal + 3 * (sh.face_off + i);
-            tn[i] = v3cast<R>(vnorm(m4_dir(M, v3<double>(nrm[0], nrm[1], nrm[2]))));
+            tn[i] = v3cast<R>(vnorm(mmulv(M, v3<double>(nrm[0], nrm[1], nrm[2]))));
         }
     } else {
         Qt<R> q;
@@ -1219,46 +1230,8 @@ __device__ inline void fvsolve_node(const WorldView<float>& W, const Duo& D, int
     }
 }
 
-// Exact build: the contacts c[0, nc) of one pair on body `me` of this lane (both lanes of the pair call these
-// together), position and velocity sweep
-__device__ inline void dsolve_pair(const WorldView<double>& W, const Duo& D, int me, double* c, int nc, double h) {
-    const double mus_own = W.material[4 * me];
-    const double mus = (mus_own + D.other(mus_own)) / 2.0;
-    Body<double> B = load_body(W, me);
-    for (int i = 0; i < nc; ++i) collision_solve(W, D, B, c + 12 * i, h, mus);
-    store_pose(W, B);
-}
-
-__device__ inline void dvsolve_pair(const WorldView<double>& W, const Duo& D, int me, const double* c, int nc, double h) {
-    // anchors rotated by the current orientation (the poses do not change here)
-    const double4_32a q4 = W.rot[me];
-    const Qt<double> q = qt<double>(q4.x, q4.y, q4.z, q4.w);
-    double sI[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) sI[i] = W.inv_inertia[6 * me + i];
-    const M3<double> I = world_tensor(q, msym(sI));
-    const double invm = W.inv_mass[me];
-    const bool fixed = W.fixed[me] != 0;
-    V3<double> v = v3<double>(W.vel[3 * me], W.vel[3 * me + 1], W.vel[3 * me + 2]);
-    V3<double> w = v3<double>(W.omega[3 * me], W.omega[3 * me + 1], W.omega[3 * me + 2]);
-    const V3<double> pv = v3<double>(W.prev_vel[3 * me], W.prev_vel[3 * me + 1], W.prev_vel[3 * me + 2]);
-    const V3<double> pw = v3<double>(W.prev_omega[3 * me], W.prev_omega[3 * me + 1], W.prev_omega[3 * me + 2]);
-    const double mud_own = W.material[4 * me + 1], e_own = W.material[4 * me + 2];
-    const double mud = (mud_own + D.other(mud_own)) / (double)2.0f;
-    const double e = e_own * D.other(e_own);
-    for (int i = 0; i < nc; ++i) {
-        const double* ci = c + 12 * i;
-        const V3<double> r = qrotate(q, v3<double>(ci[4 * D.side], ci[4 * D.side + 1], ci[4 * D.side + 2]));
-        const V3<double> n = D.own(v3<double>(ci[8], ci[9], ci[10]));
-        contact_velocity(D, r, I, n, invm, fixed, ci[3], h, mud, e, v, w, pv, pw);
-    }
-    if (!fixed) {
-        W.vel[3 * me] = v.x; W.vel[3 * me + 1] = v.y; W.vel[3 * me + 2] = v.z;
-        W.omega[3 * me] = w.x; W.omega[3 * me + 1] = w.y; W.omega[3 * me + 2] = w.z;
-    }
-}
-
-__device__ inline void dsolve_node(const WorldView<double>& W, const Duo& D, int s, int k, double h) {
+// Exact build: a node by its eight lanes
+__device__ inline void dsolve_node(const WorldView<double>& W, const Oct& D, int s, int k, double h) {
     const int e0 = W.scene_ext[s], ne = W.scene_ext[s + 1] - e0;
     if (k < ne) {
         ext_solve(W, D, W.ext[e0 + k], W.ext_lambda + 4 * (size_t)(e0 + k), h);
@@ -1271,7 +1244,7 @@ __device__ inline void dsolve_node(const WorldView<double>& W, const Duo& D, int
     dsolve_pair(W, D, D.side ? pr.y : pr.x, W.contacts + 12 * (size_t)(W.scene_contact_cap[s] + W.pair_cstart[p]), nc, h);
 }
 
-__device__ inline void dvsolve_node(const WorldView<double>& W, const Duo& D, int s, int k, double h) {
+__device__ inline void dvsolve_node(const WorldView<double>& W, const Oct& D, int s, int k, double h) {
     const int ne = W.scene_ext[s + 1] - W.scene_ext[s];
     if (k < ne) return;
     const int p = W.scene_pair_cap[s] + (k - ne);
@@ -1281,18 +1254,25 @@ __device__ inline void dvsolve_node(const WorldView<double>& W, const Duo& D, in
     dvsolve_pair(W, D, D.side ? pr.y : pr.x, W.contacts + 12 * (size_t)(W.scene_contact_cap[s] + W.pair_cstart[p]), nc, h);
 }
 
-// The nodes [lo, hi) of a level by a group's threads, a lane pair per node, consecutive nodes in different
+// The nodes [lo, hi) of a level by a group's threads, LANES of them a node, consecutive nodes in different
 // warps (a warp runs as long as its longest node). alike: both bodies of a contact round alike.
 template <typename R, bool EXACT, bool VELOCITY>
 __device__ __forceinline__ void sweep_level(const WorldView<R>& W, int s, const int* nodes, int lo, int hi, int rank, int size, R h,
                                             bool alike = false) {
-    Duo D = duo_of_lane();
-    if (alike) D.second_right = false;
-    for (int i = lo + ((rank & 31) >> 1) * (size >> 5) + (rank >> 5); i < hi; i += size >> 1) {
-        if constexpr (EXACT) {
-            if (VELOCITY) dvsolve_node(W, D, s, nodes[i], h);
-            else dsolve_node(W, D, s, nodes[i], h);
-        } else {
+    constexpr int LANES = EXACT ? 8 : 2;
+    // warp w of block b is the group's warp w nblocks + b: few nodes go to different SMs first
+    const int wpb = (int)blockDim.x >> 5, nb = size / (int)blockDim.x, w = rank >> 5;
+    const int first = lo + (rank & 31) / LANES * (size >> 5) + w % wpb * nb + w / wpb;
+    if constexpr (EXACT) {
+        const Oct O = oct_of_lane();
+        for (int i = first; i < hi; i += size / LANES) {
+            if (VELOCITY) dvsolve_node(W, O, s, nodes[i], h);
+            else dsolve_node(W, O, s, nodes[i], h);
+        }
+    } else {
+        Duo D = duo_of_lane();
+        if (alike) D.second_right = false;
+        for (int i = first; i < hi; i += size / LANES) {
             if (VELOCITY) fvsolve_node(W, D, s, nodes[i], h);
             else fsolve_node(W, D, s, nodes[i], h);
         }
@@ -1306,14 +1286,15 @@ __device__ __forceinline__ void sweep_level(const WorldView<R>& W, int s, const 
 // levels that each hold at most SOLO_NODES nodes is swept by CTA 0 alone, separated by
 // __syncthreads, while the other CTAs wait at one grid barrier: the dependent chain of small levels
 // then costs a block barrier per level instead of a grid barrier. Larger levels use the whole grid.
-constexpr int SOLO_NODES = 2 * BLOCK;   // default of WorldView::solo_nodes
+// The exact build hands a level to CTA 0 only while its SM sub-partitions hold a warp (four nodes) each: more
+// warps of a sub-partition take turns at its FP64 unit, and a node takes several times a grid barrier's few us.
 
 template <typename R, bool EXACT, bool VELOCITY, class G>
 __device__ void sweep_levels(const WorldView<R>& W, const G& g, int s, R hR) {
     const SchedView<R> v = sched_view(W, s, VELOCITY ? 1 : 0);
     const int L = *(volatile int*)v.levels;
     const int* lstart = v.count;
-    const int solo = W.solo_nodes > 0 ? W.solo_nodes : SOLO_NODES;
+    const int solo = W.solo_nodes > 0 ? W.solo_nodes : (EXACT ? SOLO_NODES_FP64 : SOLO_NODES);
     int l = 0;
     while (l < L) {
         int cnt = lstart[l + 1] - lstart[l];

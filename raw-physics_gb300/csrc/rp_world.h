@@ -101,6 +101,9 @@ struct __align__(16) HullRef {
     int32_t vstride, fstride;    // lines per record
 };
 
+// default of WorldView::solo_nodes (rp_step.cuh, sweep_levels)
+constexpr int SOLO_NODES = 512, SOLO_NODES_FP64 = 16;
+
 template <typename R>
 struct WorldView {
     // ---- batch layout --------------------------------------------------------------------
@@ -228,7 +231,7 @@ struct WorldView {
     const int32_t* scene_order;  // [S] scenes by decreasing size (the order warps take them in)
     int32_t cta_scenes;          // the first cta_scenes of scene_order are swept by a whole CTA each
     int32_t max_colliders_per_body;
-    int32_t solo_nodes;          // grid sweeps: levels of at most this many nodes run on CTA 0 alone
+    int32_t solo_nodes;          // grid sweeps: levels of at most this many nodes run on CTA 0 alone (0: the default)
     // ---- control ----------------------------------------------------------------------------
     uint32_t* status;        // [S] status bits per scene
     unsigned int* barrier;   // [1] grid barrier arrival counter (zeroed before each launch sequence)
