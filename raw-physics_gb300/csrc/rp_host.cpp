@@ -1992,7 +1992,7 @@ rp_status rp_autotune(rp_world* w, double dt, uint32_t substeps, uint32_t iters,
             if (s == RP_OK && g != group0) s = consider(RP_MODE_PHASED, g, cta0, solo0);
         const int g = best[1];
         if (w->grid_mode) {
-            for (int solo : {fp64 ? 64 : 128, 256, 1024, 2048})
+            for (int solo : {64, 128, 256, 512})
                 if (s == RP_OK) s = consider(RP_MODE_PHASED, g, cta0, solo);
         } else {
             // the sweeps' scene assignment: every scene a warp, every scene a CTA, or the largest a CTA
@@ -2000,7 +2000,7 @@ rp_status rp_autotune(rp_world* w, double dt, uint32_t substeps, uint32_t iters,
                 if (s == RP_OK && cta != cta0) s = consider(RP_MODE_PHASED, g, cta, solo0);
         }
     } else if (s == RP_OK && w->grid_mode) {
-        for (int solo : {fp64 ? 64 : 128, 256, 1024, 2048})
+        for (int solo : {64, 128, 256, 512})
             if (s == RP_OK) s = consider(RP_MODE_PERSISTENT, group0, 0, solo);
     }
     cudaEventDestroy(e0);

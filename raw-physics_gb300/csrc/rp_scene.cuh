@@ -130,7 +130,7 @@ __device__ __noinline__ void solve_scene_general(const WorldView<R>& W, int s, d
     for (int it = 0; it < iters; ++it) sweep_levels<R, EXACT, false>(W, g, s, (R)h);
 }
 
-// alike: levels of at most 512 nodes round both bodies of a contact alike (the single large scene's small
+// alike: levels of at most ALIKE_NODES nodes round both bodies of a contact alike (the single large scene's small
 // levels, see sweep_levels). predict: the next substep's predict follows (false in a frame's last substep,
 // which records the schedules for rp_last_schedule instead); reset: this launch also zeroes the
 // next substep's narrowphase counters.
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(SOLVE_BLOCK, 2) k_solve(WorldView<R> W, const 
             int lo = 0;
             for (int l = 0; l < sh.L[0]; ++l) {
                 const int hi = sh.cnt[0][l];
-                if (alike) D.second_right = D.side != 0 && hi - lo > 512;
+                if (alike) D.second_right = D.side != 0 && hi - lo > ALIKE_NODES;
                 for (int i = lo + first; i < hi; i += step) {
                     const NodeRec r = rec[ord[i]];
                     if constexpr (EXACT) {

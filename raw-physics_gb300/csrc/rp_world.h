@@ -102,7 +102,9 @@ struct __align__(16) HullRef {
 };
 
 // default of WorldView::solo_nodes (rp_step.cuh, sweep_levels)
-constexpr int SOLO_NODES = 512, SOLO_NODES_FP64 = 16;
+constexpr int SOLO_NODES = 32, SOLO_NODES_FP64 = 16;
+// FP32 build: the single large scene's levels of at most this many nodes round both bodies of a contact alike
+constexpr int ALIKE_NODES = 512;
 
 template <typename R>
 struct WorldView {
