@@ -144,7 +144,7 @@ struct rp_world {
     DevBuf d_colliders, d_shapes, d_shape_verts, d_face_normal, d_shape_verts_f, d_face_normal_f, d_face_elem_start, d_face_elem, d_csr_start, d_csr_data;
     DevBuf d_tverts, d_tnorms, d_ext;
     DevBuf d_sort_key, d_sort_val, d_sort_hist, d_sort_hi;
-    DevBuf d_pair_count, d_pairs, d_row_count, d_uf_parent, d_island_awake, d_node_body, d_node_pred, d_node_level;
+    DevBuf d_pair_count, d_pairs, d_row_count, d_uf_parent, d_island_awake, d_node_body, d_node_pred, d_node_level, d_node_done;
     DevBuf d_tl_count, d_tl_start, d_tl, d_level_count, d_level_fill, d_scan_tmp, d_level_nodes, d_scene_levels,
         d_scene_nodes, d_pair_cstart, d_pair_ccount, d_contact_count, d_work, d_contacts, d_ext_lambda, d_status, d_barrier,
         d_counters, d_phase, d_kat_out, d_kat_count, d_deg;
@@ -583,6 +583,7 @@ rp_status build_device(rp_world* w) {
     RP_CUDA(w->d_node_body.ensure(std::max<size_t>(NN, 1) * 8));
     RP_CUDA(w->d_node_pred.ensure(std::max<size_t>(NN, 1) * 8));
     RP_CUDA(w->d_node_level.ensure(std::max<size_t>(NN, 1) * 4));
+    RP_CUDA(w->d_node_done.ensure(std::max<size_t>(w->grid_mode ? NN : 0, 1) * 8));
     RP_CUDA(w->d_tl_count.ensure(std::max<size_t>(N, 1) * 4));
     RP_CUDA(w->d_tl_start.ensure((N + 1) * 4));
     RP_CUDA(w->d_tl.ensure(std::max<size_t>(NN, 1) * 8));
@@ -795,6 +796,7 @@ WorldView<R> make_view(rp_world* w) {
     V.node_body = w->d_node_body.as<int32_t>();
     V.node_pred = w->d_node_pred.as<int32_t>();
     V.node_level = w->d_node_level.as<int32_t>();
+    V.node_done = w->d_node_done.as<int32_t>();
     V.body_tl_count = w->d_tl_count.as<int32_t>();
     V.body_tl_start = w->d_tl_start.as<int32_t>();
     V.body_tl = w->d_tl.as<int32_t>();

@@ -865,14 +865,14 @@ __global__ void __launch_bounds__(SWEEP_WARP_BLOCK, 4) k_sweep_warp(WorldView<R>
 }
 
 template <typename R, bool EXACT, bool VELOCITY>
-__global__ void __launch_bounds__(BLOCK) k_sweep_grid(WorldView<R> W, double h, int resched_first) {
+__global__ void __launch_bounds__(BLOCK) k_sweep_grid(WorldView<R> W, double h, int it) {
     if (frame_abandoned(W.status)) return;
     GridGroup g;
     g.bar = W.barrier;
     g.status = W.status;
     g.limit_ns = W.wait_ns;
-    if (!VELOCITY && resched_first) resched(W, g, 0);
-    sweep_levels<R, EXACT, VELOCITY>(W, g, 0, (R)h);
+    if (!VELOCITY && it == 0) resched(W, g, 0);
+    sweep_levels<R, EXACT, VELOCITY>(W, g, 0, (R)h, it);
 }
 
 }  // namespace rp
@@ -1032,7 +1032,7 @@ struct PipeLauncher {
             }
             for (int it = 0; it < P.num_pos_iters; ++it) {
                 const int first = it == 0 ? 1 : 0;   // the substep's schedules are built by its first sweep
-                if (d.grid_mode) e = coop(k_sweep_grid<R, EXACT, false>, c.sweep_grid_blocks, BLOCK, st, W, h, first);
+                if (d.grid_mode) e = coop(k_sweep_grid<R, EXACT, false>, c.sweep_grid_blocks, BLOCK, st, W, h, it);
                 else if (c.sweep_cta) k_sweep_cta<R, EXACT, false><<<d.num_scenes, BLOCK, 0, st>>>(W, h, first), e = cudaGetLastError();
                 else e = sweep_warp<false>(W, c, st, h, first);
                 if (e != cudaSuccess) return e;

@@ -679,6 +679,7 @@ struct SchedView {   // one of the two schedules of scene s
     int* list;       // [nodes] active nodes, unordered
     int* levels;     // number of levels of the scene
     int* active;     // number of active nodes of the scene
+    int* done;       // [nodes] grid sweeps only
 };
 
 template <typename R>
@@ -693,6 +694,7 @@ __device__ __forceinline__ SchedView<R> sched_view(const WorldView<R>& W, int s,
     v.list = W.act_list + (size_t)which * W.scene_node_cap[W.num_scenes] + nbase;
     v.levels = (which ? W.scene_vlevels : W.scene_levels) + s;
     v.active = W.act_count + 2 * s + which;
+    v.done = W.node_done + (size_t)which * W.scene_node_cap[W.num_scenes] + nbase;
     return v;
 }
 
@@ -828,6 +830,7 @@ __device__ void resched(const WorldView<R>& W, const G& g, int s) {
         const bool a0 = live && (k < ne || contacts);
         v0.lev[k] = a0 ? unset : -1;
         v1.lev[k] = contacts ? unset : -1;
+        if constexpr (std::is_same<G, GridGroup>::value) { v0.done[k] = 0; v1.done[k] = 0; }
         for (int side = 0; side < 2; ++side)
             if (nbody[2 * k + side] < 0) { v0.pred[2 * k + side] = -1; v1.pred[2 * k + side] = -1; }
         if (a0) v0.list[atomicAdd(v0.active, 1)] = k;
@@ -838,13 +841,15 @@ __device__ void resched(const WorldView<R>& W, const G& g, int s) {
     if (g.rank() == 0) { *v0.levels = 0; *v1.levels = 0; }
     if constexpr (std::is_same<G, GridGroup>::value) {
         if (n0 + n1 <= RESCHED_ONE_CTA) {
+            // the two schedules at once, a CTA each
+            const int other = g.nblocks() > 1 ? 1 : 0;
+            SubBlock q;
             if (g.block() == 0) {
-                SubBlock q;
-                if (n0 + n1 > 0) {
-                    relax_schedule(W, q, s, v0, n0, order);
-                    relax_schedule(W, q, s, v1, n1, order);
-                }
+                relax_schedule(W, q, s, v0, n0, order);
                 bucket_schedule(W, q, s, v0, n0, true);
+            }
+            if (g.block() == other) {
+                relax_schedule(W, q, s, v1, n1, order);
                 bucket_schedule(W, q, s, v1, n1, false);
             }
         } else {
@@ -1290,32 +1295,98 @@ __device__ __forceinline__ void sweep_level(const WorldView<R>& W, int s, const 
 // take turns. On 4096 bodies a CTA took 84 and 97 k cycles for a level of 446 nodes (position, velocity sweep),
 // the grid 29 and 15 k for 728, and a grid barrier 3 k. FP64: four nodes a warp, a warp an SM sub-partition,
 // whose FP64 unit the warps take turns at.
+//
+// A run of larger levels is swept without barriers (sweep_run): a node waits for its predecessors on its two
+// bodies instead of for the slowest node of the previous level, so that a node of 30 contacts holds up only
+// what rests on it.
+// Nodes are taken in level order, a level's by different warps first, so the node a warp waits for is one that
+// a warp of this or an earlier turn has taken, and every wait ends while all CTAs are resident (a cooperative
+// launch); a wait has the grid barrier's limits besides. done[k] = tag when node k is solved.
+template <typename R, bool EXACT, bool VELOCITY>
+__device__ void sweep_run(const WorldView<R>& W, const GridGroup& g, int s, const SchedView<R>& v, int l0, int l1, int tag, R h) {
+    constexpr int LANES = EXACT ? 8 : 2;
+    const int wpb = (int)blockDim.x >> 5, rank = g.rank() >> 5, w = rank % wpb * g.nblocks() + rank / wpb, nw = g.size() >> 5;
+    const int lane = (int)threadIdx.x & 31, slot = lane / LANES, side = EXACT ? lane >> 2 & 1 : lane & 1;
+    const Oct O = oct_of_lane();
+    Duo D = duo_of_lane();
+    unsigned* done = reinterpret_cast<unsigned*>(v.done);
+    bool gave_up = false;
+    for (int l = l0; l < l1; ++l) {
+        const int lo = v.count[l], hi = v.count[l + 1];
+        D.second_right = D.side != 0 && hi - lo > ALIKE_NODES;
+        for (int r = lo; r + w < hi; r += nw * (32 / LANES)) {
+            const int i = r + slot * nw + w;
+            const bool has = i < hi;
+            const int k = has ? v.nodes[i] : -1;
+            int p = has ? v.pred[2 * k + side] : -1;
+            if (p >= 0 && v.lev[p] < l0) p = -1;   // solved before the run
+            bool ready = p < 0 || gave_up || ld_acquire_gpu(done + p) == (unsigned)tag;
+            unsigned long long t0 = 0;
+            for (unsigned polls = 1; !__all_sync(0xffffffffu, ready); ++polls) {
+                __nanosleep(20);
+                if (!ready) ready = ld_acquire_gpu(done + p) == (unsigned)tag;
+                if ((polls & 63u) == 0u) {
+                    if (t0 == 0) t0 = global_ns();
+                    gave_up = __any_sync(0xffffffffu, global_ns() - t0 > g.limit_ns || frame_abandoned(W.status));
+                    if (gave_up) {
+                        if (lane == 0) atomicOr(W.status, (uint32_t)ST_BARRIER_TIMEOUT);
+                        ready = true;
+                    }
+                }
+            }
+            if (has && !gave_up) {
+                if constexpr (EXACT) {
+                    if (VELOCITY) dvsolve_node(W, O, s, k, h);
+                    else dsolve_node(W, O, s, k, h);
+                } else {
+                    if (VELOCITY) fvsolve_node(W, D, s, k, h);
+                    else fsolve_node(W, D, s, k, h);
+                }
+                __syncwarp(EXACT ? O.oct : D.mask);
+                if (lane % LANES == 0) {
+                    __threadfence();
+                    *reinterpret_cast<volatile unsigned*>(done + k) = (unsigned)tag;
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// pass: the position iteration, counted from 0
 template <typename R, bool EXACT, bool VELOCITY, class G>
-__device__ void sweep_levels(const WorldView<R>& W, const G& g, int s, R hR) {
+__device__ void sweep_levels(const WorldView<R>& W, const G& g, int s, R hR, int pass = 0) {
     const SchedView<R> v = sched_view(W, s, VELOCITY ? 1 : 0);
     const int L = *(volatile int*)v.levels;
     const int* lstart = v.count;
     const int solo = W.solo_nodes > 0 ? W.solo_nodes : (EXACT ? SOLO_NODES_FP64 : SOLO_NODES);
     int l = 0;
     while (l < L) {
-        int cnt = lstart[l + 1] - lstart[l];
-        if (g.nblocks() == 1 || cnt > solo) {
-            sweep_level<R, EXACT, VELOCITY>(W, s, v.nodes, lstart[l], lstart[l + 1], g.rank(), g.size(), hR,
-                                             g.nblocks() > 1 && cnt <= ALIKE_NODES);
-            g.sync();
-            ++l;
-            continue;
-        }
-        int l2 = l;
-        while (l2 < L && lstart[l2 + 1] - lstart[l2] <= solo) ++l2;
-        if (g.block() == 0) {
-            for (int k = l; k < l2; ++k) {
-                sweep_level<R, EXACT, VELOCITY>(W, s, v.nodes, lstart[k], lstart[k + 1], (int)threadIdx.x, (int)blockDim.x, hR, true);
-                __syncthreads();
+        if constexpr (std::is_same<G, GridGroup>::value) {
+            if (g.nblocks() > 1) {
+                const bool small = lstart[l + 1] - lstart[l] <= solo;
+                int l2 = l + 1;
+                while (l2 < L && (lstart[l2 + 1] - lstart[l2] <= solo) == small) ++l2;
+                if (!small && W.sweep_order == SWEEP_REFERENCE) {
+                    sweep_run<R, EXACT, VELOCITY>(W, g, s, v, l, l2, pass + 1, hR);
+                } else if (small) {
+                    for (int k = l; g.block() == 0 && k < l2; ++k) {
+                        sweep_level<R, EXACT, VELOCITY>(W, s, v.nodes, lstart[k], lstart[k + 1], (int)threadIdx.x, (int)blockDim.x, hR, true);
+                        __syncthreads();
+                    }
+                } else {
+                    l2 = l + 1;   // a colour
+                    sweep_level<R, EXACT, VELOCITY>(W, s, v.nodes, lstart[l], lstart[l2], g.rank(), g.size(), hR,
+                                                     lstart[l2] - lstart[l] <= ALIKE_NODES);
+                }
+                g.sync();
+                l = l2;
+                continue;
             }
         }
+        sweep_level<R, EXACT, VELOCITY>(W, s, v.nodes, lstart[l], lstart[l + 1], g.rank(), g.size(), hR);
         g.sync();
-        l = l2;
+        ++l;
     }
 }
 
@@ -1384,7 +1455,7 @@ __device__ void step_scene(const WorldView<R>& W, const G& g, int s, const StepP
         mark(PH_NARROW);
         resched(W, g, s);
         mark(PH_SCHEDULE);
-        for (int it = 0; it < P.num_pos_iters; ++it) sweep_levels<R, EXACT, false>(W, g, s, hR);
+        for (int it = 0; it < P.num_pos_iters; ++it) sweep_levels<R, EXACT, false>(W, g, s, hR, it);
         mark(PH_SOLVE);
         for (int b = b0 + g.rank(); b < b1; b += g.size()) {
             if constexpr (!EXACT) fold_body(W, b);

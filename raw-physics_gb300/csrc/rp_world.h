@@ -167,6 +167,7 @@ struct WorldView {
     int32_t* node_body;      // [2 * nodes] the node's two bodies (-1 when fixed)
     int32_t* node_pred;      // [2 * nodes] predecessor node on each body (-1: none)
     int32_t* node_level;     // [nodes]
+    int32_t* node_done;      // [2 * nodes] grid sweeps: the sweep that has solved a node (position, then velocity sweep)
     int32_t* body_tl_count;  // [N] timeline lengths / fill counters
     int32_t* body_tl_start;  // [N+1] timeline CSR starts (per scene relative to node base)
     int32_t* body_tl;        // [2 * nodes] timeline entries
