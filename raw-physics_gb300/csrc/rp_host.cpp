@@ -160,9 +160,13 @@ struct rp_world {
     HostBuf h_state;                               // pinned staging of the body state (rp_state_set / _get)
     HostBuf h_rec;                                 // pinned staging of the state records (device-side packing)
     DevBuf d_rec, d_slot_entity;                   // the records on the device; entity of each body slot
+    cudaEvent_t ev_hull = nullptr;                 // the vertices of a hull query are on the host
     cudaEvent_t ev_rec = nullptr;                  // the last record upload (h_rec is refilled after it)
     double adj_prof[6] = {0, 0, 0, 0, 0, 0};      // last adjoint's slowest scene (rp_adjoint_profile)
-    DevBuf d_pose_f, d_body_scene, d_col_body, d_scene_order, d_gjk_list, d_hit_list, d_work_list, d_work_state, d_work_simplex, d_work_epa, d_queue, d_work_off, d_work_face, d_fallback, d_tstamp, d_tlist, d_single_hull, d_pair_base, d_solve_scenes, d_hull_ref, d_topo_rec;
+    DevBuf d_pose_f, d_col_body, d_tables, d_hull_ref, d_gjk_list, d_hit_list, d_work_list, d_work_state, d_work_simplex, d_work_epa, d_queue, d_work_off, d_work_face, d_fallback, d_tstamp, d_tlist, d_pair_base;
+    // in d_tables
+    const int32_t *t_body_scene = nullptr, *t_scene_order = nullptr;
+    const uint8_t *t_single_hull = nullptr, *t_topo_rec = nullptr;
     int mode = RP_MODE_AUTO;          // RP_MODE_*: how a frame is launched
     int solo_nodes = 0;               // tunable: grid sweeps run levels up to this size on one CTA (0: the default)
     int cta_from = 0;                 // tunable: batched sweeps give a whole CTA to scenes of this cost or more (0: none)
@@ -230,29 +234,28 @@ std::vector<unsigned char> as_working(const std::vector<double>& v, size_t rsize
 
 rp_status sync_state_to_host(rp_world* w);
 
+// work(lo, hi) over [0, n) in up to 16 chunks on as many threads, none smaller than `least`
+template <typename Work>
+void in_chunks(size_t n, size_t least, const Work& work) {
+    const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    const size_t chunks = std::max<size_t>(1, std::min<size_t>(hw, (n + least - 1) / least));
+    std::vector<std::thread> th;
+    for (size_t c = 1; c < chunks; ++c) th.emplace_back([&work, n, c, chunks] { work(n * c / chunks, n * (c + 1) / chunks); });
+    work(0, n / chunks);
+    for (std::thread& t : th) t.join();
+}
+
 // Copies n doubles in parallel chunks (state records of a large batch are hundreds of MB: one core's
 // memcpy would dominate a frame); with `check`, also returns false if any is not finite.
 bool copy_records(double* dst, const double* src, size_t n, bool check) {
-    const size_t chunk_min = (size_t)1 << 18;
-    const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    const size_t chunks = std::max<size_t>(1, std::min<size_t>(hw, (n + chunk_min - 1) / chunk_min));
     std::atomic<bool> ok(true);
-    auto work = [&](size_t c) {
-        const size_t lo = n * c / chunks, hi = n * (c + 1) / chunks;
+    in_chunks(n, (size_t)1 << 18, [&](size_t lo, size_t hi) {
         bool good = true;
         if (check)
             for (size_t i = lo; i < hi; ++i) good = good && std::isfinite(src[i]);
         if (!good) ok = false;
         std::memcpy(dst + lo, src + lo, (hi - lo) * sizeof(double));
-    };
-    if (chunks == 1) {
-        work(0);
-    } else {
-        std::vector<std::thread> th;
-        for (size_t c = 1; c < chunks; ++c) th.emplace_back(work, c);
-        work(0);
-        for (std::thread& t : th) t.join();
-    }
+    });
     return ok;
 }
 
@@ -616,7 +619,6 @@ rp_status build_device(rp_world* w) {
             for (int32_t b = w->scene_body[(size_t)sc]; b < w->scene_body[(size_t)sc + 1]; ++b) body_scene[(size_t)b] = sc;
         for (size_t slot = 0; slot < N; ++slot)
             for (int32_t c = col_start[slot]; c < col_start[slot + 1]; ++c) col_body[(size_t)c] = (int32_t)slot;
-        RP_CUDA(upload(w->d_body_scene, body_scene, st));
         RP_CUDA(upload(w->d_slot_entity, w->slot_to_entity, st));
         RP_CUDA(upload(w->d_col_body, col_body, st));
         std::vector<uint8_t> single(std::max<size_t>(N, 1), 0);
@@ -637,10 +639,7 @@ rp_status build_device(rp_world* w) {
         }
         w->dims.pair_cap = (int)P;
         w->dims.general = std::any_of(single.begin(), single.begin() + (ptrdiff_t)N, [](uint8_t x) { return !x; }) ? 1 : 0;
-        RP_CUDA(upload(w->d_hull_ref, refs, st));
         rec.resize(rec.size() + 512, 0);   // lanes past a record's end read on
-        RP_CUDA(upload(w->d_topo_rec, rec, st));
-        RP_CUDA(upload(w->d_single_hull, single, st));
         RP_CUDA(w->d_pose_f.ensure(std::max<size_t>(N, 1) * 32));
         for (DevBuf* b : {&w->d_sdx, &w->d_sdq, &w->d_pred_d, &w->d_prev_qf}) {
             RP_CUDA(b->ensure(std::max<size_t>(N, 1) * 16));
@@ -664,7 +663,6 @@ rp_status build_device(rp_world* w) {
                    8LL * (w->scene_ext[(size_t)x + 1] - w->scene_ext[(size_t)x]);
         };
         std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return cost(x) > cost(y); });
-        RP_CUDA(upload(w->d_scene_order, order, st));
         w->order_cost.assign((size_t)S, 0);
         for (int sc = 0; sc < S; ++sc) w->order_cost[(size_t)sc] = cost(order[(size_t)sc]);
         set_cta_scenes(w);
@@ -695,8 +693,25 @@ rp_status build_device(rp_world* w) {
             }
             // one large scene of the exact build is bound by FP64 arithmetic: its sweeps keep every SM
             w->solve_fits = fits && !(w->grid_mode && w->precision == RP_PRECISION_FP64);
-            RP_CUDA(upload(w->d_solve_scenes, list, st));
-            d.solve_scenes = w->d_solve_scenes.as<int32_t>();
+            // the small tables in one upload
+            std::vector<unsigned char> blob;
+            auto put = [&](const auto& v) {
+                const size_t at = (blob.size() + 255) & ~(size_t)255, n = v.size() * sizeof(v[0]);
+                blob.resize(at + n);
+                if (n) std::memcpy(&blob[at], v.data(), n);
+                return at;
+            };
+            blob.reserve(body_scene.size() * 4 + rec.size() + single.size() + 8 * (size_t)S + 6 * 256);
+            const size_t o_scene = put(body_scene), o_rec = put(rec), o_single = put(single), o_order = put(order),
+                         o_list = put(list);
+            RP_CUDA(upload(w->d_tables, blob, st));
+            RP_CUDA(upload(w->d_hull_ref, refs, st));
+            const unsigned char* t = w->d_tables.as<unsigned char>();
+            w->t_body_scene = reinterpret_cast<const int32_t*>(t + o_scene);
+            w->t_topo_rec = t + o_rec;
+            w->t_single_hull = t + o_single;
+            w->t_scene_order = reinterpret_cast<const int32_t*>(t + o_order);
+            d.solve_scenes = reinterpret_cast<const int32_t*>(t + o_list);
         }
         RP_CUDA(w->d_queue.ensure(64));
         RP_CUDA(cudaMemsetAsync(w->d_queue.p, 0, 64, st));
@@ -827,19 +842,19 @@ WorldView<R> make_view(rp_world* w) {
     V.barrier = w->d_barrier.as<unsigned int>();
     V.counters = w->d_counters.as<unsigned long long>();
     V.phase_ns = w->d_phase.as<unsigned long long>();
-    V.body_scene = w->d_body_scene.as<int32_t>();
+    V.body_scene = w->t_body_scene;
     V.pose_f = w->d_pose_f.as<float4>();
     V.sdx = w->d_sdx.as<float4>();
     V.sdq = w->d_sdq.as<float4>();
     V.pred_d = w->d_pred_d.as<float4>();
     V.prev_qf = w->d_prev_qf.as<float4>();
     V.col_body = w->d_col_body.as<int32_t>();
-    V.single_hull = w->d_single_hull.as<uint8_t>();
+    V.single_hull = w->t_single_hull;
     V.work_list = w->d_work_list.as<int32_t>();
     V.work_state = w->d_work_state.as<int32_t>();
     V.gjk_list = w->d_gjk_list.as<int4>();
     V.hull_ref = w->d_hull_ref.as<HullRef>();
-    V.topo_rec = w->d_topo_rec.as<uint8_t>();
+    V.topo_rec = w->t_topo_rec;
     V.hit_list = w->d_hit_list.as<int4>();
     V.work_simplex = w->d_work_simplex.as<R>();
     V.work_epa = w->d_work_epa.as<double>();
@@ -850,7 +865,7 @@ WorldView<R> make_view(rp_world* w) {
     V.queue = w->d_queue.as<int32_t>();
     V.tstamp = w->d_tstamp.as<int32_t>();
     V.tlist = w->d_tlist.as<int32_t>();
-    V.scene_order = w->d_scene_order.as<int32_t>();
+    V.scene_order = w->t_scene_order;
     V.solo_nodes = w->solo_nodes;
     V.cta_scenes = w->cta_scenes;
     V.wait_ns = w->wait_ns;
@@ -1194,6 +1209,7 @@ void rp_world_destroy(rp_world* w) {
     if (w->ev0) cudaEventDestroy(w->ev0);
     if (w->ev1) cudaEventDestroy(w->ev1);
     if (w->ev_rec) cudaEventDestroy(w->ev_rec);
+    if (w->ev_hull) cudaEventDestroy(w->ev_hull);
     if (w->graph) cudaGraphExecDestroy(w->graph);
     for (cudaEvent_t ev : w->marks) cudaEventDestroy(ev);
     if (w->pipe.side) {
@@ -2412,6 +2428,7 @@ rp_status rp_transformed_hulls(rp_world* w, double* vertices_out, double* normal
     RP_CUDA(w->d_hull_v.ensure(vb));
     RP_CUDA(w->d_hull_n.ensure(nb));
     RP_CUDA(w->h_hull.ensure(vb + nb));
+    if (!w->ev_hull) RP_CUDA(cudaEventCreateWithFlags(&w->ev_hull, cudaEventDisableTiming));
     WorldHullsArgs a;
     a.colliders = w->d_colliders.as<Collider>();
     a.col_body = w->d_col_body.as<int32_t>();
@@ -2425,23 +2442,37 @@ rp_status rp_transformed_hulls(rp_world* w, double* vertices_out, double* normal
     a.normals_out = w->d_hull_n.as<double>();
     RP_CUDA(world_hulls(a, w->stream));
     w->launches++;
+    // Two copies to the host, each half handed to the caller on several threads while the other is on its way:
+    // most of the call is the pages of the caller's fresh arrays. Device order is slot order (bodies grouped by
+    // scene), the caller's is entity order.
     char* h = (char*)w->h_hull.p;
+    const size_t n = w->bodies.size();
+    std::vector<int64_t> at_v(n + 1, 0), at_n(n + 1, 0);
     RP_CUDA(cudaMemcpyAsync(h, a.vertices_out, (size_t)w->hull_nv * 24, cudaMemcpyDeviceToHost, w->stream));
+    RP_CUDA(cudaEventRecord(w->ev_hull, w->stream));
     RP_CUDA(cudaMemcpyAsync(h + vb, a.normals_out, (size_t)w->hull_nn * 24, cudaMemcpyDeviceToHost, w->stream));
-    RP_CUDA(cudaStreamSynchronize(w->stream));
-    w->d2h_bytes += (uint64_t)(w->hull_nv + w->hull_nn) * 24;
-    // device order is slot order (bodies grouped by scene); the output is in entity order
-    const double* hv = (const double*)h;
-    const double* hn = (const double*)(h + vb);
-    int64_t sv = 0, sn = 0;
-    for (size_t slot = 0; slot < w->bodies.size(); ++slot) {
+    for (size_t slot = 0; slot < n; ++slot) {
         const size_t e = (size_t)w->slot_to_entity[slot];
-        const int64_t nv = w->hull_v_off[e + 1] - w->hull_v_off[e], nn = w->hull_n_off[e + 1] - w->hull_n_off[e];
-        std::memcpy(vertices_out + 3 * w->hull_v_off[e], hv + 3 * sv, (size_t)nv * 24);
-        std::memcpy(normals_out + 3 * w->hull_n_off[e], hn + 3 * sn, (size_t)nn * 24);
-        sv += nv;
-        sn += nn;
+        at_v[slot + 1] = at_v[slot] + w->hull_v_off[e + 1] - w->hull_v_off[e];
+        at_n[slot + 1] = at_n[slot] + w->hull_n_off[e + 1] - w->hull_n_off[e];
     }
+    auto hand_over = [&](double* out, const double* in, const std::vector<int64_t>& at, const std::vector<int64_t>& off) {
+        in_chunks(n, (size_t)1 << 11, [&](size_t lo, size_t hi) {
+            for (size_t slot = lo; slot < hi;) {
+                // bodies that are neighbours in both orders go in one piece
+                const size_t e = (size_t)w->slot_to_entity[slot];
+                size_t k = 1;
+                while (slot + k < hi && (size_t)w->slot_to_entity[slot + k] == e + k) ++k;
+                std::memcpy(out + 3 * off[e], in + 3 * at[slot], (size_t)(at[slot + k] - at[slot]) * 24);
+                slot += k;
+            }
+        });
+    };
+    RP_CUDA(cudaEventSynchronize(w->ev_hull));
+    hand_over(vertices_out, (const double*)h, at_v, w->hull_v_off);
+    RP_CUDA(cudaStreamSynchronize(w->stream));
+    hand_over(normals_out, (const double*)(h + vb), at_n, w->hull_n_off);
+    w->d2h_bytes += (uint64_t)(w->hull_nv + w->hull_nn) * 24;
     return RP_OK;
 }
 

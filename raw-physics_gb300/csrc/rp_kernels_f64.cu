@@ -18,8 +18,8 @@ cudaError_t contacts_f64(const WorldView<double>& W, int a, int b, double* out, 
     return Launcher<double, true>::contacts(W, a, b, out, cap, count, st);
 }
 
-// One warp per hull collider; the exact build's transform (model matrix, point with its divide by w,
-// normalised direction), so the result is what colliders_update computes on the host.
+// One warp per hull collider; the exact build's transform, so the result is what colliders_update computes on
+// the host.
 __global__ void __launch_bounds__(256) world_hulls_kernel(WorldHullsArgs a) {
     const int lane = threadIdx.x & 31;
     const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -27,17 +27,14 @@ __global__ void __launch_bounds__(256) world_hulls_kernel(WorldHullsArgs a) {
         const Collider col = a.colliders[ci];
         if (col.type != COL_HULL) continue;
         const Shape sh = a.shapes[col.shape];
-        const double4_32a p4 = a.pos[a.col_body[ci]], q4 = a.rot[a.col_body[ci]];
-        const M4<double> M = model_matrix(qt<double>(q4.x, q4.y, q4.z, q4.w), v3<double>(p4.x, p4.y, p4.z));
+        const ExactPose M(a.pos[a.col_body[ci]], a.rot[a.col_body[ci]]);
         for (int i = lane; i < sh.nv; i += 32) {
-            const double* v = a.shape_verts + 3 * (size_t)(sh.vert_off + i);
-            const V3<double> o = m4_point(M, v3<double>(v[0], v[1], v[2]));
+            const V3<double> o = M.point(a.shape_verts + 3 * (size_t)(sh.vert_off + i));
             double* d = a.vertices_out + 3 * (size_t)(col.tv_off + i);
             d[0] = o.x; d[1] = o.y; d[2] = o.z;
         }
         for (int i = lane; i < sh.nf; i += 32) {
-            const double* n = a.face_normal + 3 * (size_t)(sh.face_off + i);
-            const V3<double> o = vnorm(m4_dir(M, v3<double>(n[0], n[1], n[2])));
+            const V3<double> o = M.normal(a.face_normal + 3 * (size_t)(sh.face_off + i));
             double* d = a.normals_out + 3 * (size_t)(col.tn_off + i);
             d[0] = o.x; d[1] = o.y; d[2] = o.z;
         }

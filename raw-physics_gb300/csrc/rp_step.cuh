@@ -883,6 +883,25 @@ __device__ void resched(const WorldView<R>& W, const G& g, int s) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// util_get_model_matrix_no_scale with collider_update's point and direction transforms (util.cpp:60-74,
+// collider.cpp:414-422) in FP64, without the products with the matrices' constant ones and zeros, which change
+// no bit: 69 FP64 instructions for the matrix and 18 a point instead of 150 and 41.
+struct ExactPose {
+    M3<double> m;
+    V3<double> o;
+    __device__ __forceinline__ ExactPose(double4_32a p, double4_32a q) : m(qmat3(qt<double>(q.x, q.y, q.z, q.w))) {
+        const double t[3] = {p.x, p.y, p.z};
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) m.d[i][j] = m.d[i][j] + t[i] * 0.0;
+        o = v3<double>(0.0 + t[0], 0.0 + t[1], 0.0 + t[2]);
+    }
+    __device__ __forceinline__ V3<double> point(const double* v) const { return vadd(mmulv(m, v3<double>(v[0], v[1], v[2])), o); }
+    __device__ __forceinline__ V3<double> normal(const double* n) const { return vnorm(mmulv(m, v3<double>(n[0], n[1], n[2]))); }
+};
+
+// ---------------------------------------------------------------------------------------------
 // Hull transform (colliders_update, collider.cpp:409-446): one collider of body b by `nsub` threads
 // (index `lane` among them)
 // POSE_F: take the FP32 build's orientation from the predict phase's FP32 copy (pose_f, the same
@@ -893,26 +912,9 @@ __device__ void transform_collider(const WorldView<R>& W, const Collider& col, i
     V3<R>* tv = (V3<R>*)(W.tverts) + col.tv_off;
     V3<R>* tn = (V3<R>*)(W.tnorms) + col.tn_off;
     if (EXACT) {
-        const double4_32a p4 = W.pos[b], q4 = W.rot[b];
-        // util_get_model_matrix_no_scale and the point transform (util.cpp:60-74, collider.cpp:414-422) without the
-        // products with the matrices' constant ones and zeros, which change no bit: 69 FP64 instructions for the
-        // matrix and 18 a vertex instead of 150 and 41
-        M3<double> M = qmat3(qt<double>(q4.x, q4.y, q4.z, q4.w));
-        const double t[3] = {p4.x, p4.y, p4.z};
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) M.d[i][j] = M.d[i][j] + t[i] * 0.0;
-        const V3<double> o = v3<double>(0.0 + t[0], 0.0 + t[1], 0.0 + t[2]);
-        for (int i = lane; i < sh.nv; i += nsub) {
-            const double* v = W.shape_verts + 3 * (sh.vert_off + i);
-            const V3<double> m = mmulv(M, v3<double>(v[0], v[1], v[2]));
-            tv[i] = v3cast<R>(vadd(m, o));
-        }
-        for (int i = lane; i < sh.nf; i += nsub) {
-            const double* nrm = W.face_normal + 3 * (sh.face_off + i);
-            tn[i] = v3cast<R>(vnorm(mmulv(M, v3<double>(nrm[0], nrm[1], nrm[2]))));
-        }
+        const ExactPose M(W.pos[b], W.rot[b]);
+        for (int i = lane; i < sh.nv; i += nsub) tv[i] = v3cast<R>(M.point(W.shape_verts + 3 * (sh.vert_off + i)));
+        for (int i = lane; i < sh.nf; i += nsub) tn[i] = v3cast<R>(M.normal(W.face_normal + 3 * (sh.face_off + i)));
     } else {
         Qt<R> q;
         if (POSE_F) {

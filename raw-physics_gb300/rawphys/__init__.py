@@ -355,9 +355,9 @@ class World:
         return b.value
 
     def broad_pairs(self, scene: int = 0) -> np.ndarray:
-        cap = 1 << 16
+        cap = max(1 << 16, 8 * self.num_entities())   # a call with too small a buffer is made again
         while True:
-            out = np.zeros(2 * cap, dtype=np.uint32)
+            out = np.empty(2 * cap, dtype=np.uint32)
             n = _u()
             rc = self.lib.rp_broad_pairs(self.h, scene, out.ctypes.data_as(_P(_u)), cap, C.byref(n))
             if rc == 0 and n.value <= cap:
@@ -443,7 +443,7 @@ class World:
         entity (rp_transformed_hulls: colliders_update computed on the device in FP64)."""
         nv, nn = _u64(), _u64()
         self._check(self.lib.rp_transformed_hulls_size(self.h, C.byref(nv), C.byref(nn)))
-        v, n = np.zeros((max(nv.value, 1), 3)), np.zeros((max(nn.value, 1), 3))
+        v, n = np.empty((max(nv.value, 1), 3)), np.empty((max(nn.value, 1), 3))
         self._check(self.lib.rp_transformed_hulls(self.h, _dp(v), _dp(n)))
         return v[: nv.value], n[: nn.value]
 
