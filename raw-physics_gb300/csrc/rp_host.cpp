@@ -592,7 +592,7 @@ rp_status build_device(rp_world* w) {
     RP_CUDA(w->d_tl.ensure(std::max<size_t>(NN, 1) * 8));
     RP_CUDA(w->d_level_count.ensure((size_t)S * (size_t)(w->max_levels + 1) * 4));
     RP_CUDA(w->d_level_fill.ensure((size_t)S * (size_t)(w->max_levels + 1) * 4));
-    RP_CUDA(w->d_scan_tmp.ensure(4096 * 4));
+    RP_CUDA(w->d_scan_tmp.ensure(SCAN_TMP_WORDS * 4));
     RP_CUDA(w->d_level_nodes.ensure(std::max<size_t>(NN, 1) * 4));
     RP_CUDA(w->d_scene_levels.ensure((size_t)S * 4));
     RP_CUDA(w->d_node_vpred.ensure(std::max<size_t>(NN, 1) * 8));

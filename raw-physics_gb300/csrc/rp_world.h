@@ -101,6 +101,8 @@ struct __align__(16) HullRef {
     int32_t vstride, fstride;    // lines per record
 };
 
+// scratch words of a grid group: one per block, and two counters at the end
+constexpr int SCAN_TMP_WORDS = 4096;
 // default of WorldView::solo_nodes (rp_step.cuh, sweep_levels)
 constexpr int SOLO_NODES = 32, SOLO_NODES_FP64 = 16;
 // FP32 build: the single large scene's levels of at most this many nodes round both bodies of a contact alike
