@@ -948,14 +948,18 @@ struct PipeLauncher {
     static size_t solve_bytes(int bodies, int joints) { return solve_smem<R>(solve_room(bodies, joints)); }
 
     // The solver half of a substep, scene by scene (k_solve): the larger scenes with 256 threads each, the
-    // others with 128 and less shared memory, side by side on two branches.
+    // others with 128 and less shared memory, side by side on two branches. Registers hold four CTAs of 128
+    // threads on an SM; more scenes than that take 64 threads, so that they still run at once: a small scene is
+    // bound by its chain of levels, and a nearly empty second wave doubles it (768 chains of 33 links: 3.3 -> 2.7 ms
+    // a frame; 4096 heaps: the same within 0.5 %).
     static cudaError_t solve(const WorldView<R>& W, const StepParams& P, const PipeConfig& c, const PipeDims& d, cudaStream_t st,
                              double h, int predict) {
         cudaError_t e = cudaSuccess;
         const int alike = d.grid_mode;
         auto launch = [&](int k, cudaStream_t s, int reset) -> cudaError_t {
             const SolveRoom room = solve_room(d.solve_bodies[k], d.solve_joints[k]);
-            k_solve<R, EXACT><<<d.solve_count[k], k == 0 ? SOLVE_BLOCK : SOLVE_BLOCK / 2, solve_smem<R>(room), s>>>(
+            const int threads = k == 0 ? SOLVE_BLOCK : (d.solve_count[1] > 4 * c.sms ? SOLVE_BLOCK / 4 : SOLVE_BLOCK / 2);
+            k_solve<R, EXACT><<<d.solve_count[k], threads, solve_smem<R>(room), s>>>(
                 W, d.solve_scenes + (k ? d.solve_count[0] : 0), room, h, 1.0 / h, P.num_pos_iters, alike, predict, reset);
             return cudaGetLastError();
         };
