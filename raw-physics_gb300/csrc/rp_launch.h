@@ -14,7 +14,7 @@ inline int transform_group_for(bool fp64, int colliders, int sms) { return fp64 
 struct PipeConfig {
     int sms = 0;
     int cull_blocks = 0, gjk_blocks = 0, epa_blocks = 0, manifold_blocks = 0, general_blocks = 0;
-    int setup_grid_blocks = 0, sweep_grid_blocks = 0, vsweep_grid_blocks = 0, sweep_warp_blocks = 0;
+    int setup_grid_blocks = 0, sweep_grid_blocks = 0, sweep_warp_blocks = 0;
     // tunable (rp_autotune): the schedule does not depend on them (FP64 results identical, FP32 to rounding)
     int transform_group = 0;     // threads per collider in the hull transform; 0: transform_group_for
     int sweep_cta = 0;           // batched sweeps: one CTA per scene instead of one warp per scene
