@@ -54,10 +54,10 @@ sys.path.insert(0, ROOT)
 
 METRIC = "body-substeps/s batched vs plain GPU at ≤1e-4 m pos err vs FP64 CPU; grad/s"
 UNIT = "body-substeps/s"
-# Algorithmic bytes of one position sweep: every contact record read (48 B) and its two lambdas
-# written back (8 B); per solved pair node, both bodies' pose read and written (2 x 64 B) and their
-# inverse mass and inertia read (2 x 28 B).
-SWEEP_CONTACT_B, SWEEP_NODE_B = 56, 2 * (64 + 64 + 28)
+# Algorithmic bytes of a substep's solver half (schedules, sweeps, velocity update and predict in one kernel):
+# every contact record read by both sweeps (2 x 48 B) and its two lambdas written back (8 B); per solved pair
+# node, both bodies' pose read and written (2 x 64 B) and their inverse mass and inertia read (2 x 28 B).
+SWEEP_CONTACT_B, SWEEP_NODE_B = 104, 2 * (64 + 64 + 28)
 # Algorithmic FP32 flops of the narrowphase (per device-counted operation): a support call is one dot
 # product and a compare per hull vertex (6 V); a GJK iteration's simplex update ~60; an EPA iteration
 # ~40 per new face plus 6 per face scanned.
@@ -421,13 +421,12 @@ def fp32_pipe(c0, c1, frames, phase, verts_avg):
     return out
 
 
-def roofline_of(phase, c0, c1, frames, substeps, pos_iters, kernels, summary):
-    """Roofline object of the dominant kernel. The position sweep (one launch per substep and
-    iteration) has the HBM byte model above; other phases are reported with their share only."""
+def roofline_of(phase, c0, c1, frames, substeps, kernels, summary):
+    """Roofline object of the dominant kernel. The solver half (one launch per substep) has the HBM byte
+    model above; other phases are reported with their share only."""
     peak, peak_kind = measured_peak_hbm()
-    sweeps = substeps * pos_iters
     alg_bytes = ((c1[5] - c0[5]) / frames * SWEEP_CONTACT_B + (c1[2] - c0[2]) / frames * SWEEP_NODE_B) / substeps
-    launch_ms = phase["solve"] / sweeps if sweeps else 0.0
+    launch_ms = phase["solve"] / substeps if substeps else 0.0
     achieved = alg_bytes / (launch_ms / 1e3) / 1e9 if launch_ms > 0 else 0.0
     traffic, src = profile_traffic(summary, kernels["solve"])
     frame_ms = sum(phase.values())
@@ -491,8 +490,8 @@ def measure_batched(args, dev, rank, world_size, with_oracle):
     verts_avg = float(np.mean(verts[batch.mesh]))
     out = {"value": value, "total_ms": total_ms, "ms": ms, "clocks": clocks, "launches": launches, "status": status,
            "degenerate_first": degenerate, "phase": phase, "e2e": e2e, "tuned": tuned, "nd": nd,
-           "roofline": roofline_of(phase, c0, c1, args.steps, batch.substeps, batch.pos_iters,
-                                   {"solve": "k_sweep_warp (position sweep, one warp per scene)"}, "pipeline_batched16384.md"),
+           "roofline": roofline_of(phase, c0, c1, args.steps, batch.substeps,
+                                   {"solve": "k_solve (solver half of a substep, a block per scene)"}, "pipeline_batched16384.md"),
            "fp32_pipe": fp32_pipe(c0, c1, args.steps, phase, verts_avg),
            "pairs_per_step": (c1[6] - c0[6]) / args.steps, "contacts_per_step": (c1[5] - c0[5]) / args.steps}
     if with_oracle:
@@ -572,8 +571,8 @@ def measure_plain(args, dev, precision, steps, start_from=None, with_oracle=Fals
            "autotuned": tuned, "start_state": start_state,
            "e2e": {"value": scene.num_dynamic * scene.substeps * max(3, steps // 2) / e2e_wall, "unit": UNIT,
                    "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-           "roofline": roofline_of(phase, c0, c1, steps, scene.substeps, scene.pos_iters,
-                                   {"solve": "k_sweep_grid (position sweep, cooperative grid)"}, "pipeline_large4096.md"),
+           "roofline": roofline_of(phase, c0, c1, steps, scene.substeps,
+                                   {"solve": "k_solve_grid (solver half of a substep, cooperative grid)"}, "pipeline_large4096.md"),
            "pairs_per_step": (c1[6] - c0[6]) / steps, "contacts_per_step": (c1[5] - c0[5]) / steps,
            "levels_per_step": (c1[7] - c0[7]) / steps}
     if with_oracle:

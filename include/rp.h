@@ -107,7 +107,7 @@ rp_status rp_world_set_stream(rp_world* w, void* cuda_stream);
  * clipping's float roundings are differentiated as identity. Static friction only enters through a
  * comparison, so its gradient is zero. Scenes whose contact pairs involve sphere colliders report
  * RP_ERR_INVALID with collisions on. The forward pass is the all-FP64 step: its loss equals the FP64
- * build's. Reverse mode over a tape, one scene per GPU thread, with the trajectory checkpointed
+ * build's. Reverse mode over a tape per substep, many substeps taped at once, with the trajectory checkpointed
  * every `checkpoint_every` frames and recomputed segment by segment. Starts from the world's current
  * state, which it does not change. target: 3 doubles per scene. */
 rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t num_substeps, uint32_t num_pos_iters,
@@ -125,8 +125,10 @@ rp_status rp_world_set_mode(rp_world* w, int32_t mode);
  * then also picks the colouring's priority scheme. No counterpart in the reference. */
 enum { RP_SWEEP_REFERENCE = 0, RP_SWEEP_COLOURED = 1 };
 rp_status rp_world_set_sweep_order(rp_world* w, int32_t order);
-/* How a batch's sweeps spread scenes over the GPU (a launch shape: the same schedule under every
- * choice, so FP64 results are identical and FP32 results agree to rounding):
+/* How the sweeps of a batch spread scenes over the GPU where scenes are swept by kernels of their own: in
+ * worlds with a scene of more than 640 bodies, and in the coloured order (other worlds solve a scene per CTA,
+ * whatever is set here). A launch shape: the same schedule under every choice, so FP64 results are identical
+ * and FP32 results agree to rounding:
  * 0 one warp per scene (the default), 1 one CTA per scene, n >= 2 a whole CTA for every scene whose
  * sweep cost (dynamic bodies + 8 per joint) is n or more and one warp for each other scene.
  * rp_autotune chooses among these (its choice[2]). No counterpart in the reference. */
@@ -140,8 +142,8 @@ rp_status rp_world_set_sweep_assignment(rp_world* w, int32_t cta);
 rp_status rp_world_set_wait_limit(rp_world* w, uint64_t microseconds);
 /* Autotuner (no counterpart in the reference): times `frames` frames of the world's current scenes
  * from their current state under each candidate launch configuration — launch mode, threads per
- * collider in the hull transform (4/8/16/32), and the sweep layout (levels swept by one CTA below
- * 128..2048 nodes for one large scene; for a batch, which scenes a warp and which a whole CTA sweeps) —
+ * collider in the hull transform (4/8/16/32), and the sweep layout (levels swept by one CTA up to
+ * 16..512 nodes for one large scene; for a batch, which scenes a warp and which a whole CTA sweeps) —
  * keeps the fastest, and restores the state. Every configuration runs the same schedule: results are
  * identical in RP_PRECISION_FP64 and agree to rounding in RP_PRECISION_FP32 (each kernel instantiation
  * may contract multiply-adds differently). Each candidate is timed twice; one replaces the default only

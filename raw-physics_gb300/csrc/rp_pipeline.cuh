@@ -6,10 +6,12 @@
 // small kernel, launched over the whole batch, and a frame is the fixed sequence
 //
 //   setup (per scene: broad phase, islands, schedule, work-list reservation)
-//   per substep: predict, hull transform, GJK, EPA, contact manifold, position sweep(s),
-//                velocity update, velocity sweep
+//   predict; per substep: cull, hull transform, GJK, EPA, contact manifold, solver half
 //
-// replayed from a CUDA graph. Every SM then runs one phase's code at a time, the narrowphase
+// The solver half (schedules, position sweeps, velocity update, velocity sweep, next predict) is one kernel:
+// k_solve (rp_scene.cuh, a CTA per scene) where every scene fits a CTA, k_solve_grid for one large scene;
+// worlds with a larger scene among others, and coloured sweeps of a batch, run it as a kernel per phase. The
+// sequence is replayed from a CUDA graph. Every SM then runs one phase's code at a time, the narrowphase
 // kernels run at the occupancy their register and shared-memory needs allow, and the work is
 // spread over all SMs regardless of how it is split into scenes. Results are identical to the
 // persistent kernels: the same device functions run in the same order per scene.
@@ -21,6 +23,7 @@
 //   k_gjk       warp per GJK candidate: GJK on the two staged hulls; a hit stores its simplex and
 //               joins hit_list
 //   k_epa       warp per hit: EPA from the stored simplex; stores the FP64 normal and the penetration
+//               (or the final face, for k_epa_finish, a thread per hit)
 //   k_manifold  warp per hit_list entry: contact manifold (or the general path); writes contacts
 #pragma once
 #include "rp_step.cuh"

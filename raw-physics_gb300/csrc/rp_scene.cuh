@@ -16,7 +16,7 @@
 //
 // Measured (GB300; sweeps, velocity update and predict of one substep, before as four kernels -> after): one
 // scene of 150 bodies 133 -> 60 us; 96 scenes of up to 512 bodies, a quarter with chains, 754 -> 340 us;
-// 768 chains of 33 links 250 -> 150 us.
+// 768 chains of 33 links 250 -> 94 us.
 #pragma once
 #include "rp_step.cuh"
 #include "rp_launch.h"
