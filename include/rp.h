@@ -345,7 +345,8 @@ uint64_t  rp_kernel_launches(const rp_world* w);
  * [1] islands and sleeping, [2] solver schedule, [3] predict, [4] hull transform, [5] narrowphase
  * (persistent kernel: all of it; phase-major form: the cull kernel), [6] position solve, [7] velocity
  * update, [8] velocity solve, [9] GJK, [10] EPA, [11] contact manifold (the phase-major form's
- * narrowphase kernels). The phase-major form is timed with CUDA events after each kernel while
+ * narrowphase kernels). Where one kernel runs several of these its time is in the last for the
+ * narrowphase ([11]) and in the first for the solver half ([6], with the next substep's predict). The phase-major form is timed with CUDA events after each kernel while
  * timing is on (rp_set_timing; those frames run outside the CUDA graph); the persistent kernel with
  * the global timer as seen by each scene's first thread. */
 #define RP_NUM_PHASES 12

@@ -638,6 +638,7 @@ rp_status build_device(rp_world* w) {
             refs[slot].tn_off = c.tn_off;
         }
         w->dims.pair_cap = (int)P;
+        w->dims.one_pass = contact_in_one_pass((int)P, w->num_sms) ? 1 : 0;
         w->dims.general = std::any_of(single.begin(), single.begin() + (ptrdiff_t)N, [](uint8_t x) { return !x; }) ? 1 : 0;
         rec.resize(rec.size() + 512, 0);   // lanes past a record's end read on
         RP_CUDA(w->d_pose_f.ensure(std::max<size_t>(N, 1) * 32));

@@ -222,8 +222,9 @@ __device__ void hull_manifold(NarrowSmem<R>& sm, const WorldView<R>& W, const Re
         } else {
             double d = 0.0;
             if (lane < 2) {
-                const V3<double> m = face_normal64(W, lane ? hb.face_off + f2 : ha.face_off + f1, lane ? body_b : body_a);
-                d = vdot(m, lane ? vinv(normal64) : normal64);
+                const double4_32a q = W.rot[lane ? body_b : body_a];
+                const V3<double> n = lane ? vinv(normal64) : normal64;
+                d = turned_dot(W.face_normal + 3 * (lane ? hb.face_off + f2 : ha.face_off + f1), q.x, q.y, q.z, q.w, n.x, n.y, n.z);
             }
             ref1 = __shfl_sync(0xffffffffu, d, 0) > __shfl_sync(0xffffffffu, d, 1);
         }

@@ -11,9 +11,13 @@ namespace rp {
 // and always in FP64, whose time is the instructions of a warp; else four.
 inline int transform_group_for(bool fp64, int colliders, int sms) { return fp64 || colliders <= 16 * sms ? 32 : 4; }
 
+// Whether GJK, EPA and manifold are one kernel (k_contact): there are 16 pair slots a body and about half a hit,
+// so 48 slots a resident warp (16 on an SM) are up to one and a half hits a warp, where both forms take as long.
+inline bool contact_in_one_pass(int pair_cap, int sms) { return pair_cap <= 48 * 16 * sms; }
+
 struct PipeConfig {
     int sms = 0;
-    int cull_blocks = 0, gjk_blocks = 0, epa_blocks = 0, manifold_blocks = 0, general_blocks = 0;
+    int cull_blocks = 0, contact_blocks = 0, gjk_blocks = 0, epa_blocks = 0, manifold_blocks = 0, general_blocks = 0;
     int setup_grid_blocks = 0, sweep_grid_blocks = 0, sweep_warp_blocks = 0;
     // tunable (rp_autotune): the schedule does not depend on them (FP64 results identical, FP32 to rounding)
     int transform_group = 0;     // threads per collider in the hull transform; 0: transform_group_for
@@ -25,6 +29,7 @@ struct PipeConfig {
 struct PipeDims {
     int nbodies = 0, ncolliders = 0, next = 0, num_scenes = 0;
     int pair_cap = 0;    // pair slots of the world
+    int one_pass = 0;    // contact_in_one_pass
     int general = 0;     // some body is not a single hull of at most 64 vertices
     int node_words = 0;  // words of the node bitmap (node capacity / 32 + 1)
     int grid_mode = 0;   // one large scene: cooperative setup and sweeps

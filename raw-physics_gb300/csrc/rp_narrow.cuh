@@ -161,6 +161,13 @@ struct ColView {
     int body;                // the body's slot (its FP64 orientation is read only for decisions made in FP64)
 };
 
+// One function for every kernel that decides by it: between faces that rest on each other the comparison is
+// one of roundings.
+static __device__ __noinline__ double turned_dot(const double* n, double qx, double qy, double qz, double qw, double dx, double dy, double dz) {
+    const V3<double> m = vnorm_fast(mmulv(qmat3(qt<double>(qx, qy, qz, qw)), v3<double>(n[0], n[1], n[2])));
+    return vdot(m, v3<double>(dx, dy, dz));
+}
+
 // A face normal of a hull rotated by the body's FP64 orientation (collider_update's normal
 // transform, collider.cpp:425-429), for the FP32 build's FP64 reference-face decision.
 template <typename R>
@@ -636,6 +643,17 @@ __device__ __forceinline__ void epa_face_f32(const V3<float>* poly, int npoly, u
     d_out = d;
 }
 
+// The FP64 normal and depth of EPA's final face from its three points and FP32 normal (epa.cpp:32-77
+// on the face EPA stopped at): one function for every kernel that needs them.
+__device__ __forceinline__ void epa_face_finish(const float* f, V3<double>& n64, double& d64) {
+    const V3<double> a = v3<double>(f[0], f[1], f[2]), b = v3<double>(f[3], f[4], f[5]), c = v3<double>(f[6], f[7], f[8]);
+    n64 = vnorm_fast(vcross(vsub(b, a), vsub(c, a)));
+    if (vdot(n64, v3<double>(f[9], f[10], f[11])) < 0.0) n64 = vinv(n64);
+    d64 = vdot(n64, a);
+}
+// The same as a function of its own, for kernels whose other FP64 arithmetic it must not be contracted with.
+static __device__ __noinline__ void epa_face_finish_call(const float* f, V3<double>& n64, double& d64) { epa_face_finish(f, n64, d64); }
+
 // face_out (optional): when FP32 decides the termination, lane 0 writes the final face's three
 // points and its FP32 normal there (12 floats) and *deferred is set, leaving the FP64 normal and depth
 // to a thread-per-pair kernel (k_epa_finish) instead of the warp; otherwise they are computed here.
@@ -643,7 +661,8 @@ __device__ __forceinline__ void epa_face_f32(const V3<float>* poly, int npoly, u
 // their position, so that coincident edges are equal keys and the horizon is one match across the lanes
 // instead of a scan per lane, and the bounds of the FP32 termination test use approximate roots: 14.7 k ->
 // 11.4 k SM cycles a call in a batch of 4096 heaps (2 iterations a call), 11.7 k -> 10.3 k in one of 96.
-template <typename R, class Mink>
+// CALL: the FP64 face by epa_face_finish_call.
+template <typename R, bool CALL = false, class Mink>
 __device__ bool epa_fast(NarrowSmem<R>& smr, const Mink& mink, const Simplex<R>& s,
                          V3<double>& out_n, double& out_pen, int& iters, long long* support_cycles = nullptr,
                          float* face_out = nullptr, bool* deferred = nullptr) {
@@ -717,11 +736,11 @@ __device__ bool epa_fast(NarrowSmem<R>& smr, const Mink& mink, const Simplex<R>&
         V3<double> n64 = v3<double>(0, 0, 0);
         double d64 = 0.0;
         if (mi != 0x7fffffff && (need64 || done)) {
-            uchar4 f = sm.f[mi];
-            V3<double> a = v3cast<double>(sm.poly[f.x]), b = v3cast<double>(sm.poly[f.y]), c = v3cast<double>(sm.poly[f.z]);
-            n64 = vnorm_fast(vcross(vsub(b, a), vsub(c, a)));
-            if (vdot(n64, v3cast<double>(min_n)) < 0.0) n64 = vinv(n64);
-            d64 = vdot(n64, a);
+            const uchar4 f = sm.f[mi];
+            const V3<float> pa = sm.poly[f.x], pb = sm.poly[f.y], pc = sm.poly[f.z];
+            const float v[12] = {pa.x, pa.y, pa.z, pb.x, pb.y, pb.z, pc.x, pc.y, pc.z, min_n.x, min_n.y, min_n.z};
+            if (CALL) epa_face_finish_call(v, n64, d64);
+            else epa_face_finish(v, n64, d64);
         }
         if (need64) done = fabs(vdot(n64, v3cast<double>(sp)) - d64) < 0.0001;
         if (done) {
@@ -851,21 +870,18 @@ __device__ bool epa_fast(NarrowSmem<R>& smr, const Mink& mink, const Simplex<R>&
     return false;
 }
 
-// The FP64 normal and depth of EPA's final face from its three points and FP32 normal (epa.cpp:32-77
-// on the face EPA stopped at), as epa_fast computes them in the warp: one thread per pair.
-__device__ __forceinline__ void epa_face_finish(const float* f, V3<double>& n64, double& d64) {
-    const V3<double> a = v3<double>(f[0], f[1], f[2]), b = v3<double>(f[3], f[4], f[5]), c = v3<double>(f[6], f[7], f[8]);
-    n64 = vnorm_fast(vcross(vsub(b, a), vsub(c, a)));
-    if (vdot(n64, v3<double>(f[9], f[10], f[11])) < 0.0) n64 = vinv(n64);
-    d64 = vdot(n64, a);
-}
-
 // ---------------------------------------------------------------------------------------------
 // Clipping (clipping.cpp)
 template <typename R>
 __device__ __forceinline__ bool in_plane(V3<R> pn, V3<R> pp, V3<R> pos) {
     float distance = -vdot(pn, pp);
     return !(vdot(pos, pn) + (R)distance < (R)0.0);
+}
+
+template <typename R>
+__device__ __forceinline__ V3<R> clip_axpy(R s, V3<R> v, V3<R> c) {   // c + s v
+    if constexpr (std::is_same<R, float>::value) return axpy_f(s, v, c);
+    else return vadd(c, vscale(s, v));
 }
 
 template <typename R>
@@ -876,11 +892,11 @@ __device__ __forceinline__ bool plane_edge(V3<R> pn, V3<R> pp, V3<R> start, V3<R
     // lies between them, so the FP32 comparison decides exactly the same
     if (fabsf(ab_p) > 1e-6f) {
         float distance = -vdot(pn, pp);
-        V3<R> p_co = vscale((R)(-distance), pn);
-        float fac = -vdot(pn, vsub(start, p_co)) / (R)ab_p;
+        // start - (-distance) pn
+        float fac = -vdot(pn, clip_axpy((R)distance, pn, start)) / (R)ab_p;
         R mx = ((R)fac > (R)0.0) ? (R)fac : (R)0.0;
         fac = (float)((mx < (R)1.0) ? mx : (R)1.0);
-        out = vadd(start, vscale((R)fac, ab));
+        out = clip_axpy((R)fac, ab, start);
         return true;
     }
     return false;

@@ -25,6 +25,7 @@
 //   k_epa       warp per hit: EPA from the stored simplex; stores the FP64 normal and the penetration
 //               (or the final face, for k_epa_finish, a thread per hit)
 //   k_manifold  warp per hit_list entry: contact manifold (or the general path); writes contacts
+//   k_contact   the last three in one, warp per GJK candidate, for worlds with a warp for nearly every hit
 #pragma once
 #include "rp_step.cuh"
 #include "rp_scene.cuh"
@@ -388,6 +389,47 @@ __global__ void __launch_bounds__(PIPE_BLOCK, 3) k_gjk(WorldView<R> W) {
     t.flush(W.counters, slots);
 }
 
+// EPA of one hit by a warp: the state the pair goes on with. WS_EPA_FACE: normal and depth are left to
+// epa_face_finish (work_face holds the face); t: EPA iterations, calls, cycles, cap hits, -, support cycles.
+template <typename R, bool EXACT, bool CALL>
+__device__ __forceinline__ int epa_pair(const WorldView<R>& W, NarrowSmem<R>& sm, int4 item, const RegHull<R>& ra, const RegHull<R>& rb,
+                                        const Simplex<R>& sx, V3<double>& nrm, double& pen, WarpTally& t) {
+    const int lane = threadIdx.x & 31, k = item.x, gp = item.y, a = item.z, b = item.w;
+    if (lane == 0) { sm.status = 0; }
+    pen = 0.0;
+    int ei = 0;
+    const long long t0 = clock64();
+    long long tsup = 0;
+    bool deferred = false;
+    bool ok;
+    if constexpr (EXACT || !kEpaFast) ok = epa(sm, RegMink<R>{ra, rb}, sx, nrm, pen, ei);
+    else ok = epa_fast<R, CALL>(sm, RegMink<R>{ra, rb}, sx, nrm, pen, ei, &tsup, W.work_face + 12 * (size_t)k, &deferred);
+    t.v[0] += ei;
+    t.v[1] += 1;
+    t.v[2] += clock64() - t0;
+    t.v[3] += ei >= 100;
+    t.v[5] += tsup;
+    const int s = W.body_scene[a];
+    if (!EXACT && (sm.status & (ST_DEG_EPA_NORMAL | ST_DEG_EPA_COPLANAR))) {
+        // FP32 resolved this polytope to a degenerate one: the pair is redone in FP64 (k_fallback),
+        // which decides it as the reference would
+        if (lane == 0) W.fallback_list[atomicAdd(&W.queue[5], 1)] = k;
+        return WS_FALLBACK;
+    }
+    if (lane == 0) {
+        if (!ok) {
+            atomicOr(&W.status[s], (uint32_t)ST_EPA_NOT_CONVERGED);
+            W.pair_ccount[gp] = 0;
+            W.pair_cstart[gp] = 0;
+        }
+        if (sm.status) {
+            atomicOr(&W.status[s], (uint32_t)sm.status);
+            note_degenerate(W, (uint32_t)sm.status, s, a, b);
+        }
+    }
+    return ok ? (deferred ? WS_EPA_FACE : WS_EPA_OK) : WS_NONE;
+}
+
 template <typename R, bool EXACT>
 __global__ void __launch_bounds__(PIPE_BLOCK, EXACT ? 2 : 3) k_epa(WorldView<R> W) {
     if (frame_abandoned(W.status)) return;
@@ -396,74 +438,37 @@ __global__ void __launch_bounds__(PIPE_BLOCK, EXACT ? 2 : 3) k_epa(WorldView<R> 
     const int lane = threadIdx.x & 31;
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     const int n = W.queue[3];
-    WarpTally t;   // EPA iterations, EPA calls, EPA cycles, EPA cap hits
+    WarpTally t;
     for (int j = gw; j < n; j += nw) {
         const int4 item = W.hit_list[j];
         const int k = item.x;
         if (W.work_state[k] != WS_HIT) continue;
-        {
-            const int gp = item.y, a = item.z, b = item.w;
-            if (lane == 0) { sm.status = 0; }
-            const long long tv = clock64();
-            const RegHull<R> ra = load_reghull(W, W.hull_ref[a], v3<R>(0, 0, 0));
-            const RegHull<R> rb = load_reghull(W, W.hull_ref[b], pair_offset<R, EXACT>(W, k));
-            const R* in = W.work_simplex + 16 * (size_t)k;
-            Simplex<R> sx;
-            sx.a = v3<R>(in[0], in[1], in[2]);
-            sx.b = v3<R>(in[3], in[4], in[5]);
-            sx.c = v3<R>(in[6], in[7], in[8]);
-            sx.d = v3<R>(in[9], in[10], in[11]);
-            sx.num = 4;
-            V3<double> nrm;
-            double pen = 0.0;
-            int ei = 0;
-            const long long t0 = clock64();
-            long long tsup = 0;
-            bool deferred = false;
-            bool ok;
-            if constexpr (EXACT || !kEpaFast) ok = epa(sm, RegMink<R>{ra, rb}, sx, nrm, pen, ei);
-            else ok = epa_fast(sm, RegMink<R>{ra, rb}, sx, nrm, pen, ei, &tsup, W.work_face + 12 * (size_t)k, &deferred);
-            t.v[0] += ei;
-            t.v[1] += 1;
-            t.v[2] += clock64() - t0;
-            t.v[3] += ei >= 100;
-            t.v[4] += t0 - tv;
-            t.v[5] += tsup;
-            const int s = W.body_scene[a];
-            if (!EXACT && (sm.status & (ST_DEG_EPA_NORMAL | ST_DEG_EPA_COPLANAR))) {
-                // FP32 resolved this polytope to a degenerate one: the pair is redone in FP64 (k_fallback),
-                // which decides it as the reference would
-                if (lane == 0) {
-                    W.work_state[k] = WS_FALLBACK;
-                    W.fallback_list[atomicAdd(&W.queue[5], 1)] = k;
-                }
-                __syncwarp();
-                continue;
-            }
-            if (lane == 0) {
-                if (!ok) atomicOr(&W.status[s], (uint32_t)ST_EPA_NOT_CONVERGED);
-                if (sm.status) {
-                    atomicOr(&W.status[s], (uint32_t)sm.status);
-                    note_degenerate(W, (uint32_t)sm.status, s, a, b);
-                }
-                if (ok && deferred) {
-                    W.work_state[k] = WS_EPA_FACE;
-                } else if (ok) {
-                    double* o = W.work_epa + 4 * (size_t)k;
-                    o[0] = nrm.x; o[1] = nrm.y; o[2] = nrm.z; o[3] = pen;
-                    if (!EXACT) {
-                        float* fo = W.work_face + 12 * (size_t)k;
-                        fo[0] = (float)nrm.x; fo[1] = (float)nrm.y; fo[2] = (float)nrm.z; fo[3] = (float)pen;
-                    }
-                    W.work_state[k] = WS_EPA_OK;
-                } else {
-                    W.work_state[k] = WS_NONE;
-                    W.pair_ccount[gp] = 0;
-                    W.pair_cstart[gp] = 0;
+        const long long tv = clock64();
+        const RegHull<R> ra = load_reghull(W, W.hull_ref[item.z], v3<R>(0, 0, 0));
+        const RegHull<R> rb = load_reghull(W, W.hull_ref[item.w], pair_offset<R, EXACT>(W, k));
+        const R* in = W.work_simplex + 16 * (size_t)k;
+        Simplex<R> sx;
+        sx.a = v3<R>(in[0], in[1], in[2]);
+        sx.b = v3<R>(in[3], in[4], in[5]);
+        sx.c = v3<R>(in[6], in[7], in[8]);
+        sx.d = v3<R>(in[9], in[10], in[11]);
+        sx.num = 4;
+        t.v[4] += clock64() - tv;
+        V3<double> nrm;
+        double pen;
+        const int state = epa_pair<R, EXACT, false>(W, sm, item, ra, rb, sx, nrm, pen, t);
+        if (lane == 0) {
+            if (state == WS_EPA_OK) {
+                double* o = W.work_epa + 4 * (size_t)k;
+                o[0] = nrm.x; o[1] = nrm.y; o[2] = nrm.z; o[3] = pen;
+                if (!EXACT) {
+                    float* fo = W.work_face + 12 * (size_t)k;
+                    fo[0] = (float)nrm.x; fo[1] = (float)nrm.y; fo[2] = (float)nrm.z; fo[3] = (float)pen;
                 }
             }
-            __syncwarp();
+            W.work_state[k] = state;
         }
+        __syncwarp();
     }
     const int slots[8] = {1, 2, 13, 7, 17, 18, -1, -1};
     t.flush(W.counters, slots);
@@ -490,6 +495,27 @@ __global__ void __launch_bounds__(PIPE_BLOCK) k_epa_finish(WorldView<R> W) {
     }
 }
 
+// The contact manifold of one pair of single hulls by a warp, from the EPA normal n64 (FP32 build: and its FP32
+// copy nf). False when FP32 finds the edges of an edge contact parallel: the pair is redone in FP64.
+template <typename R, bool EXACT>
+__device__ __forceinline__ bool manifold_pair(const WorldView<R>& W, NarrowSmem<R>& sm, int4 item, const RegHull<R>& ra,
+                                              const RegHull<R>& rb, const HullRef& ha, const HullRef& hb, V3<R> offb, V3<double> n64,
+                                              V3<R> nf) {
+    const int lane = threadIdx.x & 31, k = item.x, a = item.z, b = item.w;
+    if (lane == 0) { sm.ncontacts = 0; sm.status = 0; }
+    __syncwarp();
+    const PairFrame<R, EXACT> fr = pair_frame<R, EXACT>(W, a, b, offb);
+    sm.va[lane] = ra.v0; sm.va[lane + 32] = ra.v1;
+    sm.vb[lane] = rb.v0; sm.vb[lane + 32] = rb.v1;
+    __syncwarp();
+    hull_manifold<R, EXACT>(sm, W, ra, rb, ha, hb, a, b, nf, n64, fr);
+    if (!EXACT && (sm.status & ST_DEG_SKEW)) {
+        if (lane == 0) W.fallback_list[atomicAdd(&W.queue[5], 1)] = k;
+        return false;
+    }
+    return true;
+}
+
 // GENERAL: the pairs of the general path (compound bodies, sphere colliders: the whole
 // colliders_get_contacts per pair); otherwise the contact manifolds of the EPA hits. Two instantiations
 // keep the common kernel's code and registers free of the general path.
@@ -507,51 +533,120 @@ __global__ void __launch_bounds__(PIPE_BLOCK, (GENERAL || EXACT) ? 2 : 3) k_mani
         const int k = item.x;
         const int st = W.work_state[k];
         if (st != (GENERAL ? WS_GENERAL : WS_EPA_OK)) continue;
-        {
-            const int gp = item.y, a = item.z, b = item.w;
-            const int s = W.body_scene[a];
-            const long long t0 = clock64();
-            long long t1 = t0;
-            if constexpr (GENERAL) {
-                pair_contacts<R, EXACT>(W, sm, a, b, false);
-            } else {
-                if (lane == 0) { sm.ncontacts = 0; sm.status = 0; }
-                __syncwarp();
-                const V3<R> offb = pair_offset<R, EXACT>(W, k);
-                const HullRef ha = W.hull_ref[a], hb = W.hull_ref[b];
-                const RegHull<R> ra = load_reghull(W, ha, v3<R>(0, 0, 0)), rb = load_reghull(W, hb, offb);
-                const PairFrame<R, EXACT> fr = pair_frame<R, EXACT>(W, a, b, offb);
-                sm.va[lane] = ra.v0; sm.va[lane + 32] = ra.v1;
-                sm.vb[lane] = rb.v0; sm.vb[lane + 32] = rb.v1;
-                __syncwarp();
-                const double* e = W.work_epa + 4 * (size_t)k;
-                const V3<double> n64 = v3<double>(e[0], e[1], e[2]);
-                t1 = clock64();
-                if constexpr (EXACT) {
-                    hull_manifold<R, EXACT>(sm, W, ra, rb, ha, hb, a, b, v3cast<R>(n64), n64, fr);
-                } else {
-                    // the FP32 normal stored beside the FP64 one (no conversion in the warp)
-                    const float* f = W.work_face + 12 * (size_t)k;
-                    hull_manifold<R, EXACT>(sm, W, ra, rb, ha, hb, a, b, v3<R>(f[0], f[1], f[2]), n64, fr);
-                }
+        const int s = W.body_scene[item.z];
+        const long long t0 = clock64();
+        long long t1 = t0;
+        bool ok = true;
+        if constexpr (GENERAL) {
+            pair_contacts<R, EXACT>(W, sm, item.z, item.w, false);
+        } else {
+            const V3<R> offb = pair_offset<R, EXACT>(W, k);
+            const HullRef ha = W.hull_ref[item.z], hb = W.hull_ref[item.w];
+            const RegHull<R> ra = load_reghull(W, ha, v3<R>(0, 0, 0)), rb = load_reghull(W, hb, offb);
+            const double* e = W.work_epa + 4 * (size_t)k;
+            const V3<double> n64 = v3<double>(e[0], e[1], e[2]);
+            V3<R> nf;
+            if constexpr (EXACT) {
+                nf = v3cast<R>(n64);
+            } else {   // the FP32 normal stored beside the FP64 one (no conversion in the warp)
+                const float* f = W.work_face + 12 * (size_t)k;
+                nf = v3<R>(f[0], f[1], f[2]);
             }
-            const long long t2 = clock64();
-            t.v[1] += t2 - t0;
-            t.v[2] += t1 - t0;
-            if (!EXACT && !GENERAL && (sm.status & ST_DEG_SKEW)) {
-                if (lane == 0) {
-                    W.work_state[k] = WS_FALLBACK;
-                    W.fallback_list[atomicAdd(&W.queue[5], 1)] = k;
-                }
-                __syncwarp();
-                continue;
-            }
-            emit_contacts(W, sm, s, gp, t.v[0]);
-            t.v[3] += clock64() - t2;
+            t1 = clock64();
+            ok = manifold_pair<R, EXACT>(W, sm, item, ra, rb, ha, hb, offb, n64, nf);
         }
+        const long long t2 = clock64();
+        t.v[1] += t2 - t0;
+        t.v[2] += t1 - t0;
+        if (!ok) {
+            if (lane == 0) W.work_state[k] = WS_FALLBACK;
+            __syncwarp();
+            continue;
+        }
+        emit_contacts(W, sm, s, item.y, t.v[0]);
+        t.v[3] += clock64() - t2;
     }
     const int slots[8] = {3, 14, 19, 20, -1, -1, -1, -1};
     t.flush(W.counters, slots);
+}
+
+// GJK of two register hulls as a function of its own: inlined into k_contact its FP32 sums are contracted
+// differently from k_gjk's, and the simplex of a tie is then another (22 of 1400 hits).
+template <typename R>
+__device__ __noinline__ bool gjk_pair(const RegHull<R>& ra, const RegHull<R>& rb, Simplex<R>& sx, int& gi, long long& tsup, R* saved,
+                                      bool& cycled) {
+    return gjk_run(RegMink<R>{ra, rb}, sx, gi, tsup, saved, cycled);
+}
+
+// A uniform vector as lane 0 has it: what follows is rounded as if it had been stored and loaded, not fused with
+// the operations it came from, so that a pair's contacts are the same bits in one kernel as in several.
+template <typename T>
+__device__ __forceinline__ V3<T> settle(V3<T> v) {
+    return v3<T>(__shfl_sync(0xffffffffu, v.x, 0), __shfl_sync(0xffffffffu, v.y, 0), __shfl_sync(0xffffffffu, v.z, 0));
+}
+
+// GJK, EPA and contact manifold of a pair in one go, a warp per candidate: k_gjk, k_epa, k_epa_finish and
+// k_manifold for worlds whose hits nearly all have a warp of their own (contact_in_one_pass). There the time is
+// latency, and each of those kernels starts with a launch and the same chain of loads (list, references,
+// vertices) over again; with several hits a warp their leaner registers, and the FP64 finish of 32 pairs at once,
+// count for more. Frames, apart -> in one: ten cubes 1.20 -> 1.07 ms, 150 bodies 2.46 -> 2.20, 640 bodies
+// 4.19 -> 3.74, 4096 bodies 5.59 -> 5.21, 96 towers of 64 cubes 4.46 -> 3.87; 96 heaps of up to 512 bodies
+// 11.0 -> 11.9, and those stay apart.
+template <typename R, bool EXACT>
+__global__ void __launch_bounds__(PIPE_BLOCK, 2) k_contact(WorldView<R> W) {
+    if (frame_abandoned(W.status)) return;
+    extern __shared__ __align__(16) unsigned char dyn_smem[];
+    NarrowSmem<R>& sm = reinterpret_cast<NarrowSmem<R>*>(dyn_smem)[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    const int n = W.queue[2];
+    for (int j = gw; j < n; j += nw) {
+        const int4 item = W.gjk_list[j];
+        const int k = item.x, gp = item.y;
+        const HullRef ha = W.hull_ref[item.z], hb = W.hull_ref[item.w];
+        const V3<R> offb = pair_offset<R, EXACT>(W, k);
+        const RegHull<R> ra = load_reghull(W, ha, v3<R>(0, 0, 0)), rb = load_reghull(W, hb, offb);
+        WarpTally t;
+        {
+            Simplex<R> sx;
+            int gi = 0;
+            long long tsup = 0;
+            bool cycled = false;
+            const long long t0 = clock64();
+            const bool hit = gjk_pair(ra, rb, sx, gi, tsup, sm.gjk_saved, cycled);
+            if (lane == 0 && W.counters) {
+                atomicAdd(&W.counters[0], (unsigned long long)gi);
+                if (gi >= 100) atomicAdd(&W.counters[4], 1ull);
+                atomicAdd(&W.counters[12], (unsigned long long)(clock64() - t0));
+                atomicAdd(&W.counters[15], (unsigned long long)tsup);
+                if (cycled) atomicAdd(&W.counters[16], 1ull);
+                atomicAdd(&W.counters[10], 1ull);
+            }
+            int state = WS_NONE;
+            V3<double> n64;
+            double pen;
+            if (hit) {
+                sx.a = settle(sx.a); sx.b = settle(sx.b); sx.c = settle(sx.c); sx.d = settle(sx.d);
+                state = epa_pair<R, EXACT, true>(W, sm, item, ra, rb, sx, n64, pen, t);
+                __syncwarp();
+            } else if (lane == 0) {
+                W.pair_ccount[gp] = 0;
+                W.pair_cstart[gp] = 0;
+            }
+            if (state == WS_EPA_FACE) epa_face_finish_call(W.work_face + 12 * (size_t)k, n64, pen);
+            if (state == WS_EPA_FACE || state == WS_EPA_OK) {
+                const long long t1 = clock64();
+                n64 = settle(n64);
+                state = manifold_pair<R, EXACT>(W, sm, item, ra, rb, ha, hb, offb, n64, v3cast<R>(n64)) ? WS_EPA_OK : WS_FALLBACK;
+                t.v[6] = clock64() - t1;
+                if (state == WS_EPA_OK) emit_contacts(W, sm, W.body_scene[item.z], gp, t.v[7]);
+            }
+            if (lane == 0) W.work_state[k] = state;
+        }
+        const int slots[8] = {1, 2, 13, 7, -1, 18, 14, 3};
+        t.flush(W.counters, slots);
+        __syncwarp();
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -912,6 +1007,7 @@ struct PipeLauncher {
     static cudaError_t configure(PipeConfig& c, int sms) {
         cudaError_t e = cudaFuncSetAttribute(k_gjk<R, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gjk_smem());
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k_epa<R, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)narrow_smem());
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_contact<R, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)narrow_smem());
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k_manifold<R, EXACT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)narrow_smem());
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k_manifold<R, EXACT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)narrow_smem());
         if (e == cudaSuccess && !EXACT)
@@ -924,6 +1020,8 @@ struct PipeLauncher {
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, block, smem) != cudaSuccess) b = 1;
             return b < 1 ? 1 : b;
         };
+        nb = occ((const void*)k_contact<R, EXACT>, PIPE_BLOCK, narrow_smem());
+        c.contact_blocks = 4 * nb * sms;   // a warp per candidate: blocks start as others end, the work is uneven
         nb = occ((const void*)k_gjk<R, EXACT>, PIPE_BLOCK, gjk_smem());
         c.gjk_blocks = nb * sms;
         nb = occ((const void*)k_epa<R, EXACT>, PIPE_BLOCK, narrow_smem());
@@ -1030,17 +1128,22 @@ struct PipeLauncher {
             if (P.enable_collisions) {
                 k_transform<R, EXACT><<<col_blocks, PIPE_BLOCK, 0, st>>>(W, group);
                 if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(PH_TRANSFORM)) != cudaSuccess) return e;
-                k_gjk<R, EXACT><<<std::min(c.gjk_blocks, warp_blocks), PIPE_BLOCK, gjk_smem(), st>>>(W);
-                if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(PH_GJK)) != cudaSuccess) return e;
-                k_epa<R, EXACT><<<std::min(c.epa_blocks, warp_blocks), PIPE_BLOCK, narrow_smem(), st>>>(W);
-                if ((e = cudaGetLastError()) != cudaSuccess) return e;
-                if (!EXACT) {
-                    k_epa_finish<R><<<by_thread, PIPE_BLOCK, 0, st>>>(W);
+                if (d.one_pass) {
+                    k_contact<R, EXACT><<<std::min(c.contact_blocks, warp_blocks), PIPE_BLOCK, narrow_smem(), st>>>(W);
+                    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+                } else {
+                    k_gjk<R, EXACT><<<std::min(c.gjk_blocks, warp_blocks), PIPE_BLOCK, gjk_smem(), st>>>(W);
+                    if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(PH_GJK)) != cudaSuccess) return e;
+                    k_epa<R, EXACT><<<std::min(c.epa_blocks, warp_blocks), PIPE_BLOCK, narrow_smem(), st>>>(W);
+                    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+                    if (!EXACT) {
+                        k_epa_finish<R><<<by_thread, PIPE_BLOCK, 0, st>>>(W);
+                        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+                    }
+                    if ((e = mark(PH_EPA)) != cudaSuccess) return e;
+                    k_manifold<R, EXACT, false><<<std::min(c.manifold_blocks, warp_blocks), PIPE_BLOCK, narrow_smem(), st>>>(W);
                     if ((e = cudaGetLastError()) != cudaSuccess) return e;
                 }
-                if ((e = mark(PH_EPA)) != cudaSuccess) return e;
-                k_manifold<R, EXACT, false><<<std::min(c.manifold_blocks, warp_blocks), PIPE_BLOCK, narrow_smem(), st>>>(W);
-                if ((e = cudaGetLastError()) != cudaSuccess) return e;
                 if (d.general) {   // compound bodies, spheres or large hulls in the world
                     k_manifold<R, EXACT, true><<<std::min(c.general_blocks, warp_blocks), PIPE_BLOCK, narrow_smem(), st>>>(W);
                     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -1078,7 +1181,9 @@ struct PipeLauncher {
         return cudaSuccess;
     }
 
-    static int narrow_launches(const PipeDims& d) { return (EXACT ? 5 : 7) + (d.general ? 1 : 0); }
+    static int narrow_launches(const PipeDims& d) {
+        return 2 + (d.one_pass ? 1 : (EXACT ? 3 : 4)) + (EXACT ? 0 : 1) + (d.general ? 1 : 0);
+    }
 
     static int launches_per_frame(const StepParams& P, const PipeDims& d) {
         if (d.solve)

@@ -128,6 +128,24 @@ def test_many_small_scenes_equal_few(precision):
             assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_one_pass_contacts_equal_separate_kernels(precision):
+    # a small world takes EPA and manifold in one kernel with GJK, one of more pair slots (16 a body) than 48 a
+    # resident warp, 116736, apart
+    piles = [S.random_pile_scene(n, seed=n) for n in (2, 9, 20)] + [S.tower_scene(8, seed=1), S.chain_scene(6, "spherical", seed=3)]
+    others = [S.random_pile_scene(24, seed=k % 8) for k in range(400)]
+    states = []
+    for scs in (piles, piles + others):
+        w = rawphys.World(0, precision)
+        first = [w.load(sc, 0 if k == 0 else w.new_scene()) for k, sc in enumerate(scs)]
+        w.simulate(1.0 / 60.0, 20, 1, True, 40)
+        state = w.get_state()
+        states.append([state[f:f + sc.num_bodies] for f, sc in zip(first, piles)])
+        w.close()
+    for sc, a, b in zip(piles, *states):
+        assert np.array_equal(a, b), sc.name
+
+
 def test_adjoint_in_groups_equals_all_at_once():
     # 64 scenes tape a few substeps at a time, one scene all of its segment's: the same gradients, bit for bit
     batch, last, target = S.domino_batch(64, seed=2, min_dominoes=1, max_dominoes=3)
