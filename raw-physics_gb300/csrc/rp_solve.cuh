@@ -25,39 +25,6 @@ namespace rp {
 
 constexpr double PI_REF = 3.14159265358979;   // PI_F of include/gm.h:8
 
-template <typename R>
-struct Body {
-    V3<double> x;
-    Qt<double> q;
-    R invm;
-    M3<R> Iinv;       // local inverse inertia
-    bool fixed;
-    int idx;
-};
-
-template <typename R>
-__device__ __forceinline__ Body<R> load_body(const WorldView<R>& W, int b) {
-    Body<R> B;
-    double4_32a p = W.pos[b], q = W.rot[b];
-    B.x = v3<double>(p.x, p.y, p.z);
-    B.q = qt<double>(q.x, q.y, q.z, q.w);
-    B.invm = W.inv_mass[b];
-    R s[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) s[i] = W.inv_inertia[6 * b + i];
-    B.Iinv = msym(s);
-    B.fixed = W.fixed[b] != 0;
-    B.idx = b;
-    return B;
-}
-
-template <typename R>
-__device__ __forceinline__ void store_pose(const WorldView<R>& W, const Body<R>& B) {
-    if (B.fixed) return;
-    W.pos[B.idx] = make_double4_32a(B.x.x, B.x.y, B.x.z, 0.0);
-    W.rot[B.idx] = make_double4_32a(B.q.x, B.q.y, B.q.z, B.q.w);
-}
-
 // Rotation used for the working-precision algebra of a body.
 template <typename R>
 __device__ __forceinline__ Qt<R> wq(const Qt<double>& q) { return qcast<R>(q); }
@@ -97,19 +64,6 @@ __device__ __forceinline__ Qt<double> qnormalize_fast(Qt<double> q) {
     double r = (double)rsqrtf((float)n2);
     r = __dmul_rn(r, __fma_rn(-__dmul_rn(__dmul_rn(0.5, n2), r), r, 1.5));
     return qt<double>(q.x * r, q.y * r, q.z * r, q.w * r);
-}
-
-// q <- normalize(q + s * dq): the linearised orientation update, accumulated in FP64
-template <typename R>
-__device__ __forceinline__ void q_add_normalize(Qt<double>& q, Qt<R> d, double s) {
-    if (sizeof(R) == 8) {
-        q.x = q.x + s * (double)d.x; q.y = q.y + s * (double)d.y; q.z = q.z + s * (double)d.z; q.w = q.w + s * (double)d.w;
-        q = qnormalize(q);
-    } else {
-        q.x = q.x + (double)((R)s * d.x); q.y = q.y + (double)((R)s * d.y);
-        q.z = q.z + (double)((R)s * d.z); q.w = q.w + (double)((R)s * d.w);
-        q = qnormalize_fast(q);
-    }
 }
 
 // limit_angle (pbd.cpp:175-217)
