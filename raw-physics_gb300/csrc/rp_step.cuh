@@ -931,23 +931,27 @@ __device__ void resched(const WorldView<R>& W, const G& g, int s) {
     }
     g.sync();
     const int n0 = *(volatile int*)v0.active, n1 = *(volatile int*)v1.active;
-    if (g.rank() == 0) { *v0.levels = 0; *v1.levels = 0; }
     if constexpr (std::is_same<G, GridGroup>::value) {
         if (n0 + n1 <= RESCHED_ONE_CTA) {
-            // the two schedules at once, a CTA each
+            // the two schedules at once, a CTA each, which also resets its level count: the block barriers of
+            // relax_schedule order the reset before the counting (another CTA's could come after it)
             const int other = g.nblocks() > 1 ? 1 : 0;
             SubBlock q;
             if (g.block() == 0) {
+                if (q.rank() == 0) *v0.levels = 0;
                 relax_schedule(W, q, s, v0, n0, order);
                 bucket_schedule(W, q, s, v0, n0, true);
             }
             if (g.block() == other) {
+                if (q.rank() == 0) *v1.levels = 0;
                 relax_schedule(W, q, s, v1, n1, order);
                 bucket_schedule(W, q, s, v1, n1, false);
             }
         } else {
             SubGrid q{g};
             if (g.rank() == 0) {
+                *v0.levels = 0;
+                *v1.levels = 0;
                 int* f0 = v0.fill + W.max_levels - 2;
                 int* f1 = v1.fill + W.max_levels - 2;
                 f0[0] = f0[1] = f0[2] = 0;
@@ -960,7 +964,10 @@ __device__ void resched(const WorldView<R>& W, const G& g, int s) {
             bucket_schedule(W, q, s, v1, n1, false);
         }
         g.sync();
-    } else if constexpr (std::is_same<G, WarpGroup>::value) {
+        return;
+    }
+    if (g.rank() == 0) { *v0.levels = 0; *v1.levels = 0; }
+    if constexpr (std::is_same<G, WarpGroup>::value) {
         SubWarp q;
         relax_schedule(W, q, s, v0, n0, order);
         relax_schedule(W, q, s, v1, n1, order);
