@@ -259,13 +259,16 @@ __global__ void __launch_bounds__(SOLVE_BLOCK, 2) k_solve(WorldView<R> W, const 
             for (int which = 0; which < 2; ++which) {
                 const SchedView<R> v = sched_view(W, s, which);
                 const int L = sh.L[which];
-                for (int l = tid; l <= L; l += nt) { v.count[l] = l ? sh.cnt[which][l - 1] : 0; v.fill[l] = 0; }
-                if (tid == 0) *v.levels = L;
+                // zero beyond L up to the levels of the schedule recorded before: resched counts on it
+                const int used = max(L, min(*(volatile int*)v.levels + 1, W.max_levels));
+                for (int l = tid; l <= used; l += nt) { v.count[l] = l && l <= L ? sh.cnt[which][l - 1] : 0; v.fill[l] = 0; }
                 const int m = L ? sh.cnt[which][L - 1] : 0;
                 for (int i = tid; i < m; i += nt) {
                     const int r = ord[which * room.nodes + i];
                     v.nodes[i] = rec[r].pair < 0 ? r : rec[r].pair - pbase + ne;
                 }
+                __syncthreads();
+                if (tid == 0) *v.levels = L;
             }
         }
         // lane pairs (exact build: eight lanes) take a level's nodes, consecutive nodes in different warps (a warp runs as long as its
