@@ -388,6 +388,18 @@ rp_status build_device(rp_world* w) {
         shapes.push_back(sh);
     }
     fstart.push_back((int32_t)felem.size());
+    // A hull takes the general narrowphase path when its counts do not fit the records' bytes, or when a topology
+    // made by the caller lacks what the records lead to: a face's first vertex, a face of a vertex with neighbours.
+    std::vector<uint8_t> recordable(w->hulls.size(), 0);
+    for (size_t h = 0; h < w->hulls.size(); ++h) {
+        const Hull& H = *w->hulls[h];
+        bool ok = H.nv() <= 64 && H.nf() <= 255;
+        for (const auto* rows : {&H.faces, &H.v2f, &H.v2n, &H.f2n})
+            for (const auto& r : *rows) ok = ok && r.size() <= 255;
+        for (const auto& r : H.faces) ok = ok && !r.empty();
+        for (size_t v = 0; ok && v < H.v2f.size(); ++v) ok = !H.v2f[v].empty() || H.v2n[v].empty();
+        recordable[h] = ok;
+    }
     // byte records of each distinct topology for the narrowphase's warp kernels (HullRef, rp_world.h)
     std::vector<uint8_t> rec;
     std::vector<HullRef> hull_recs(w->hulls.size());
@@ -397,7 +409,7 @@ rp_status build_device(rp_world* w) {
             const Hull& H = *w->hulls[h];
             HullRef r;
             std::memset(&r, 0, sizeof(r));
-            if (H.nv() <= 64) {
+            if (recordable[h]) {
                 auto it = done.find(shapes[h].elem_off);
                 if (it == done.end()) {
                     auto emit = [&](size_t rows, auto&& bytes_of, int32_t& first, int32_t& stride) {
@@ -417,6 +429,11 @@ rp_status build_device(rp_world* w) {
                     emit((size_t)H.nv(), [&](size_t v) {
                         std::vector<uint8_t> b{(uint8_t)H.v2f[v].size(), (uint8_t)H.v2n[v].size()};
                         for (int f : H.v2f[v]) b.push_back((uint8_t)f);
+                        if (H.v2f[v].empty()) {   // a vertex of no triangle: the face read for it as a support point
+                            size_t u = v;
+                            while (u < H.v2f.size() && H.v2f[u].empty()) ++u;
+                            b.push_back(u < H.v2f.size() ? (uint8_t)H.v2f[u][0] : (uint8_t)0);
+                        }
                         for (int u : H.v2n[v]) b.push_back((uint8_t)u);
                         return b;
                     }, r.vrec, r.vstride);
@@ -436,15 +453,6 @@ rp_status build_device(rp_world* w) {
             r.face_off = shapes[h].face_off;
             hull_recs[h] = r;
         }
-    }
-    // a hull whose counts do not fit the records' bytes takes the general narrowphase path
-    std::vector<uint8_t> recordable(w->hulls.size(), 0);
-    for (size_t h = 0; h < w->hulls.size(); ++h) {
-        const Hull& H = *w->hulls[h];
-        bool ok = H.nv() <= 64 && H.nf() <= 255;
-        for (const auto* rows : {&H.faces, &H.v2f, &H.v2n, &H.f2n})
-            for (const auto& r : *rows) ok = ok && r.size() <= 255;
-        recordable[h] = ok;
     }
     // colliders, transformed-geometry offsets
     std::vector<Collider> cols;

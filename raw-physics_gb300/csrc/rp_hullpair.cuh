@@ -234,13 +234,16 @@ __device__ void hull_manifold(NarrowSmem<R>& sm, const WorldView<R>& W, const Re
     const V3<R>* rn = ref1 ? na : nb;
     const V3<R>* rv = ref1 ? sm.va : sm.vb;
     const V3<R>* iv = ref1 ? sm.vb : sm.va;
-    const int nref = rr[0], npl = rr[1], ninc = ri[0];
+    const int nref = rr[0], neighbours = rr[1], corners = ri[0];
+    // a face has as many neighbours as faces share a vertex with it, up to the record's 255
+    if ((neighbours > CLIP_MAX || corners > CLIP_MAX) && lane == 0) atomicOr(&sm.status, (int)ST_CLIP_OVERFLOW);
+    const int npl = min(neighbours, CLIP_MAX), ninc = min(corners, CLIP_MAX);
     for (int base = 0; base < ninc; base += WARP) {
         const int k = base + lane, v = ri[2 + k];
         if (k < ninc) sm.u.clip.buf[0][k] = iv[v];
     }
     for (int base = 0; base < npl; base += WARP) {
-        const int k = base + lane, nf = rr[2 + nref + k], v = rr[2 + nref + npl + k];
+        const int k = base + lane, nf = rr[2 + nref + k], v = rr[2 + nref + neighbours + k];
         if (k < npl) {
             sm.u.clip.pp[k] = rv[v];
             sm.u.clip.pn[k] = vinv(rn[nf]);
