@@ -84,6 +84,7 @@ __device__ __forceinline__ AVar a_leaf(double x) {
     }
     s_tape.level[i] = 0;
     s_tape.n = i + 1;
+    s_tape.levels = max(s_tape.levels, 1);   // a tape of inputs alone (a scene of fixed bodies) has one level
     return AVar(x, i, 0);
 }
 __device__ __noinline__ AVar a_op1(double v, const AVar& a, double da) {

@@ -1,0 +1,34 @@
+"""The adjoint's tapes: scenes without anything to differentiate, and how much scratch a call takes."""
+import numpy as np
+import pytest
+
+import rawphys
+from rawphys import scenes as S
+
+pytestmark = pytest.mark.gpu
+KEYS = ("grad_v", "grad_w", "grad_mass", "grad_friction")
+
+
+@pytest.mark.parametrize("collisions", [True, False])
+def test_a_scene_of_fixed_bodies_in_a_batch(collisions):
+    # its tape holds inputs only; the scenes beside it are what they are without it
+    batch, last, target = S.domino_batch(3, seed=5, min_dominoes=1, max_dominoes=2)
+    floor = S._Builder("floor")
+    S._floor(floor)
+    floor.hull_body("cube", (0.5, 0.5, 0.5), (0.0, 0.4, 0.0), fixed=True)
+    floor = floor.finish(dt=1.0 / 60.0, substeps=20, pos_iters=1, collisions=True, steps=1)
+    w = rawphys.World(0, "fp64")
+    w.load_batch(batch)
+    alone = w.adjoint(2, last, target, substeps=5, collisions=collisions)
+    w.close()
+    w = rawphys.World(0, "fp64")
+    n = w.load_batch(batch) + batch.num_bodies
+    f = w.load(floor, w.new_scene())
+    assert f == n
+    res = w.adjoint(2, [int(e) for e in last] + [f + 1], np.vstack([target, [[1.0, 2.0, 3.0]]]), substeps=5, collisions=collisions)
+    w.close()
+    assert np.array_equal(res["loss"][:3], alone["loss"])
+    assert res["loss"][3] == 1.0 + 1.6 ** 2 + 9.0
+    for k in KEYS:
+        assert np.array_equal(res[k][:n], alone[k]), k
+        assert not np.any(res[k][n:]), k
