@@ -109,7 +109,11 @@ rp_status rp_world_set_stream(rp_world* w, void* cuda_stream);
  * RP_ERR_INVALID with collisions on. The forward pass is the all-FP64 step: its loss equals the FP64
  * build's. Reverse mode over a tape per substep, many substeps taped at once, with the trajectory checkpointed
  * every `checkpoint_every` frames and recomputed segment by segment. Starts from the world's current
- * state, which it does not change. target: 3 doubles per scene. */
+ * state, which it does not change. target: 3 doubles per scene.
+ * Device memory: the trajectory's checkpoints and one segment's substeps, and the tapes, with collisions about 600 KB
+ * per body and position iteration for a substep. As many substeps are taped at once as the GPU runs, within 8 GB and half of
+ * the free memory; scenes whose tapes do not fit beside each other take turns. A longer tape than provided for makes
+ * it four times as long, twice at most, then RP_ERR_CAPACITY. The memory stays with the world until it is destroyed. */
 rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t num_substeps, uint32_t num_pos_iters,
                                 int32_t enable_collisions, uint32_t frames, uint32_t checkpoint_every,
                                 const int32_t* loss_entity, const double* target, double* loss_out, double* grad_v,

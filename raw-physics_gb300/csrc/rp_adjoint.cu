@@ -552,8 +552,9 @@ __global__ void __launch_bounds__(REV_BLOCK) k_adjoint_reverse(const AdjointScen
     }
 }
 
-cudaError_t adjoint_launch(const AdjointScene* scenes, int nscenes, const AdjointWorker* workers, int G, const AdjointParams& P,
-                           cudaStream_t st, int* launches) {
+cudaError_t adjoint_launch(const AdjointScene* scenes, const int* turns, int nturns, const AdjointWorker* workers, int G,
+                           const AdjointParams& P, cudaStream_t st, int* launches) {
+    const int nscenes = turns[nturns];
     const size_t smem = (size_t)ADJ_RING * 8 + (size_t)CHUNK_EDGES * 12 + (size_t)(CHUNK_ENTRIES + 1) * 4;
     cudaError_t e = cudaFuncSetAttribute(k_adjoint_reverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -566,11 +567,13 @@ cudaError_t adjoint_launch(const AdjointScene* scenes, int nscenes, const Adjoin
             ++*launches;
         }
         const int nsub = (min(P.frames, (seg + 1) * K) - seg * K) * P.substeps;
-        for (int last = nsub - 1; last >= 0; last -= G) {
-            k_adjoint_tape<<<nscenes * G, TAPE_BLOCK, 0, st>>>(scenes, workers, P, G, last);
-            k_adjoint_reverse<<<nscenes, REV_BLOCK, smem, st>>>(scenes, workers, G, last);
-            *launches += 2;
-        }
+        for (int last = nsub - 1; last >= 0; last -= G)
+            for (int t = 0; t < nturns; ++t) {
+                const int s0 = turns[t], n = turns[t + 1] - s0;
+                k_adjoint_tape<<<n * G, TAPE_BLOCK, 0, st>>>(scenes + s0, workers + s0 * G, P, G, last);
+                k_adjoint_reverse<<<n, REV_BLOCK, smem, st>>>(scenes + s0, workers + s0 * G, G, last);
+                *launches += 2;
+            }
     }
     return cudaGetLastError();
 }

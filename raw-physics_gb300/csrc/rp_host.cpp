@@ -2041,7 +2041,7 @@ rp_status rp_autotune(rp_world* w, double dt, uint32_t substeps, uint32_t iters,
     return s != RP_OK ? s : r;
 }
 
-constexpr size_t ADJ_TAPE_BYTES = (size_t)8 << 30;   // scratch of the substeps an adjoint tapes at once
+constexpr size_t ADJ_TAPE_BYTES = (size_t)8 << 30;   // scratch of the substeps an adjoint tapes at once, at most
 
 rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint32_t iters, int32_t collisions,
                                 uint32_t frames, uint32_t checkpoint_every, const int32_t* loss_entity, const double* target,
@@ -2211,23 +2211,64 @@ rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint3
             v.mcap = o.mcap;
             return used;
         };
-        // Substeps taped at once, of each scene: enough for four blocks on every SM (a block is one thread's
-        // serial work), no more than a segment has, within ADJ_TAPE_BYTES of scratch; the groups of a segment
-        // are of one size as nearly as can be.
-        size_t each = 0;
-        for (int s = 0; s < S; ++s) each += worker(s, nullptr, nullptr);
-        const int nsub = (int)(std::min<size_t>(K, frames) * substeps);
-        int G = std::max(1, std::min(nsub, 4 * sms / S));
-        while (G > 1 && each * (size_t)G > ADJ_TAPE_BYTES) --G;
-        const int groups = (nsub + G - 1) / G;
-        G = (nsub + groups - 1) / groups;
-        for (int s = 0; s < S; ++s) off[(size_t)s].worker = take((size_t)G * worker(s, nullptr, nullptr));
         const size_t inputs = (13 + 1 + 12 + 3 + 6 + 1) * N * 8 + 2 * N + 256;
-        RP_CUDA(w->d_adj_data.ensure(total + inputs + 1024));
+        std::vector<size_t> one((size_t)S);   // bytes of a scene's worker
+        size_t each = 0;
+        for (int s = 0; s < S; ++s) each += one[(size_t)s] = worker(s, nullptr, nullptr);
+        const int nsub = (int)(std::min<size_t>(K, frames) * substeps);
+        // Substeps taped at once, of each scene: enough for four blocks on every SM (a block is one thread's
+        // serial work), no more than a segment has, within `most` bytes of scratch; the groups of a segment
+        // are of one size as nearly as can be. Scenes whose workers do not fit `room` together take turns in it.
+        int G = 1;
+        std::vector<int> turns;   // first scene of each turn, and S
+        auto lay_out = [&](size_t most, size_t room) -> size_t {
+            G = std::max(1, std::min(nsub, 4 * sms / S));
+            while (G > 1 && each * (size_t)G > most) --G;
+            const int groups = (nsub + G - 1) / G;
+            G = (nsub + groups - 1) / groups;
+            turns.assign(1, 0);
+            size_t at = 0, longest = 0;
+            for (int s = 0; s < S; ++s) {
+                const size_t bytes = one[(size_t)s] * (size_t)G;
+                if (at && at + bytes > room) {
+                    turns.push_back(s);
+                    at = 0;
+                }
+                off[(size_t)s].worker = total + at;
+                at += bytes;
+                longest = std::max(longest, at);
+            }
+            turns.push_back(S);
+            return longest;
+        };
+        // RP_ADJOINT_SCRATCH (tests only): bytes of room
+        const char* room_env = std::getenv("RP_ADJOINT_SCRATCH");
+        const size_t most_room = room_env ? (size_t)std::strtoull(room_env, nullptr, 10) : ~(size_t)0;
+        size_t region = lay_out(std::min(ADJ_TAPE_BYTES, most_room), most_room);
+        const size_t rest = total + inputs + 1024;
+        if (rest + region > w->d_adj_data.bytes) {
+            // a new buffer: at most half of the free memory for substeps side by side, the rest of it only where
+            // the scenes need it for a worker each
+            size_t free_bytes = 0, all_bytes = 0;
+            if (cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess) {
+                const size_t has = free_bytes + w->d_adj_data.bytes;
+                const size_t left = has > rest ? has - rest : 0;
+                region = lay_out(std::min({ADJ_TAPE_BYTES, most_room, left / 2}), std::min(most_room, left - left / 16));
+            }
+            const size_t least = *std::max_element(one.begin(), one.end());
+            for (size_t room = region;;) {
+                const cudaError_t e = w->d_adj_data.ensure(rest + region);
+                if (e == cudaSuccess) break;
+                if (e != cudaErrorMemoryAllocation || region <= least) return fail(RP_ERR_CUDA, cudaGetErrorString(e));
+                (void)cudaGetLastError();   // less at once gives the same gradients
+                room /= 2;
+                region = lay_out(room, room);
+            }
+        }
         RP_CUDA(w->d_adj_ext.ensure(std::max<size_t>(ext.size(), 1) * sizeof(ExtConstraint)));
         RP_CUDA(w->d_adj_scenes.ensure((size_t)S * sizeof(AdjointScene)));
         char* base = (char*)w->d_adj_data.p;
-        char* in = base + total;
+        char* in = base + total + region;
         double* d_start = (double*)in;
         double* d_invm = d_start + 13 * N;
         double* d_I = d_invm + N;
@@ -2302,9 +2343,8 @@ rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint3
             a.prof = (long long*)(base + o.prof);
             a.bodies_d = base + o.bd;
             a.lam_d = (double*)(base + o.lamd);
-            const size_t bytes = worker(s, nullptr, nullptr);
             for (int k = 0; k < G; ++k)
-                worker(s, base + o.worker + (size_t)k * bytes, &workers[(size_t)s * (size_t)G + (size_t)k]);
+                worker(s, base + o.worker + (size_t)k * one[(size_t)s], &workers[(size_t)s * (size_t)G + (size_t)k]);
         }
         RP_CUDA(cudaMemcpyAsync(w->d_adj_scenes.p, scenes.data(), scenes.size() * sizeof(AdjointScene),
                                 cudaMemcpyHostToDevice, w->stream));
@@ -2329,8 +2369,8 @@ rp_status rp_adjoint_trajectory(rp_world* w, double dt, uint32_t substeps, uint3
         P.geom.col_start = w->d_col_start.as<int32_t>();
         P.geom.radius = w->d_radius.as<double>();
         int launches = 0;
-        RP_CUDA(adjoint_launch(w->d_adj_scenes.as<AdjointScene>(), S, w->d_adj_workers.as<AdjointWorker>(), G, P, w->stream,
-                               &launches));
+        RP_CUDA(adjoint_launch(w->d_adj_scenes.as<AdjointScene>(), turns.data(), (int)turns.size() - 1,
+                               w->d_adj_workers.as<AdjointWorker>(), G, P, w->stream, &launches));
         w->launches += launches;
         // results
         std::vector<double> g(13 * N), gi(N), gmu(2 * N);

@@ -153,9 +153,10 @@ struct AdjointWorker {
     long long* cycles;                     // [1]
     int ncap, mcap;
 };
-// workers: G per scene, in scene order; *launches counts the kernels
-cudaError_t adjoint_launch(const AdjointScene* scenes, int nscenes, const AdjointWorker* workers, int G, const AdjointParams& P,
-                           cudaStream_t st, int* launches);
+// workers: G per scene, in scene order. turns[0, nturns]: the scenes turns[t] to turns[t + 1] - 1 are taped and reversed
+// together, one turn after another (their workers may share memory). *launches counts the kernels.
+cudaError_t adjoint_launch(const AdjointScene* scenes, const int* turns, int nturns, const AdjointWorker* workers, int G,
+                           const AdjointParams& P, cudaStream_t st, int* launches);
 size_t adjoint_body_bytes(bool tape);
 size_t adjoint_var_bytes();
 // scratch sizes of the contact pipeline: contact record, a round's contacts, and of the taped pass (a worker)

@@ -32,3 +32,28 @@ def test_a_scene_of_fixed_bodies_in_a_batch(collisions):
     for k in KEYS:
         assert np.array_equal(res[k][:n], alone[k]), k
         assert not np.any(res[k][n:]), k
+
+
+def test_scenes_take_turns_where_their_tapes_do_not_fit(monkeypatch):
+    # the same gradients from one substep of one scene at a time (1 byte of room), from a few scenes at a time and
+    # from all at once; the launches tell how many turns there were
+    batch, last, target = S.domino_batch(6, seed=9, min_dominoes=1, max_dominoes=4)
+    results, launches = [], []
+    for room in (None, "1", str(20 << 20)):
+        if room:
+            monkeypatch.setenv("RP_ADJOINT_SCRATCH", room)
+        w = rawphys.World(0, "fp64")
+        w.load_batch(batch)
+        w.sync()
+        before = w.kernel_launches()
+        results.append(w.adjoint(3, last, target, checkpoint_every=2, substeps=4))
+        launches.append(w.kernel_launches() - before)
+        w.close()
+    # two segments of 8 and 4 substeps: two scalar passes (all frames; the first segment again), and per
+    # group of substeps and turn a taping and a reverse sweep
+    assert launches[0] == 2 + 2 * 2
+    assert launches[1] == 2 + 2 * 6 * (8 + 4)
+    assert launches[0] < launches[2] < launches[1]
+    for res in results[1:]:
+        for k in ("loss",) + KEYS:
+            assert np.array_equal(res[k], results[0][k]), k
