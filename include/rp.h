@@ -133,8 +133,9 @@ rp_status rp_world_set_sweep_order(rp_world* w, int32_t order);
  * worlds with a scene of more than 640 bodies, and in the coloured order (other worlds solve a scene per CTA,
  * whatever is set here). A launch shape: the same schedule under every choice, so FP64 results are identical
  * and FP32 results agree to rounding:
- * 0 one warp per scene (the default), 1 one CTA per scene, n >= 2 a whole CTA for every scene whose
- * sweep cost (dynamic bodies + 8 per joint) is n or more and one warp for each other scene.
+ * 0 (the default) a warp per scene, a whole CTA for a scene of 96 bodies or more and, in the FP64 coloured order,
+ * for one of sweep cost (dynamic bodies + 8 per joint) 96; 1 one CTA per scene; n >= 2 a whole CTA for every scene
+ * whose sweep cost is n or more and one warp for each other scene.
  * rp_autotune chooses among these (its choice[2]). No counterpart in the reference. */
 rp_status rp_world_set_sweep_assignment(rp_world* w, int32_t cta);
 /* Bound of every device-side wait of this world (the grid barriers of a single large scene's
@@ -152,9 +153,8 @@ rp_status rp_world_set_wait_limit(rp_world* w, uint64_t microseconds);
  * identical in RP_PRECISION_FP64 and agree to rounding in RP_PRECISION_FP32 (each kernel instantiation
  * may contract multiply-adds differently). Each candidate is timed twice; one replaces the default only
  * when at least 1 % faster. Call it with
- * no forces pending. choice receives {mode, transform threads, batch sweep assignment (0: a warp per
- * scene, 1: a CTA per scene, n >= 2: a CTA for scenes of n or more bodies plus 8 per joint, a warp for
- * the rest), solo level size}. */
+ * no forces pending. choice receives {mode, transform threads, batch sweep assignment
+ * (rp_world_set_sweep_assignment), solo level size}. */
 rp_status rp_autotune(rp_world* w, double dt, uint32_t num_substeps, uint32_t num_pos_iters, int32_t enable_collisions,
                       uint32_t frames, int32_t choice[4]);
 const char* rp_last_error(void);

@@ -165,13 +165,14 @@ struct rp_world {
     double adj_prof[6] = {0, 0, 0, 0, 0, 0};      // last adjoint's slowest scene (rp_adjoint_profile)
     DevBuf d_pose_f, d_col_body, d_tables, d_hull_ref, d_gjk_list, d_hit_list, d_work_list, d_work_state, d_work_simplex, d_work_epa, d_queue, d_work_off, d_work_face, d_fallback, d_tstamp, d_tlist, d_pair_base;
     // in d_tables
-    const int32_t *t_body_scene = nullptr, *t_scene_order = nullptr;
+    const int32_t *t_body_scene = nullptr, *t_scene_order = nullptr, *t_wide_order = nullptr;
     const uint8_t *t_single_hull = nullptr, *t_topo_rec = nullptr;
     int mode = RP_MODE_AUTO;          // RP_MODE_*: how a frame is launched
     int solo_nodes = 0;               // tunable: grid sweeps run levels up to this size on one CTA (0: the default)
-    int cta_from = 0;                 // tunable: batched sweeps give a whole CTA to scenes of this cost or more (0: none)
+    int cta_from = 0;                 // tunable: batched sweeps give a whole CTA to scenes of this cost or more (0: wide ones)
     std::vector<int64_t> order_cost;  // sweep cost of the scenes in scene_order (decreasing)
     int cta_scenes = 0;               // how many leading scenes of scene_order that is
+    int wide_scenes = 0, costly_scenes = 0;   // scenes of WIDE_SCENE bodies or more; of that cost or more
     uint64_t wait_ns = 1000000000ull; // bound of every device-side wait (rp_world_set_wait_limit)
     int sweep_order = RP_SWEEP_REFERENCE;   // Gauss–Seidel order of the sweeps (rp_world_set_sweep_order)
     bool pipe_ready = false;
@@ -675,6 +676,12 @@ rp_status build_device(rp_world* w) {
         w->order_cost.assign((size_t)S, 0);
         for (int sc = 0; sc < S; ++sc) w->order_cost[(size_t)sc] = cost(order[(size_t)sc]);
         set_cta_scenes(w);
+        std::vector<int32_t> wide = order;   // the wide scenes first
+        const auto narrow = std::stable_partition(wide.begin(), wide.end(), [&](int32_t x) {
+            return w->scene_body[(size_t)x + 1] - w->scene_body[(size_t)x] >= WIDE_SCENE;
+        });
+        w->wide_scenes = (int)(narrow - wide.begin());
+        w->costly_scenes = (int)std::count_if(w->order_cost.begin(), w->order_cost.end(), [](int64_t c) { return c >= WIDE_SCENE; });
         {   // scene-resident solves: two size classes, each in decreasing cost order
             std::vector<int32_t> list;
             PipeDims& d = w->dims;
@@ -710,9 +717,9 @@ rp_status build_device(rp_world* w) {
                 if (n) std::memcpy(&blob[at], v.data(), n);
                 return at;
             };
-            blob.reserve(body_scene.size() * 4 + rec.size() + single.size() + 8 * (size_t)S + 6 * 256);
+            blob.reserve(body_scene.size() * 4 + rec.size() + single.size() + 12 * (size_t)S + 7 * 256);
             const size_t o_scene = put(body_scene), o_rec = put(rec), o_single = put(single), o_order = put(order),
-                         o_list = put(list);
+                         o_wide = put(wide), o_list = put(list);
             RP_CUDA(upload(w->d_tables, blob, st));
             RP_CUDA(upload(w->d_hull_ref, refs, st));
             const unsigned char* t = w->d_tables.as<unsigned char>();
@@ -720,6 +727,7 @@ rp_status build_device(rp_world* w) {
             w->t_topo_rec = t + o_rec;
             w->t_single_hull = t + o_single;
             w->t_scene_order = reinterpret_cast<const int32_t*>(t + o_order);
+            w->t_wide_order = reinterpret_cast<const int32_t*>(t + o_wide);
             d.solve_scenes = reinterpret_cast<const int32_t*>(t + o_list);
         }
         RP_CUDA(w->d_queue.ensure(64));
@@ -875,8 +883,18 @@ WorldView<R> make_view(rp_world* w) {
     V.tstamp = w->d_tstamp.as<int32_t>();
     V.tlist = w->d_tlist.as<int32_t>();
     V.scene_order = w->t_scene_order;
-    V.solo_nodes = w->solo_nodes;
     V.cta_scenes = w->cta_scenes;
+    if (w->cta_from == 0) {
+        // A warp takes 16 nodes of a level at once (FP64: 4). Wider levels go in turns, so by default the scenes
+        // that have them get a whole CTA: those of WIDE_SCENE bodies, and in FP64 the coloured chains of that cost.
+        // Frames, coloured, a warp each -> so, FP32: 24 scenes of up to 512 bodies 11.9 -> 7.4 ms, 96 14.8 -> 10.0,
+        // 4096 83 -> 70; a chain's colours are half its links wide, which suits a warp there (4096 of 33 links
+        // 5.6 ms, a CTA each 7.2); FP64: 96 scenes 176 -> 83, 768 chains of 33 links 8.1 -> 5.4, of 65 15.0 -> 9.2.
+        const bool costly = w->precision == RP_PRECISION_FP64 && w->sweep_order == RP_SWEEP_COLOURED;
+        V.scene_order = costly ? w->t_scene_order : w->t_wide_order;
+        V.cta_scenes = costly ? w->costly_scenes : w->wide_scenes;
+    }
+    V.solo_nodes = w->solo_nodes;
     V.wait_ns = w->wait_ns;
     V.deg_first = w->d_deg.as<int32_t>();
     return V;
@@ -1980,8 +1998,8 @@ rp_status rp_autotune(rp_world* w, double dt, uint32_t substeps, uint32_t iters,
             return fail(RP_ERR_CUDA, "event timing");
         return RP_OK;
     };
-    // cta: how a batch's sweeps assign scenes: 1 = one CTA per scene (k_sweep_cta); 0 = one warp per
-    // scene; n >= 2 = scenes of sweep cost n or more get a whole CTA, the rest a warp each
+    // cta: how a batch's sweeps assign scenes: 1 = one CTA per scene (k_sweep_cta); 0 = wide scenes a whole
+    // CTA, the rest a warp each; n >= 2 = so for scenes of sweep cost n or more
     auto set_tune = [&](int mode, int group, int cta, int solo) {
         w->mode = mode;
         w->pipe.transform_group = group;
@@ -2022,7 +2040,7 @@ rp_status rp_autotune(rp_world* w, double dt, uint32_t substeps, uint32_t iters,
             for (int solo : {64, 128, 256, 512})
                 if (s == RP_OK) s = consider(RP_MODE_PHASED, g, cta0, solo);
         } else {
-            // the sweeps' scene assignment: every scene a warp, every scene a CTA, or the largest a CTA
+            // the sweeps' scene assignment: the wide scenes a CTA, every scene, or the costlier ones
             for (int cta : {0, 1, 96, 160, 256, 384})
                 if (s == RP_OK && cta != cta0) s = consider(RP_MODE_PHASED, g, cta, solo0);
         }

@@ -781,9 +781,10 @@ __global__ void __launch_bounds__(BLOCK) k_sweep_cta(WorldView<R> W, double h, i
     }
 }
 
-// One warp per scene: a scene's levels are mostly a few nodes wide, so a warp (barrier: __syncwarp)
-// sweeps them as fast as a CTA would while many more scenes are in flight per SM. Warps take scenes
-// from a counter (queue[1], zeroed before the launch) in decreasing-size order. The first position
+// One warp per scene, but for the W.cta_scenes first ones: a small scene's levels are mostly a few nodes wide, so
+// a warp (barrier: __syncwarp; 16 nodes at once, FP64 4) sweeps them as fast as a CTA would while many more
+// scenes are in flight per SM; a scene with wider levels gets a CTA (make_view has the rule). Warps take scenes
+// from a counter (queue[1], zeroed before the launch), costly ones first. The first position
 // sweep of a substep builds the substep's schedules first (resched).
 constexpr int SWEEP_WARP_BLOCK = 128;
 

@@ -105,6 +105,8 @@ struct __align__(16) HullRef {
 constexpr int SCAN_TMP_WORDS = 4096;
 // default of WorldView::solo_nodes (rp_step.cuh, sweep_levels)
 constexpr int SOLO_NODES = 32, SOLO_NODES_FP64 = 16;
+// batched sweeps: scenes of this many bodies have levels too wide for a warp
+constexpr int WIDE_SCENE = 96;
 // FP32 build: the single large scene's levels of at most this many nodes round both bodies of a contact alike
 constexpr int ALIKE_NODES = 512;
 

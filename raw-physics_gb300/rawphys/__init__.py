@@ -464,9 +464,9 @@ class World:
         self._check(self.lib.rp_world_set_sweep_order(self.h, self.SWEEP_ORDERS[order]))
 
     def set_sweep_assignment(self, cta: int):
-        """Scenes per warp or CTA in a batch's sweeps: 0 one warp per scene (default), 1 one CTA per
-        scene, n >= 2 a CTA for scenes of sweep cost n or more (a launch shape: FP64 results identical,
-        FP32 equal to rounding)."""
+        """Scenes per warp or CTA in a batch's sweeps: 0 a CTA for wide scenes and a warp for the others
+        (default), 1 one CTA per scene, n >= 2 a CTA for scenes of sweep cost n or more (a launch shape: FP64
+        results identical, FP32 equal to rounding)."""
         self._check(self.lib.rp_world_set_sweep_assignment(self.h, int(cta)))
 
     def set_wait_limit(self, microseconds: int):
@@ -483,7 +483,7 @@ class World:
                                          int(frames), out))
         modes = {v: k for k, v in self.MODES.items()}
         return {"mode": modes.get(out[0], out[0]), "transform_threads": out[1],
-                "batch_sweep_assignment": {0: "warp per scene", 1: "CTA per scene"}.get(out[2], "CTA for scenes of cost >= %d" % out[2]),
+                "batch_sweep_assignment": {0: "CTA for wide scenes", 1: "CTA per scene"}.get(out[2], "CTA for scenes of cost >= %d" % out[2]),
                 "solo_level_nodes": out[3]}
 
     def counters(self):
