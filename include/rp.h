@@ -148,9 +148,9 @@ rp_status rp_world_set_wait_limit(rp_world* w, uint64_t microseconds);
 /* Autotuner (no counterpart in the reference): times `frames` frames of the world's current scenes
  * from their current state under each candidate launch configuration — launch mode, threads per
  * collider in the hull transform (4/8/16/32), and the sweep layout (levels swept by one CTA up to
- * 16..512 nodes for one large scene; for a batch, which scenes a warp and which a whole CTA sweeps) —
- * keeps the fastest, and restores the state. Every configuration runs the same schedule: results are
- * identical in RP_PRECISION_FP64 and agree to rounding in RP_PRECISION_FP32 (each kernel instantiation
+ * 16..512 nodes for one large scene; for a batch, which scenes a warp and which a whole CTA sweeps;
+ * neither where every scene is solved by a CTA of its own) — keeps the fastest, and restores the state.
+ * Every configuration runs the same schedule: results are identical in RP_PRECISION_FP64 and agree to rounding in RP_PRECISION_FP32 (each kernel instantiation
  * may contract multiply-adds differently). Each candidate is timed twice; one replaces the default only
  * when at least 1 % faster. Call it with
  * no forces pending. choice receives {mode, transform threads, batch sweep assignment

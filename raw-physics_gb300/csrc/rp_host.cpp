@@ -2036,7 +2036,9 @@ rp_status rp_autotune(rp_world* w, double dt, uint32_t substeps, uint32_t iters,
         for (int g : {4, 8, 16, 32})
             if (s == RP_OK && g != group0) s = consider(RP_MODE_PHASED, g, cta0, solo0);
         const int g = best[1];
-        if (w->grid_mode) {
+        if (w->dims.solve) {
+            // no sweep kernels: their layout changes nothing
+        } else if (w->grid_mode) {
             for (int solo : {64, 128, 256, 512})
                 if (s == RP_OK) s = consider(RP_MODE_PHASED, g, cta0, solo);
         } else {

@@ -29,3 +29,26 @@ def test_wide_scenes_on_a_cta_equal_warps(precision, order):
         states.append(w.get_state())
         w.close()
     assert np.array_equal(*states)
+
+
+@pytest.mark.parametrize("solved", [True, False])
+def test_autotune_times_sweep_layouts_only_where_sweeps_run(solved):
+    # phased, persistent and three other transform groups; five more sweep assignments in the coloured order
+    w = rawphys.World(0, "fp32")
+    for k in range(4):
+        w.load(S.stack_scene(4, seed=k), 0 if k == 0 else w.new_scene())
+    if not solved:
+        w.set_sweep_order("coloured")
+    w.step(1)
+    before = w.kernel_launches()
+    w.step(10)
+    frame = (w.kernel_launches() - before) // 10
+    before = w.kernel_launches()
+    choice = w.autotune(frames=4)
+    frames = (w.kernel_launches() - before) / frame
+    trials = 2 * (1 + 4)   # each candidate twice, a warm-up and four frames (and the state's upload)
+    if choice["mode"] == "phased":
+        assert (4 if solved else 9) * trials <= frames <= (4 if solved else 9) * trials + 3 * trials
+    if solved:
+        assert choice["batch_sweep_assignment"] == "CTA for wide scenes"
+    w.close()
