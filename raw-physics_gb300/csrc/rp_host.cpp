@@ -17,9 +17,10 @@
 #include <atomic>
 #include <map>
 #include <memory>
+#include <string>
+#include <system_error>
 #include <thread>
 #include <type_traits>
-#include <string>
 #include <vector>
 
 namespace rp {
@@ -235,15 +236,22 @@ std::vector<unsigned char> as_working(const std::vector<double>& v, size_t rsize
 
 rp_status sync_state_to_host(rp_world* w);
 
-// work(lo, hi) over [0, n) in up to 16 chunks on as many threads, none smaller than `least`
+// work(lo, hi) over [0, n) in up to 16 chunks on as many threads, none smaller than `least`; what the system gives
+// no thread for is done here
 template <typename Work>
 void in_chunks(size_t n, size_t least, const Work& work) {
     const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
     const size_t chunks = std::max<size_t>(1, std::min<size_t>(hw, (n + least - 1) / least));
-    std::vector<std::thread> th;
-    for (size_t c = 1; c < chunks; ++c) th.emplace_back([&work, n, c, chunks] { work(n * c / chunks, n * (c + 1) / chunks); });
+    std::thread th[16];
+    size_t started = 1;
+    try {
+        for (; started < chunks; ++started)
+            th[started] = std::thread([&work, n, started, chunks] { work(n * started / chunks, n * (started + 1) / chunks); });
+    } catch (const std::system_error&) {
+    }
     work(0, n / chunks);
-    for (std::thread& t : th) t.join();
+    if (started < chunks) work(n * started / chunks, n);
+    for (size_t c = 1; c < started; ++c) th[c].join();
 }
 
 // Copies n doubles in parallel chunks (state records of a large batch are hundreds of MB: one core's
