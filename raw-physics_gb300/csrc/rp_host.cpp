@@ -746,6 +746,7 @@ rp_status build_device(rp_world* w) {
         RP_CUDA(w->d_tlist.ensure(std::max<size_t>(N, 1) * 4));
         w->dims.nbodies = (int)N;
         w->dims.ncolliders = (int)cols.size();
+        w->dims.collider_rows = cols.empty() ? 0 : (int)((std::max(tv, tn) + (int64_t)cols.size() - 1) / (int64_t)cols.size());
         w->dims.next = (int)E;
         w->dims.num_scenes = S;
         w->dims.grid_mode = w->grid_mode ? 1 : 0;
@@ -2019,7 +2020,7 @@ rp_status rp_autotune(rp_world* w, double dt, uint32_t substeps, uint32_t iters,
     };
     const int cta0 = w->pipe.sweep_cta ? 1 : w->cta_from;
     const bool fp64 = w->precision == RP_PRECISION_FP64;
-    const int group0 = transform_group_for(fp64, w->dims.ncolliders, w->num_sms), solo0 = fp64 ? SOLO_NODES_FP64 : SOLO_NODES;
+    const int group0 = transform_group_for(fp64, w->dims.ncolliders, w->dims.collider_rows, w->num_sms), solo0 = fp64 ? SOLO_NODES_FP64 : SOLO_NODES;
     int best[4] = {RP_MODE_PHASED, group0, cta0, solo0};
     float best_ms = 0.f;
     // each candidate timed twice (the faster run counts); a later candidate replaces the best only

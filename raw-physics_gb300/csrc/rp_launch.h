@@ -7,9 +7,17 @@
 namespace rp {
 
 // Launch shapes of the phase-major pipeline, chosen once per device (occupancy) and per world.
-// Threads per collider in the hull transform: a warp while every SM has room for the colliders' warps at once,
-// and always in FP64, whose time is the instructions of a warp; else four.
-inline int transform_group_for(bool fp64, int colliders, int sms) { return fp64 || colliders <= 16 * sms ? 32 : 4; }
+// Threads per collider in the hull transform. FP32: a warp while every SM has room for the colliders' warps at once,
+// else four. FP64, whose time is the instructions of a warp (69 for the pose, 18 a vertex and 45 a normal of its own
+// lanes): as many as a collider has vertices or faces on average (rows), up to a warp; further lanes only
+// repeat the pose. Transforms of a frame, four / eight / 32 threads: 8000 towers of 12 cubes 4.0 / 4.9 / 18.2 ms,
+// 1024 0.84 / 0.79 / 2.5; hulls of 32 rows: 12000 bodies 4.2 / 3.1 / 2.8, 217000 40.9 / 36.7 / 39.8.
+inline int transform_group_for(bool fp64, int colliders, int rows, int sms) {
+    if (!fp64) return colliders <= 16 * sms ? 32 : 4;
+    int g = 4;
+    while (g < 32 && g < rows) g *= 2;
+    return g;
+}
 
 // Whether GJK, EPA and manifold are one kernel (k_contact): there are 16 pair slots a body and about half a hit,
 // so 48 slots a resident warp (16 on an SM) are up to one and a half hits a warp, where both forms take as long.
@@ -28,6 +36,7 @@ struct PipeConfig {
 };
 struct PipeDims {
     int nbodies = 0, ncolliders = 0, next = 0, num_scenes = 0;
+    int collider_rows = 0;   // vertices or faces of a collider, the larger mean
     int pair_cap = 0;    // pair slots of the world
     int one_pass = 0;    // contact_in_one_pass
     int general = 0;     // some body is not a single hull of at most 64 vertices

@@ -1109,7 +1109,7 @@ struct PipeLauncher {
         const int by_thread = std::max(1, std::min(c.cull_blocks, (d.pair_cap + PIPE_BLOCK - 1) / PIPE_BLOCK));
         const int warp_blocks = std::max(1, (d.pair_cap + PIPE_WARPS - 1) / PIPE_WARPS);
         const int body_blocks = (d.nbodies * (EXACT ? 4 : 1) + d.next + PIPE_BLOCK - 1) / PIPE_BLOCK + 1;
-        const int group = c.transform_group ? c.transform_group : transform_group_for(EXACT, d.ncolliders, c.sms);
+        const int group = c.transform_group ? c.transform_group : transform_group_for(EXACT, d.ncolliders, d.collider_rows, c.sms);
         const int col_blocks = (d.ncolliders * group + PIPE_BLOCK - 1) / PIPE_BLOCK + 1;
         if ((e = mark(-1)) != cudaSuccess) return e;
         if (d.grid_mode) e = coop(k_setup_grid<R>, c.setup_grid_blocks, BLOCK, st, W, P.dt);
